@@ -31,6 +31,7 @@ cudaError_t run_inv_y_rev(const InvYArgs<6, float2>& a, const PassGeom& g, cudaS
 cudaError_t run_fwd_y_rev(const FwdYArgs<>& a, const PassGeom& g, cudaStream_t st);
 cudaError_t run_fwd_y_rev(const FwdYArgs<float2>& a, const PassGeom& g, cudaStream_t st);
 cudaError_t prepare_xy_rev(const PassGeom& g);
+cudaError_t prepare_xy_rev_f32(const PassGeom& g, int tile);  // the FP32 half (k_xy_rev32.cu)
 
 // FP64 scratch (double2) and the FP32 precision mode (float2 scratch).
 cudaError_t run_inv_x(const InvXArgs<3>& a, const PassGeom& g, cudaStream_t st);
@@ -50,6 +51,7 @@ cudaError_t run_z(const ZArgs<6, float2>& a, const PassGeom& g, cudaStream_t st)
 // Launch attributes of the pipelined passes for this geometry on the current
 // device; called when a handle is created (outside any stream capture).
 cudaError_t prepare_xy(const PassGeom& g);
+cudaError_t prepare_xy_f32(const PassGeom& g);  // the FP32 half (k_xy32.cu)
 cudaError_t prepare_fwdx(const PassGeom& g);
 cudaError_t prepare_fwdx_f32(const PassGeom& g);  // the FP32 half (k_fwdx32.cu)
 // Plain 3-D transforms (k_fft3d.cu): one complex line pass along x (axis 0)

@@ -173,7 +173,7 @@ constexpr int prec_tag() { return sizeof(C) == 16 ? 0 : 100; }
 template <int N, int P, int NF, typename C, int V = 0>
 cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStream_t st,
                            bool prepare_only) {
-  const long long lines = (long long)g.Ny * g.Mz * nbatch(g);
+  const long long lines = 8LL * g.nlive * nbatch(g);
   using S = PassSmem<N, P, C, double2, V>;
   const unsigned grid = persistent_grid<KTag<0, N, P, NF + prec_tag<C>() + 1000 * V>>(
       inv_x_kernel<N, P, NF, C, V>, S::BYTES, (lines + S::LPC - 1) / S::LPC);
@@ -243,7 +243,7 @@ template <int N, int P>
 cudaError_t launch_inv_y_tma(const InvYArgs<3, double2>& a, const PassGeom& g, cudaStream_t st,
                              bool prepare_only) {
   using S = InvYTmaSmem<N, P>;
-  const long long groups = (long long)g.Nx * ((g.Mz + S::LPC - 1) / S::LPC);
+  const long long groups = (long long)g.Nx * ((g.Zp + S::LPC - 1) / S::LPC);
   const unsigned grid = persistent_grid<KTag<90, N, P, 3>, NS3D_Y_TMA_PERSIST != 0>(
       inv_y_tma_kernel<N, P, 3>, S::BYTES, groups);
   if (prepare_only) return cudaGetLastError();
@@ -269,7 +269,7 @@ cudaError_t launch_inv_y_p(const InvYArgs<NF, C>& a, const PassGeom& g, cudaStre
       if (!prepare_only || e != cudaSuccess) return e;
     }
   }
-  const long long lines = (long long)g.Nx * g.Mz;
+  const long long lines = (long long)g.Nx * g.Zp;
   using S = PassSmem<N, P, C, C, V>;
   const unsigned grid = persistent_grid<KTag<1, N, P, NF + prec_tag<C>() + 1000 * V>>(
       inv_y_kernel<N, P, NF, C, V>, S::BYTES, (lines + S::LPC - 1) / S::LPC);

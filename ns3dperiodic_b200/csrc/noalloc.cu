@@ -26,6 +26,9 @@
 #include "../../include/ns3d.h"
 #include "dispatch.h"
 #include "launch.cuh"
+#include "solver_internal.h"
+
+using ns3d_detail::LiveTables;
 
 namespace {
 
@@ -53,11 +56,23 @@ struct DeviceSlot {
   // grid whose tables are currently in the scratch
   int Nx = 0, Ny = 0, Nz = 0;
   double Lx = 0, Ly = 0, Lz = 0;
+  // what that grid's mask leaves (PassGeom); the tables follow the cut-offs
+  int Zc = 0, Zp = 0, nlive = 0;
 };
+
+// the live blocks and row cut-offs, after the Nx Ny cut-offs
+int* live_tables(uint16_t* qcut, int Nx, int Ny) {
+  return (int*)(qcut + ((size_t)Nx * Ny + 7) / 8 * 8);
+}
 
 std::mutex g_mutex;
 DeviceSlot g_slots[kMaxDevices];
 uint16_t g_host_qcut[kQcutWords * 8];
+// the cut-off slots also hold the list of live blocks and the row cut-offs: an
+// extent is at least 8, so the cut-offs (Nx Ny <= kMaxPoints / 5 of 2 bytes),
+// the blocks (at most Ny Mz <= kMaxPoints / 8 of 4 bytes) and Ny rows fit
+static_assert(kMaxPoints / 5 * 2 + (kMaxPoints / 8) * 4 + kMaxExtent * 2 + 64 <=
+                  kQcutWords * 16, "tables in the cut-off slots");
 double g_host_tw[3][2 * kMaxExtent];
 
 }  // namespace
@@ -118,6 +133,17 @@ extern "C" ns3d_status ns3d_convolution_noalloc(int Nx, int Ny, int Nz, double L
     if (cudaMemcpyAsync(qcut, g_host_qcut, sizeof(uint16_t) * Nx * Ny, cudaMemcpyHostToDevice,
                         st) != cudaSuccess)
       return NS3D_ERR_CUDA;
+    const LiveTables lt = ns3d_detail::build_live(Nx, Ny, Mz, g_host_qcut);
+    const size_t n = lt.live.size();
+    int* live = live_tables(qcut, Nx, Ny);
+    if (cudaMemcpyAsync(live, lt.live.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st) !=
+            cudaSuccess ||
+        cudaMemcpyAsync(live + n, lt.ycut.data(), sizeof(uint16_t) * Ny, cudaMemcpyHostToDevice,
+                        st) != cudaSuccess)
+      return NS3D_ERR_CUDA;
+    slot.Zc = lt.Zc;
+    slot.Zp = lt.Zp;
+    slot.nlive = (int)n;
     // the host staging arrays are reused by the next refresh
     if (cudaStreamSynchronize(st) != cudaSuccess) return NS3D_ERR_CUDA;
     slot.Nx = Nx; slot.Ny = Ny; slot.Nz = Nz;
@@ -130,6 +156,11 @@ extern "C" ns3d_status ns3d_convolution_noalloc(int Nx, int Ny, int Nz, double L
   g.kfy = 2.0 * M_PI / Ly;
   g.kfz = 2.0 * M_PI / Lz;
   g.inv_vol = 1.0 / (1.0 * Nx * Ny * Nz);
+  g.Zc = slot.Zc;
+  g.Zp = slot.Zp;
+  g.nlive = slot.nlive;
+  g.live = live_tables(qcut, Nx, Ny);
+  g.ycut = (const uint16_t*)(g.live + slot.nlive);
 
   // carve A, B, C, D, E (3 components each) out of the fixed array; every
   // entry is written before it is read, so nothing needs clearing

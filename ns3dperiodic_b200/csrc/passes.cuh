@@ -65,7 +65,27 @@ struct PassGeom {
   // bulk-copy form, 3 / 4 the default / alternative points per thread with
   // the reversed radix schedule (x / y families inv_x, inv_y, fwd_y).
   int tile[4];
+  // What the 2/3 mask leaves of the inverse transforms' input (build_live):
+  // Zc kz modes (every mode l >= Zc is masked on every line), per y row the
+  // ycut[y] leading modes that survive for some kx, and the nlive blocks of 8
+  // consecutive z that hold a surviving x line (y << 16 | z of the first).
+  // Everything outside is zero through inv_x and inv_y, so the passes neither
+  // compute, store nor read it, and their scratch (A..E) is compact:
+  // [Nx][Ny][Zp], Zp = Zc rounded up to whole 128-byte blocks of 8 FP64
+  // elements where that fits Mz, so that every row of the x / y passes'
+  // scratch starts on a 128-byte boundary.  Per launch on a B200 at 256^3 FP64 (whole
+  // lines at row stride Mz / the mask's lines at row stride Mz, misaligned /
+  // this layout): inv_x 217 / 177 / 173 us, inv_y 448 / 335 / 267, z 450 /
+  // 457 / 403; the RK3 step 4.84 -> 3.96 ms.
+  int Zc, Zp;
+  int nlive;
+  const int* live;
+  const uint16_t* ycut;
 };
+// kz modes of an Nz-point line that can survive the mask (l / Mz < 2/3), at most
+__host__ __device__ constexpr int zc_max(int nz) { return (2 * (nz / 2 + 1)) / 3 + 1; }
+// ... and at least (the two differ where l / Mz = 2/3 exactly, which rounding decides)
+__host__ __device__ constexpr int zc_min(int nz) { return (2 * (nz / 2 + 1) - 1) / 3 + 1; }
 enum TileFamily { kTileInvX = 0, kTileInvY = 1, kTileFwdY = 2, kTileFwdX = 3 };
 __host__ __device__ __forceinline__ int nbatch(const PassGeom& g) {
   return g.batch > 1 ? g.batch : 1;
@@ -233,18 +253,19 @@ struct PassSmem {
 
 template <int NX>
 __device__ __forceinline__ uint32_t mask_bits(const uint16_t* __restrict__ qcut, int Ny, int y,
-                                              int z, int L, bool valid, int t, int T, int P) {
+                                              int z, bool valid, int t, int T, int P) {
   uint32_t keep = 0;
   for (int s = 0; s < P; ++s) {
     const int x = t + T * s;
-    const bool k = valid && z < (int)__ldg(qcut + x * Ny + y) && !(x == 0 && L == 0);
+    const bool k = valid && z < (int)__ldg(qcut + x * Ny + y) && (x | y | z) != 0;
     keep |= (uint32_t)k << s;
   }
   return keep;
 }
 
 // ---------------------------------------------------------------------------
-// inv_x: lines along x, batch L = y*Mz + z (contiguous), NF = 3 or 6 fields
+// inv_x: lines along x at the (y, z) the mask keeps, NF = 3 or 6 fields; reads
+// the state [Nx][Ny][Mz], writes the compact scratch [Nx][Ny][Zp]
 // ---------------------------------------------------------------------------
 template <int NF, typename C = double2>
 struct InvXArgs {
@@ -269,47 +290,44 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_x_kernel(InvXArg
   LM::get(li, t);
   C* sbuf = S::sbuf(dsm, li);
   double2* pf = S::pf(dsm);
-  const int nlines = g.Ny * g.Mz;               // lines of one instance
-  const int tlines = nlines * nbatch(g);        // lines of all instances
+  const int nlines = g.Ny * g.Mz;       // x stride of the state
+  const int olines = g.Ny * g.Zp;       // x stride of the scratch
+  // only the blocks of 8 lines with a mode inside the mask: about 0.62 of the lines
+  const int tlines = 8 * g.nlive * nbatch(g);
   const int groups = (tlines + LM::LPC - 1) / LM::LPC;
-  // line G of the batch: instance G / nlines, line G % nlines of it
-  auto line_off = [&](int G) -> size_t {
-    const int b = G / nlines;
-    return (size_t)b * NX * nlines + (size_t)(G - b * nlines);
+  // Line G: block G / 8 of the batch's live blocks.  Sets its elements at
+  // x = 0 in the state and the scratch, the surviving modes, and whether it exists.
+  auto line = [&](int G, size_t& in, size_t& out, uint32_t& keep) -> bool {
+    bool valid = G < tlines;
+    const int blk = valid ? G >> 3 : 0;
+    const int inst = blk / g.nlive;
+    const int e = __ldg(g.live + (blk - inst * g.nlive));
+    const int y = e >> 16;
+    int z = (e & 0xffff) + (G & 7);
+    valid = valid && z < g.Zp;
+    z = valid ? z : 0;
+    in = (size_t)inst * NX * nlines + (size_t)(y * g.Mz + z);
+    out = (size_t)inst * NX * olines + (size_t)(y * g.Zp + z);
+    keep = mask_bits<NX>(a.qcut, g.Ny, y, z, valid, t, T, P);
+    return valid;
   };
-  // each CTA takes a contiguous range of groups, so neighbouring lines (which
-  // share partially covered 32-byte sectors) are handled back to back
+  // (a CTA handles one group unless NS3D_SCHED says otherwise)
   const GroupRange gr = group_range(groups);
   const int g_end = gr.end;
   int grp = gr.grp;
   if (grp >= g_end) return;  // uniform across the CTA
   uint32_t keep;             // bit s: mode (t + T s, y, z) survives the 2/3 mask
-  {
-    const int G = grp * LM::LPC + li;
-    const bool valid = G < tlines;
-    const int Gc = valid ? G : 0;
-    const int Lc = Gc % nlines;
-    const int y = Lc / g.Mz, z = Lc - y * g.Mz;
-    keep = mask_bits<NX>(a.qcut, g.Ny, y, z, Lc, valid, t, T, P);
-    issue_line<P, T>(pf, a.in[0], line_off(Gc), (size_t)nlines, t, keep);
-    cp_async_commit();
-  }
+  size_t off, out;           // the line's elements at x = 0
+  bool valid = line(grp * LM::LPC + li, off, out, keep);
+  issue_line<P, T>(pf, a.in[0], off, (size_t)nlines, t, keep);
+  cp_async_commit();
   int ub = 0;
   for (; grp < g_end; grp += gr.step) {
-    const int G = grp * LM::LPC + li;
-    const bool valid = G < tlines;
-    const int Gc = valid ? G : 0;
-    const size_t off = line_off(Gc);
     const int gn = grp + gr.step;
-    const int Gn = gn * LM::LPC + li;
-    const bool validn = Gn < tlines;
-    const int Gnc = validn ? Gn : 0;
-    const int Lnc = Gnc % nlines;
     uint32_t keep_next = 0;
-    if (gn < g_end) {
-      const int yn = Lnc / g.Mz, zn = Lnc - yn * g.Mz;
-      keep_next = mask_bits<NX>(a.qcut, g.Ny, yn, zn, Lnc, validn, t, T, P);
-    }
+    size_t off_next = 0, out_next = 0;
+    bool valid_next = false;
+    if (gn < g_end) valid_next = line(gn * LM::LPC + li, off_next, out_next, keep_next);
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
       const double2* cur = pf + ub * (P * kThreads);
@@ -317,7 +335,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_x_kernel(InvXArg
       if (f + 1 < NF) {
         issue_line<P, T>(nxt, a.in[f + 1], off, (size_t)nlines, t, keep);
       } else if (gn < g_end) {
-        issue_line<P, T>(nxt, a.in[0], line_off(Gnc), (size_t)nlines, t, keep_next);
+        issue_line<P, T>(nxt, a.in[0], off_next, (size_t)nlines, t, keep_next);
       }
       cp_async_commit();
       cp_async_wait<1>();
@@ -328,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_x_kernel(InvXArg
       F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
       if (valid) {
 #pragma unroll
-        for (int s = 0; s < P; ++s) a.A[f][off + (size_t)(t + T * s) * nlines] = v[s];
+        for (int s = 0; s < P; ++s) a.A[f][out + (size_t)(t + T * s) * olines] = v[s];
       }
 #pragma unroll
       for (int s = 0; s < P; ++s) {
@@ -339,17 +357,30 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_x_kernel(InvXArg
       F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
       if (valid) {
 #pragma unroll
-        for (int s = 0; s < P; ++s) a.B[f][off + (size_t)(t + T * s) * nlines] = v[s];
+        for (int s = 0; s < P; ++s) a.B[f][out + (size_t)(t + T * s) * olines] = v[s];
       }
       ub ^= 1;
     }
     keep = keep_next;
+    off = off_next;
+    out = out_next;
+    valid = valid_next;
   }
   cp_async_wait<0>();
 }
 
+// Rows y = t + T s (bit s) of the y line at mode z that inv_x wrote: the others
+// are zero by the mask and hold nothing.
+__device__ __forceinline__ uint32_t row_bits(const uint16_t* __restrict__ ycut, int z, bool valid,
+                                             int t, int T, int P) {
+  uint32_t keep = 0;
+  for (int s = 0; s < P; ++s) keep |= (uint32_t)(valid && z < (int)__ldg(ycut + t + T * s)) << s;
+  return keep;
+}
+
 // ---------------------------------------------------------------------------
-// inv_y: lines along y, batch b = x*Mz + z, base = x*Ny*Mz + z, stride Mz
+// inv_y: lines along y of the compact scratch, batch b = x*Zp + z,
+// base = x*Ny*Zp + z, stride Zp
 // ---------------------------------------------------------------------------
 struct InvYMaps;
 template <int NF, typename Cx = double2>
@@ -380,34 +411,37 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArg
   LM::get(li, t);
   C* sbuf = S::sbuf(dsm, li);
   C* pf = S::pf(dsm);
-  const int nb = g.Nx * g.Mz;
+  const int nb = g.Nx * g.Zp;
   const int groups = (nb + LM::LPC - 1) / LM::LPC;
-  const size_t stride = (size_t)g.Mz;
+  const size_t stride = (size_t)g.Zp;
   const GroupRange gr = group_range(groups);
   const int g_end = gr.end;
   int grp = gr.grp;
   if (grp >= g_end) return;
-  auto line_base = [&](int gidx) -> size_t {
+  auto line_base = [&](int gidx, uint32_t& keep) -> size_t {
     const int b = gidx * LM::LPC + li;
-    const int bc = b < nb ? b : 0;
-    const int x = bc / g.Mz, z = bc - x * g.Mz;
-    return (size_t)x * g.Ny * g.Mz + z;
+    const bool valid = b < nb;
+    const int bc = valid ? b : 0;
+    const int x = bc / g.Zp, z = bc - x * g.Zp;
+    keep = row_bits(g.ycut, z, valid, t, T, P);
+    return (size_t)x * g.Ny * g.Zp + z;
   };
-  issue_line<P, T>(pf, a.A[0], line_base(grp), stride, t);
+  uint32_t keep, keep_next = 0;  // rows inside the mask
+  size_t base = line_base(grp, keep), basen = 0;
+  issue_line<P, T>(pf, a.A[0], base, stride, t, keep);
   cp_async_commit();
   int ub = 0;
   for (; grp < g_end; grp += gr.step) {
     const bool valid = grp * LM::LPC + li < nb;
-    const size_t base = line_base(grp);
     const int gn = grp + gr.step;
-    const size_t basen = line_base(gn < g_end ? gn : grp);
-#pragma unroll
+    if (gn < g_end) basen = line_base(gn, keep_next);
+#pragma unroll 1  // one copy of the three transforms: nine (18) outgrow the instruction cache
     for (int f = 0; f < NF; ++f) {
       // unit A[f] -> C[f] = IFFT_y A, D[f] = IFFT_y(i ky A)
       {
         const C* cur = pf + ub * (P * kThreads);
         C* nxt = pf + (ub ^ 1) * (P * kThreads);
-        issue_line<P, T>(nxt, a.B[f], base, stride, t);
+        issue_line<P, T>(nxt, a.B[f], base, stride, t, keep);
         cp_async_commit();
         cp_async_wait<1>();
         C v[P];
@@ -436,9 +470,9 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArg
         const C* cur = pf + ub * (P * kThreads);
         C* nxt = pf + (ub ^ 1) * (P * kThreads);
         if (f + 1 < NF) {
-          issue_line<P, T>(nxt, a.A[f + 1], base, stride, t);
+          issue_line<P, T>(nxt, a.A[f + 1], base, stride, t, keep);
         } else if (gn < g_end) {
-          issue_line<P, T>(nxt, a.A[0], basen, stride, t);
+          issue_line<P, T>(nxt, a.A[0], basen, stride, t, keep_next);
         }
         cp_async_commit();
         cp_async_wait<1>();
@@ -453,6 +487,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArg
         ub ^= 1;
       }
     }
+    base = basen;
+    keep = keep_next;
   }
   cp_async_wait<0>();
 }
@@ -467,8 +503,9 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArg
 // one x plane, all Ny samples - with one instruction per 256 samples, into a
 // ring of NST shared-memory slots whose completions are counted on
 // mbarriers; the other threads only wait and read.  A group never straddles
-// two x planes: a plane has ceil(Mz / LPC) groups, and the lines past Mz of
-// its last group are filled with zeros by the copy and not stored.  In a
+// two x planes: a plane has ceil(Zp / LPC) groups, and the lines past Zp of
+// its last group are filled with zeros by the copy and not stored.  The rows
+// outside the mask, which inv_x does not write, are read as zeros.  In a
 // slot, sample y of line li sits at y * LPC + li (the box's own order), so
 // the lanes of a load (consecutive li, then t) read consecutive 16-byte
 // words.  A slot is refilled only after every thread has passed the CTA
@@ -484,7 +521,7 @@ constexpr int tma_box_y(int ny, int b = 256) {
   return b <= 1 ? 1 : (ny % b == 0 ? b : tma_box_y(ny, b - 1));
 }
 
-// Tensor maps of one pass: A_f at 2f, B_f at 2f + 1.  Dimensions (2 Mz
+// Tensor maps of one pass: A_f at 2f, B_f at 2f + 1.  Dimensions (2 Zp
 // doubles, Ny, planes), box (2 LPC, tma_box_y(Ny), 1).
 struct alignas(64) InvYMaps {
   CUtensorMap map[6];
@@ -538,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
   int li, t;
   LM::get(li, t);
   double2* sbuf = (double2*)(dsm + S::SBUF_OFF) + li * S::STRIDE;
-  const int gpp = (g.Mz + LPC - 1) / LPC;  // groups per x plane
+  const int gpp = (g.Zp + LPC - 1) / LPC;  // groups per x plane
   const int groups = g.Nx * gpp;
   const GroupRange gr = group_range(groups);
   if (gr.grp >= gr.end) return;  // uniform across the CTA
@@ -572,6 +609,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
   }
   F::load_tw(tw_s, a.tw);  // ends with a CTA barrier: the barriers are initialised
   if (*bad) return;        // uniform: read after the barrier
+  uint32_t keep = 0;       // the group's rows inside the mask
   for (int k = 0; k < nunits; ++k) {
     if (threadIdx.x == 0 && unseen == nunits && k + NST - 1 < nunits) {
       fence_proxy_async_smem();  // the slot's earlier reads (generic proxy) come first
@@ -584,12 +622,16 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
     const int gi = k / UPG, j = k - gi * UPG, f = j >> 1;
     const int grp = gr.grp + gi * gr.step;
     const int x = grp / gpp, z = (grp - x * gpp) * LPC + li;
-    const bool valid = z < g.Mz;
-    const size_t base = (size_t)x * g.Ny * g.Mz + (valid ? z : 0);
-    const size_t stride = (size_t)g.Mz;
+    const bool valid = z < g.Zp;
+    const size_t base = (size_t)x * g.Ny * g.Zp + (valid ? z : 0);
+    const size_t stride = (size_t)g.Zp;
+    if (j == 0) keep = row_bits(g.ycut, z, valid, t, T, P);
+    auto sample = [&](int s) {
+      return (keep >> s) & 1u ? cur[(t + T * s) * LPC] : make_double2(0.0, 0.0);
+    };
     double2 v[P];
 #pragma unroll
-    for (int s = 0; s < P; ++s) v[s] = cur[(t + T * s) * LPC];
+    for (int s = 0; s < P; ++s) v[s] = sample(s);
     F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
     if ((j & 1) == 0) {
       // unit A_f -> C_f = IFFT_y A, D_f = IFFT_y(i ky A)
@@ -599,7 +641,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
       }
 #pragma unroll
       for (int s = 0; s < P; ++s) {
-        const double2 u = cur[(t + T * s) * LPC];
+        const double2 u = sample(s);
         const double ky = g.kfy * (double)signed_idx(t + T * s, NY);
         v[s] = make_double2(-u.y * ky, u.x * ky);
       }
@@ -621,7 +663,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
 }
 
 // ---------------------------------------------------------------------------
-// z pass: lines along z (contiguous), batch b = x*Ny + y, base = b*Mz
+// z pass: lines along z (contiguous), batch b = x*Ny + y; input at b*Zp of the
+// compact scratch, product spectra at b*Mz
 // ---------------------------------------------------------------------------
 template <int NF, typename Cx = double2>
 struct ZArgs {
@@ -650,49 +693,79 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void* p, unsigned bytes) 
 #define NS3D_Z_L2PF 2
 #endif
 
-// L2 prefetch of a CTA's `nv` consecutive z lines (from element run0) of one
-// field: one contiguous run, trimmed to 16-byte boundaries inside it (FP32
-// rows of an odd Mz start at 8-byte offsets).
+// L2 prefetch of one z line's kept modes (elements base .. base + Zc - 1),
+// trimmed to 16-byte boundaries (FP32 rows of an odd Mz start at 8-byte
+// offsets).  One run per line and field: a run over the CTA's consecutive
+// lines would also fetch the masked third of every line.
 template <typename C>
-__device__ __forceinline__ void prefetch_z_run(const C* f, size_t run0, int nv, int Mz) {
-  const uintptr_t a = (uintptr_t)(f + run0) & ~(uintptr_t)15;
-  const uintptr_t e = (uintptr_t)(f + run0 + (size_t)nv * Mz) & ~(uintptr_t)15;
+__device__ __forceinline__ void prefetch_z_line(const C* f, size_t base, int Zc) {
+  const uintptr_t a = (uintptr_t)(f + base) & ~(uintptr_t)15;
+  const uintptr_t e = (uintptr_t)(f + base + (size_t)Zc) & ~(uintptr_t)15;
   if (e > a) prefetch_l2_bulk((const void*)a, (unsigned)(e - a));
 }
 
-// The CTA's runs of one z pass: lines b0 .. b0 + nv - 1 of every field.
+// One z line of a CTA's thread: its first element, the kept modes, and
+// whether this thread asks for the line's prefetches (the line's t = 0).
 struct ZRun {
-  size_t run0;
-  int nv, Mz;
+  size_t base;
+  int Zc;
+  bool ask;
 };
-__device__ __forceinline__ ZRun z_run(int lpc, int nb, int Mz) {
-  const int b0 = blockIdx.x * lpc;
-  return {(size_t)b0 * Mz, nb - b0 < lpc ? nb - b0 : lpc, Mz};
+// Whether the pass's nine FP64 fields are larger than what L2 keeps of them
+// between inv_y and this pass (126 MB): below, the prefetches only cost issue
+// slots (32^3: 18.6 us a launch without them, 24.4 us with).
+__device__ __forceinline__ bool z_prefetch(const PassGeom& g) {
+  return (size_t)g.Nx * g.Ny * g.Zp * (9 * sizeof(double2)) > ((size_t)64 << 20);
 }
-// the next transform's two input runs (threads 0 and 1 ask the bulk-copy unit)
+// the next transform's two input lines
 template <typename C>
 __device__ __forceinline__ void prefetch_z_pair(const C* f1, const C* f2, const ZRun& r) {
-  if (NS3D_Z_L2PF == 0) return;
-  if (threadIdx.x == 0) prefetch_z_run(f1, r.run0, r.nv, r.Mz);
-  if (threadIdx.x == 1 && f2 != f1) prefetch_z_run(f2, r.run0, r.nv, r.Mz);
+  if (NS3D_Z_L2PF == 0 || !r.ask) return;
+  prefetch_z_line(f1, r.base, r.Zc);
+  if (f2 != f1) prefetch_z_line(f2, r.base, r.Zc);
+}
+
+// whether every thread's sample s (k = t + T s) is a kept mode
+template <int NZ, int T>
+__host__ __device__ constexpr bool z_live(int s) {
+  const int a = T * s, b = T * s + T - 1;  // k = a .. b
+  const int qa = a > NZ / 2 ? NZ - a : a, qb = b > NZ / 2 ? NZ - b : b;
+  const bool mid = a <= NZ / 2 && b >= NZ / 2;
+  return !mid && (qa > qb ? qa : qb) < zc_min(NZ);
+}
+
+// whether sample s of every thread of an NZ-point line in T threads (k = t +
+// T s) lies above the mask's kz modes in both halves of the spectrum: about a
+// quarter of the samples, known at compile time
+template <int NZ, int T>
+__host__ __device__ constexpr bool z_dead(int s) {
+  const int lo = T * s, hi = NZ - (T * s + T - 1);  // the smallest q of each half
+  return (lo < hi ? lo : hi) >= zc_max(NZ);
 }
 
 // Load W[k] = H(X1)[k] + i H(X2)[k] for positions k = t + T s, where H is the
 // Hermitian extension of a z half-line (H[0], H[N/2] keep only real parts),
-// X = line (optionally times i kz).
+// X = line (optionally times i kz).  Modes from Zc up are zero (the mask).
 template <int NZ, int P, bool IK1, bool IK2, typename C>
 __device__ __forceinline__ void load_pair(C (&w)[P], const C* __restrict__ f1,
                                           const C* __restrict__ f2, size_t base, int t,
-                                          RealOf<C> kfz) {
+                                          RealOf<C> kfz, int Zc) {
   using Rt = RealOf<C>;
   constexpr int T = NZ / P;
 #pragma unroll
   for (int s = 0; s < P; ++s) {
+    if (z_dead<NZ, T>(s)) {
+      w[s] = mkc<C>((Rt)0, (Rt)0);
+      continue;
+    }
     const int k = t + T * s;
     const bool upper = k > NZ / 2;
     const int q = upper ? NZ - k : k;
-    C c1 = __ldg(f1 + base + q);
-    C c2 = __ldg(f2 + base + q);
+    C c1 = mkc<C>((Rt)0, (Rt)0), c2 = c1;
+    if (z_live<NZ, T>(s) || q < Zc) {
+      c1 = __ldg(f1 + base + q);
+      c2 = __ldg(f2 + base + q);
+    }
     const Rt kz = kfz * (Rt)q;
     if constexpr (IK1) c1 = mkc<C>(-c1.y * kz, c1.x * kz);
     if constexpr (IK2) c2 = mkc<C>(-c2.y * kz, c2.x * kz);
@@ -772,13 +845,13 @@ __device__ __forceinline__ void uv_component(Rt (&q)[P], int i, const ZArgs<6, C
   C w[P];
   // (d_x u_i, d_y u_i)
   prefetch_z_pair(a.C[i], a.E[3 + i], run);
-  load_pair<NZ, P, false, false>(w, a.E[i], a.D[i], base, t, kfz);
+  load_pair<NZ, P, false, false>(w, a.E[i], a.D[i], base, t, kfz, run.Zc);
   F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
   for (int s = 0; s < P; ++s) q[s] = vx[s] * (w[s].x * sc) + vy[s] * (w[s].y * sc);
   // (d_z u_i, d_x v_i)
   prefetch_z_pair(a.D[3 + i], a.C[3 + i], run);
-  load_pair<NZ, P, true, false>(w, a.C[i], a.E[3 + i], base, t, kfz);
+  load_pair<NZ, P, true, false>(w, a.C[i], a.E[3 + i], base, t, kfz, run.Zc);
   F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
   for (int s = 0; s < P; ++s) {
@@ -787,7 +860,7 @@ __device__ __forceinline__ void uv_component(Rt (&q)[P], int i, const ZArgs<6, C
   }
   // (d_y v_i, d_z v_i)
   if (i < 2) prefetch_z_pair(a.E[i + 1], a.D[i + 1], run);
-  load_pair<NZ, P, false, true>(w, a.D[3 + i], a.C[3 + i], base, t, kfz);
+  load_pair<NZ, P, false, true>(w, a.D[3 + i], a.C[3 + i], base, t, kfz, run.Zc);
   F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
   for (int s = 0; s < P; ++s) q[s] = q[s] + (uy[s] * (w[s].x * sc) + uz[s] * (w[s].y * sc));
@@ -807,11 +880,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<U
   const int nb = g.Nx * g.Ny;
   const int b = blockIdx.x * LM::LPC + li;
   const bool valid = b < nb;
-  const size_t base = (size_t)(valid ? b : 0) * g.Mz;
+  const size_t base = (size_t)(valid ? b : 0) * g.Zp;   // C, D, E
+  const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
   C* sbuf = sbuf_all[li];
   const Rt sc = (Rt)g.inv_vol;
   const Rt kfz = (Rt)g.kfz;
-  const ZRun run = z_run(LM::LPC, nb, g.Mz);  // one transform ahead into L2
+  const ZRun run{base, g.Zc, valid && t == 0 && z_prefetch(g)};  // one transform ahead into L2
   C w[P];
   Rt ux[P], uy[P], uz[P], q0[P], q1[P], q2[P];
   if constexpr (!UV) {
@@ -819,19 +893,19 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<U
     // are live at any time.
     // (u_x, u_y)
     prefetch_z_pair(a.C[2], a.C[2], run);
-    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz);
+    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s) { ux[s] = w[s].x * sc; uy[s] = w[s].y * sc; }
     // (u_z, d_z u_z) from one field
     prefetch_z_pair(a.E[2], a.D[2], run);
-    load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz);
+    load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s) { uz[s] = w[s].x * sc; q2[s] = w[s].y * sc; }
     // Q_z = u_x d_x u_z + u_y d_y u_z + u_z d_z u_z  (calc_vels_nabla_vels)
     prefetch_z_pair(a.E[0], a.D[0], run);
-    load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz);
+    load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s)
@@ -844,21 +918,21 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<U
 #pragma unroll
       for (int s = 0; s < P; ++s) {
         const int k = t + T * s;
-        if (k <= NZ / 2) a.Qh[2][base + k] = w[s];
+        if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
       }
     }
     // (d_z u_x, d_z u_y)
-    load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz);
+    load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; q1[s] = w[s].y * sc; }
     prefetch_z_pair(a.E[1], a.D[1], run);
-    load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz);
+    load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s)
       q0[s] = ux[s] * (w[s].x * sc) + uy[s] * (w[s].y * sc) + uz[s] * q0[s];
-    load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz);
+    load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s)
@@ -867,23 +941,23 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<U
 #pragma unroll
     for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
     F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-    store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], base, valid);
+    store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
     return;
   } else {
     // B(u,v)_i = (v.grad) u_i + (u.grad) v_i; fields 0..2 are u, 3..5 are v
     Rt vx[P], vy[P], vz[P];
     prefetch_z_pair(a.C[2], a.C[3], run);
-    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz);
+    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s) { ux[s] = w[s].x * sc; uy[s] = w[s].y * sc; }
     prefetch_z_pair(a.C[4], a.C[5], run);
-    load_pair<NZ, P, false, false>(w, a.C[2], a.C[3], base, t, kfz);
+    load_pair<NZ, P, false, false>(w, a.C[2], a.C[3], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s) { uz[s] = w[s].x * sc; vx[s] = w[s].y * sc; }
     prefetch_z_pair(a.E[0], a.D[0], run);
-    load_pair<NZ, P, false, false>(w, a.C[4], a.C[5], base, t, kfz);
+    load_pair<NZ, P, false, false>(w, a.C[4], a.C[5], base, t, kfz, run.Zc);
     F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
 #pragma unroll
     for (int s = 0; s < P; ++s) { vy[s] = w[s].x * sc; vz[s] = w[s].y * sc; }
@@ -895,7 +969,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<U
 #pragma unroll
   for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
   F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], base, valid);
+  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
 #pragma unroll
   for (int s = 0; s < P; ++s) w[s] = mkc<C>(q2[s], (Rt)0);
   F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
@@ -903,7 +977,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<U
 #pragma unroll
     for (int s = 0; s < P; ++s) {
       const int k = t + T * s;
-      if (k <= NZ / 2) a.Qh[2][base + k] = w[s];
+      if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
     }
   }
 }
@@ -985,17 +1059,18 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel_st(ZArgs<3, C> a
   const int nb = g.Nx * g.Ny;
   const int b = blockIdx.x * LM::LPC + li;
   const bool valid = b < nb;
-  const size_t base = (size_t)(valid ? b : 0) * g.Mz;
+  const size_t base = (size_t)(valid ? b : 0) * g.Zp;   // C, D, E
+  const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
   C* sbuf = (C*)(dsm + S::SBUF_OFF) + li * F::BUF;
   Rt* stash = (Rt*)(dsm + S::ST_OFF) + threadIdx.x;
-  // the CTA's lines are consecutive: each field's input is one run
-  const ZRun run = z_run(LM::LPC, nb, g.Mz);
+  const ZRun run{base, g.Zc, valid && t == 0 && z_prefetch(g)};
   const C* order[9] = {a.C[0], a.C[1], a.C[2], a.E[2], a.D[2], a.E[0], a.D[0], a.E[1], a.D[1]};
   auto pf = [&](int i) {
-    if (NS3D_Z_L2PF != 0 && i < 9) prefetch_z_run(order[i], run.run0, run.nv, run.Mz);
+    if (NS3D_Z_L2PF != 0 && run.ask) prefetch_z_line(order[i], run.base, run.Zc);
   };
-  if (NS3D_Z_L2PF == 1 && threadIdx.x < 9) pf(threadIdx.x);
-  if (NS3D_Z_L2PF == 2 && threadIdx.x < 2) pf(threadIdx.x);  // C0, C1
+  if (NS3D_Z_L2PF == 1)
+    for (int i = 0; i < 9; ++i) pf(i);
+  if (NS3D_Z_L2PF == 2) { pf(0); pf(1); }  // C0, C1
   auto ux = [&](int s) -> Rt& { return stash[(0 * P + s) * kThreads]; };
   auto uy = [&](int s) -> Rt& { return stash[(1 * P + s) * kThreads]; };
   auto uz = [&](int s) -> Rt& { return stash[(2 * P + s) * kThreads]; };
@@ -1049,21 +1124,21 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel_st(ZArgs<3, C> a
     }
   };
   // (u_x, u_y)
-  if (NS3D_Z_L2PF == 2 && threadIdx.x == 0) pf(2);  // C2
-  load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz);
+  if (NS3D_Z_L2PF == 2) pf(2);  // C2
+  load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
   F::template run<+1, PW>(w, t, sbuf, tw_s);
   park(0, [&](int s) { return w[s].x * sc; });
   park(1, [&](int s) { return w[s].y * sc; });
   // (u_z, d_z u_z); q0 accumulates Q_z first
-  if (NS3D_Z_L2PF == 2 && threadIdx.x < 2) pf(3 + threadIdx.x);  // E2, D2
-  load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz);
+  if (NS3D_Z_L2PF == 2) { pf(3); pf(4); }  // E2, D2
+  load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz, run.Zc);
   F::template run<+1, PW>(w, t, sbuf, tw_s);
   park(2, [&](int s) { return w[s].x * sc; });
 #pragma unroll
   for (int s = 0; s < P; ++s) q0[s] = w[s].y * sc;
   // Q_z = u_x d_x u_z + u_y d_y u_z + u_z d_z u_z
-  if (NS3D_Z_L2PF == 2 && threadIdx.x < 2) pf(5 + threadIdx.x);  // E0, D0
-  load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz);
+  if (NS3D_Z_L2PF == 2) { pf(5); pf(6); }  // E0, D0
+  load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz, run.Zc);
   F::template run<+1, PW>(w, t, sbuf, tw_s);
   product(q0);
   // R2C of Q_z alone
@@ -1074,26 +1149,26 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel_st(ZArgs<3, C> a
 #pragma unroll
     for (int s = 0; s < P; ++s) {
       const int k = t + T * s;
-      if (k <= NZ / 2) a.Qh[2][base + k] = w[s];
+      if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
     }
   }
   // (d_z u_x, d_z u_y)
-  load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz);
+  load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
   F::template run<+1, PW>(w, t, sbuf, tw_s);
 #pragma unroll
   for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; q1[s] = w[s].y * sc; }
-  if (NS3D_Z_L2PF == 2 && threadIdx.x < 2) pf(7 + threadIdx.x);  // E1, D1
-  load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz);
+  if (NS3D_Z_L2PF == 2) { pf(7); pf(8); }  // E1, D1
+  load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz, run.Zc);
   F::template run<+1, PW>(w, t, sbuf, tw_s);
   product(q0);
-  load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz);
+  load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz, run.Zc);
   F::template run<+1, PW>(w, t, sbuf, tw_s);
   product(q1);
   // R2C of (Q_x, Q_y) packed
 #pragma unroll
   for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
   F::template run<-1, PW>(w, t, sbuf, tw_s);
-  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], base, valid);
+  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
   if constexpr (TM) {
     // every thread's TMEM reads have completed (waited); free the columns
     tmem_fence_before_sync();

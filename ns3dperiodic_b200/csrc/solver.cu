@@ -1,5 +1,6 @@
 // Host side of the C ABI (include/ns3d.h): handle, scratch, RHS pipelines and
 // the steppers of Source/RK_time_step.cu rebuilt on the fused pass kernels.
+#include <algorithm>
 #include <array>
 #include <cmath>
 #include <cstdio>
@@ -96,6 +97,24 @@ bool build_mask_cutoff(int Nx, int Ny, int Nz, double Lx, double Ly, double Lz,
     }
   }
   return true;
+}
+
+LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut) {
+  LiveTables t;
+  t.ycut.assign(Ny, 0);
+  for (int j = 0; j < Nx; ++j)
+    for (int k = 0; k < Ny; ++k) t.ycut[k] = std::max(t.ycut[k], qcut[(size_t)j * Ny + k]);
+  t.Zc = std::max<int>(1, *std::max_element(t.ycut.begin(), t.ycut.end()));
+  // whole 128-byte blocks where the padded rows still fit the fields' memory
+  t.Zp = t.Zc;
+  for (int a = 8; a > 1; a /= 2)
+    if ((t.Zc + a - 1) / a * a <= Mz) {
+      t.Zp = (t.Zc + a - 1) / a * a;
+      break;
+    }
+  for (int k = 0; k < Ny; ++k)
+    for (int l = 0; l < t.ycut[k]; l += 8) t.live.push_back(k << 16 | l);
+  return t;
 }
 
 bool valid_extents(int Nx, int Ny, int Nz) {
@@ -368,8 +387,8 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // Tensor maps of inv_y's bulk-copy form over the FP64 scratch A_f, B_f (all
-// instances of a batch as x planes).  A field is dims (2 Mz doubles, Ny,
-// planes) with row strides Mz * 16 and Ny * Mz * 16 bytes; a box is
+// instances of a batch as x planes).  A field is dims (2 Zp doubles, Ny,
+// planes) with row strides Zp * 16 and Ny * Zp * 16 bytes; a box is
 // (2 LPC, tma_box_y(Ny), 1).  Any failure leaves the handle without the form
 // (ns3d_set_tiles then refuses tile 2 of the inv_y family).
 void build_inv_y_maps(ns3d_solver* h) {
@@ -382,10 +401,10 @@ void build_inv_y_maps(ns3d_solver* h) {
     bool ok = true;
     for (int f = 0; f < 6 && ok; ++f) {
       const double2* base = (f & 1) ? h->B[f >> 1] : h->A[f >> 1];
-      const cuuint64_t dims[3] = {2ull * (cuuint64_t)h->Mz, (cuuint64_t)h->Ny,
+      const cuuint64_t zp = (cuuint64_t)h->geom.Zp;
+      const cuuint64_t dims[3] = {2ull * zp, (cuuint64_t)h->Ny,
                                   (cuuint64_t)h->Nx * (cuuint64_t)h->batch};
-      const cuuint64_t strides[2] = {16ull * (cuuint64_t)h->Mz,
-                                     16ull * (cuuint64_t)h->Mz * (cuuint64_t)h->Ny};
+      const cuuint64_t strides[2] = {16ull * zp, 16ull * zp * (cuuint64_t)h->Ny};
       const cuuint32_t box[3] = {2u * (cuuint32_t)lpc, (cuuint32_t)ns3d::tma_box_y(h->Ny), 1u};
       const cuuint32_t estr[3] = {1u, 1u, 1u};
       ok = enc(&m->map[f], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, (void*)base, dims, strides, box,
@@ -439,6 +458,21 @@ ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double L
   if ((e = cudaMalloc(&h->qcut, sizeof(uint16_t) * qc.size())) != cudaSuccess)
     return bail(NS3D_ERR_OOM);
   cudaMemcpy(h->qcut, qc.data(), sizeof(uint16_t) * qc.size(), cudaMemcpyHostToDevice);
+  {
+    const LiveTables lt = build_live(Nx, Ny, h->Mz, qc.data());
+    const size_t n = lt.live.size();
+    const size_t bytes = sizeof(int) * n + sizeof(uint16_t) * Ny;
+    if (cudaMalloc(&h->live, bytes) != cudaSuccess) return bail(NS3D_ERR_OOM);
+    uint16_t* yc = reinterpret_cast<uint16_t*>(h->live + n);
+    cudaMemcpy(h->live, lt.live.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
+    cudaMemcpy(yc, lt.ycut.data(), sizeof(uint16_t) * Ny, cudaMemcpyHostToDevice);
+    h->geom.Zc = lt.Zc;
+    h->geom.Zp = lt.Zp;
+    h->geom.nlive = (int)n;
+    h->geom.live = h->live;
+    h->geom.ycut = yc;
+    h->bytes += bytes;
+  }
   const int ext[3] = {Nx, Ny, Nz};
   for (int d = 0; d < 3; ++d) {
     std::vector<double2> t;
@@ -449,7 +483,7 @@ ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double L
   const size_t field = h->nc * (size_t)batch;  // one scratch field of the whole batch
   const size_t base_bytes = sizeof(double2) * field * 21;
   if (cudaMalloc(&h->pool_base, base_bytes) != cudaSuccess) return bail(NS3D_ERR_OOM);
-  h->bytes = base_bytes + sizeof(uint16_t) * qc.size() + sizeof(double2) * (Nx + Ny + Nz);
+  h->bytes += base_bytes + sizeof(uint16_t) * qc.size() + sizeof(double2) * (Nx + Ny + Nz);
   double2* p = h->pool_base;
   for (int i = 0; i < 3; ++i) {
     h->A[i] = p; p += field;
@@ -495,6 +529,7 @@ ns3d_status ns3d_destroy(ns3d_solver* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   drop_graph(h);
   cudaFree(h->qcut);
+  cudaFree(h->live);
   for (auto* t : h->tw) cudaFree(t);
   cudaFree(h->pool_base);
   cudaFree(h->pool_uv);

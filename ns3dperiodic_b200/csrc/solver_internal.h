@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -29,6 +30,7 @@ struct ns3d_solver {
   bool own_stream = false;
   // tables
   uint16_t* qcut = nullptr;
+  int* live = nullptr;  // geom.live and geom.ycut, one allocation
   double2* tw[3] = {};
   // scratch: base pool (21 fields) and tangent pool (18 fields, lazily)
   double2* pool_base = nullptr;
@@ -86,6 +88,13 @@ constexpr int kDiagThreads = 256;
 ns3d_status fail(ns3d_solver* h, ns3d_status s, const std::string& msg);
 ns3d_status cuda_fail(ns3d_solver* h, cudaError_t e, const char* where);
 ns3d_status check_handle(ns3d_solver* h);
+// What the mask (qcut[Nx][Ny], build_mask_cutoff) leaves: the tables of PassGeom.
+struct LiveTables {
+  int Zc = 0, Zp = 0;
+  std::vector<uint16_t> ycut;  // [Ny]
+  std::vector<int> live;       // blocks of 8 lines, y << 16 | z
+};
+LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut);
 // a handle for `batch` instances of one grid (batch = 1: ns3d_create)
 ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double Ly, double Lz,
                           ns3d_solver** out);
