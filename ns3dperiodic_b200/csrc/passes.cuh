@@ -9,9 +9,8 @@
 //   inv_x : u (3)            -> A = IFFT_x(M u), B = IFFT_x(i kx M u)     (M = 2/3 mask)
 //   inv_y : A, B (6)         -> C = IFFT_y A, D = IFFT_y(i ky A), E = IFFT_y B
 //   z     : C, D, E (9)      -> C2R along z (12 real lines = 6 complex IFFTs),
-//                               Q_i = sum_j u_j d_j u_i, odd part, R2C along z
-//                               -> Qh (3) on the planes x = 0 .. Nx/2
-//   fwd_y : Qh (3) in place  -> FFT_y on those planes
+//                               Q_i = sum_j u_j d_j u_i, R2C along z  -> Qh (3)
+//   fwd_y : Qh (3) in place  -> FFT_y
 //   fwd_x : Qh (3), u, ...   -> FFT_x, Re(Qh)=0, Qh(0)=0, Leray, diffusion,
 //                               forcing, RK combination -> new state
 //
@@ -664,7 +663,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
 }
 
 // ---------------------------------------------------------------------------
-// z pass: arguments, loads and prefetches (the kernel follows)
+// z pass: lines along z (contiguous), batch b = x*Ny + y; input at b*Zp of the
+// compact scratch, product spectra at b*Mz
 // ---------------------------------------------------------------------------
 template <int NF, typename Cx = double2>
 struct ZArgs {
@@ -715,7 +715,7 @@ struct ZRun {
 // between inv_y and this pass (126 MB): below, the prefetches only cost issue
 // slots (32^3: 18.6 us a launch without them, 24.4 us with).
 __device__ __forceinline__ bool z_prefetch(const PassGeom& g) {
-  return (size_t)g.Nx * nbatch(g) * g.Ny * g.Zp * (9 * sizeof(double2)) > ((size_t)64 << 20);
+  return (size_t)g.Nx * g.Ny * g.Zp * (9 * sizeof(double2)) > ((size_t)64 << 20);
 }
 // the next transform's two input lines
 template <typename C>
@@ -832,55 +832,192 @@ struct ZLaneMap {  // lanes of one line are adjacent: the line is contiguous in 
   }
 };
 
-// ---------------------------------------------------------------------------
-// z pass: lines along z (contiguous); input at (x*Ny + y)*Zp of the compact
-// scratch, product spectra at (x*Ny + y)*Mz.
-//
-// Lines come in pairs (x, y) and (-x, -y).  The update takes only the
-// imaginary part of the products' spectrum (Re(Qh) = 0,
-// Source/advection_2_3.cu:35-70), which is the transform of the odd part
-// q(r) = (Q(r) - Q(-r)) / 2.  The pair's two thread groups form their own
-// lines' products, swap them through the line buffers, and transform the odd
-// part: the first group (q_x, q_y) packed, the second q_z.  q(-r) = -q(r) then
-// gives every later line from its mirror: only the planes x = 0 .. Nx/2 are
-// stored, fwd_y transforms those, and fwd_x rebuilds the rest of each x line
-// (G(-x) = -conj G(x)).  Half the product spectra's traffic and one of the two
-// forward transforms per line go away; per launch on a B200 at 256^3 FP64
-// (all lines -> their odd part): z 403 -> 421 us (the swap), fwd_y 153 -> 83,
-// fwd_x 283 -> 225, the RK3 step 3.96 -> 3.61 ms.
-//
-// What bounds the pass is its line transforms (FP64 pipe, then the exchanges'
-// shared memory) at the 8 warps per SM that 16 points per thread leave room
-// for.  Each Stockham exchange moves the whole line through shared memory, so
-// 16 points per thread (one exchange at 256) beat 8 (two); the velocities and
-// Q_z do not fit the registers beside the line, so each thread parks its own
-// samples in a private shared-memory slot ([component][s][thread]: the lanes
-// of a warp touch consecutive words, conflict-free); no other thread reads
-// them, so no barrier is needed.  The tangent form parks six velocities and
-// keeps its products in registers (8 points, or 12 for multiples of 3).
-// ---------------------------------------------------------------------------
+// One component of B(u,v)_i = (v.grad) u_i + (u.grad) v_i in the z pass
+// (convolute_2p3_UV, Source/advection_2_3.cu:414-466); 3 paired C2R lines.
+template <int NZ, int P, typename C, typename Rt = RealOf<C>>
+__device__ __forceinline__ void uv_component(Rt (&q)[P], int i, const ZArgs<6, C>& a, size_t base,
+                                             int t, Rt kfz, Rt sc, C* sbuf,
+                                             const C* tw_s, const Rt (&ux)[P],
+                                             const Rt (&uy)[P], const Rt (&uz)[P],
+                                             const Rt (&vx)[P], const Rt (&vy)[P],
+                                             const Rt (&vz)[P], const ZRun& run) {
+  using F = LineFFT<NZ, P>;
+  C w[P];
+  // (d_x u_i, d_y u_i)
+  prefetch_z_pair(a.C[i], a.E[3 + i], run);
+  load_pair<NZ, P, false, false>(w, a.E[i], a.D[i], base, t, kfz, run.Zc);
+  F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) q[s] = vx[s] * (w[s].x * sc) + vy[s] * (w[s].y * sc);
+  // (d_z u_i, d_x v_i)
+  prefetch_z_pair(a.D[3 + i], a.C[3 + i], run);
+  load_pair<NZ, P, true, false>(w, a.C[i], a.E[3 + i], base, t, kfz, run.Zc);
+  F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) {
+    q[s] = q[s] + vz[s] * (w[s].x * sc);
+    q[s] = q[s] + ux[s] * (w[s].y * sc);
+  }
+  // (d_y v_i, d_z v_i)
+  if (i < 2) prefetch_z_pair(a.E[i + 1], a.D[i + 1], run);
+  load_pair<NZ, P, false, true>(w, a.D[3 + i], a.C[3 + i], base, t, kfz, run.Zc);
+  F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) q[s] = q[s] + (uy[s] * (w[s].x * sc) + uz[s] * (w[s].y * sc));
+}
+
 template <int NZ, int P, bool UV, typename C>
-struct ZSmem {
+__global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<UV ? 6 : 3, C> a, PassGeom g) {
+  using F = LineFFT<NZ, P>;
+  using Rt = RealOf<C>;
+  constexpr int T = F::T;
+  using LM = ZLaneMap<T>;
+  __shared__ C tw_s[F::TWLEN];
+  __shared__ C sbuf_all[LM::LPC][F::BUF];
+  F::load_tw(tw_s, a.tw);
+  int li, t;
+  LM::get(li, t);
+  const int nb = g.Nx * g.Ny;
+  const int b = blockIdx.x * LM::LPC + li;
+  const bool valid = b < nb;
+  const size_t base = (size_t)(valid ? b : 0) * g.Zp;   // C, D, E
+  const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
+  C* sbuf = sbuf_all[li];
+  const Rt sc = (Rt)g.inv_vol;
+  const Rt kfz = (Rt)g.kfz;
+  const ZRun run{base, g.Zc, valid && t == 0 && z_prefetch(g)};  // one transform ahead into L2
+  C w[P];
+  Rt ux[P], uy[P], uz[P], q0[P], q1[P], q2[P];
+  if constexpr (!UV) {
+    // Q_z first, so at most five real lines (u_x, u_y, u_z and two products)
+    // are live at any time.
+    // (u_x, u_y)
+    prefetch_z_pair(a.C[2], a.C[2], run);
+    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s) { ux[s] = w[s].x * sc; uy[s] = w[s].y * sc; }
+    // (u_z, d_z u_z) from one field
+    prefetch_z_pair(a.E[2], a.D[2], run);
+    load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s) { uz[s] = w[s].x * sc; q2[s] = w[s].y * sc; }
+    // Q_z = u_x d_x u_z + u_y d_y u_z + u_z d_z u_z  (calc_vels_nabla_vels)
+    prefetch_z_pair(a.E[0], a.D[0], run);
+    load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s)
+      q2[s] = ux[s] * (w[s].x * sc) + uy[s] * (w[s].y * sc) + uz[s] * q2[s];
+    // R2C of Q_z alone
+#pragma unroll
+    for (int s = 0; s < P; ++s) w[s] = mkc<C>(q2[s], (Rt)0);
+    F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+    if (valid) {
+#pragma unroll
+      for (int s = 0; s < P; ++s) {
+        const int k = t + T * s;
+        if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
+      }
+    }
+    // (d_z u_x, d_z u_y)
+    load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; q1[s] = w[s].y * sc; }
+    prefetch_z_pair(a.E[1], a.D[1], run);
+    load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s)
+      q0[s] = ux[s] * (w[s].x * sc) + uy[s] * (w[s].y * sc) + uz[s] * q0[s];
+    load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s)
+      q1[s] = ux[s] * (w[s].x * sc) + uy[s] * (w[s].y * sc) + uz[s] * q1[s];
+    // R2C of (Q_x, Q_y) packed
+#pragma unroll
+    for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
+    F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+    store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
+    return;
+  } else {
+    // B(u,v)_i = (v.grad) u_i + (u.grad) v_i; fields 0..2 are u, 3..5 are v
+    Rt vx[P], vy[P], vz[P];
+    prefetch_z_pair(a.C[2], a.C[3], run);
+    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s) { ux[s] = w[s].x * sc; uy[s] = w[s].y * sc; }
+    prefetch_z_pair(a.C[4], a.C[5], run);
+    load_pair<NZ, P, false, false>(w, a.C[2], a.C[3], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s) { uz[s] = w[s].x * sc; vx[s] = w[s].y * sc; }
+    prefetch_z_pair(a.E[0], a.D[0], run);
+    load_pair<NZ, P, false, false>(w, a.C[4], a.C[5], base, t, kfz, run.Zc);
+    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s) { vy[s] = w[s].x * sc; vz[s] = w[s].y * sc; }
+    uv_component<NZ, P>(q0, 0, a, base, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, run);
+    uv_component<NZ, P>(q1, 1, a, base, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, run);
+    uv_component<NZ, P>(q2, 2, a, base, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, run);
+  }
+  // forward R2C along z: (Q0, Q1) packed, then Q2 alone
+#pragma unroll
+  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
+  F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
+#pragma unroll
+  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q2[s], (Rt)0);
+  F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
+  if (valid) {
+#pragma unroll
+    for (int s = 0; s < P; ++s) {
+      const int k = t + T * s;
+      if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// z pass with the physical velocities stashed in shared memory (the nonlinear
+// term; the tangent form keeps z_kernel).
+//
+// The line transforms are what bound the z pass: each Stockham exchange moves
+// the whole line through shared memory, so at 8 points per thread a 256-point
+// line takes two exchanges per transform (16 per line and pass) and the
+// shared-memory pipe, not HBM, sets the pace.  With 16 points per thread the
+// same transform needs one exchange, but u_x, u_y, u_z, two products and the
+// line no longer fit in registers.  Here each thread parks its own P samples
+// of u_x, u_y, u_z in a private shared-memory slot ([component][s][thread]:
+// the lanes of a warp touch consecutive words, conflict-free) right after
+// their transforms and reads them back for each product; no other thread
+// reads them, so no barrier is needed.  The arithmetic of every product is
+// the one z_kernel does.
+// ---------------------------------------------------------------------------
+template <int NZ, int P, typename C>
+struct ZStashSmem {
   using F = LineFFT<NZ, P>;
   using LM = ZLaneMap<F::T>;
   using Rt = RealOf<C>;
-  static constexpr int NST = UV ? 6 : 4;  // parked components
   static constexpr size_t SBUF_OFF = align16((size_t)F::TWLEN * sizeof(C));
   static constexpr size_t ST_OFF = align16(SBUF_OFF + (size_t)LM::LPC * F::BUF * sizeof(C));
-  static constexpr size_t BYTES = ST_OFF + (size_t)NST * P * kThreads * sizeof(Rt);
+  static constexpr size_t BYTES = ST_OFF + (size_t)3 * P * kThreads * sizeof(Rt);
   static_assert(BYTES <= 113 * 1024, "two CTAs per SM");
-  static_assert(LM::LPC % 2 == 0, "a line and its mirror in one CTA");
   // The TMEM form (NS3D_Z_TMEM) keeps the stash in tensor memory instead:
-  // TM_COLS columns per CTA (NST P doubles per thread = 2 NST P words, rounded
-  // up to a power of two).  Its launch asks for at least TM_BYTES of shared
+  // TM_COLS columns per CTA (3 P doubles per thread = 6 P words, rounded up
+  // to a power of two).  Its launch asks for at least TM_BYTES of shared
   // memory, which caps the CTAs per SM that hold columns at
   // kTmemColsPerSm / TM_COLS, so an allocation never waits for good.
-  static constexpr int W = 2 * NST * P;
-  static constexpr uint32_t TM_COLS = W <= 32 ? 32 : (W <= 64 ? 64 : (W <= 128 ? 128 : 256));
+  static constexpr uint32_t TM_COLS = 6 * P <= 32 ? 32 : (6 * P <= 64 ? 64 : (6 * P <= 128 ? 128 : 256));
   static constexpr int TM_MAXCTAS = (int)(kTmemColsPerSm / TM_COLS);
   static constexpr size_t TM_BYTES =
       BYTES > (228 * 1024) / (TM_MAXCTAS + 1) + 1 ? BYTES : (228 * 1024) / (TM_MAXCTAS + 1) + 1;
-  static constexpr bool TM_OK = sizeof(Rt) == 8 && P % 4 == 0 && W <= 256;
+  static_assert(sizeof(Rt) == 8, "the TMEM form holds FP64 stash words in pairs");
+  static_assert(P % 4 == 0 && 6 * P <= 256, "TMEM stash columns");
   static_assert((TM_BYTES + 1024) * (TM_MAXCTAS + 1) > 228 * 1024, "CTAs per SM bound");
 };
 
@@ -891,28 +1028,15 @@ struct ZSmem {
 #ifndef NS3D_Z_TMEM
 #define NS3D_Z_TMEM 2
 #endif
-template <typename C>
 __host__ __device__ constexpr bool z_tmem(int nz) {
-  return sizeof(C) == 16 && (NS3D_Z_TMEM == 1 || (NS3D_Z_TMEM == 2 && nz >= 512));
+  return NS3D_Z_TMEM == 1 || (NS3D_Z_TMEM == 2 && nz >= 512);
 }
 
-// synchronises a line with its mirror: neighbouring lines of one warp, or the CTA
-template <int T>
-__device__ __forceinline__ void pair_sync() {
-  line_sync<2 * T>();
-}
-
-// pairs (x, y), (-x, -y) of one instance: all rows of the planes 0 < x < Nx/2,
-// rows 0 .. Ny/2 of the planes 0 and Nx/2, which hold their own mirrors
-__host__ __device__ __forceinline__ int z_pairs(const PassGeom& g) {
-  return g.Nx * g.Ny / 2 + 2;
-}
-
-template <int NZ, int P, bool UV, typename C, bool TM = false>
-__global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel(ZArgs<UV ? 6 : 3, C> a, PassGeom g) {
+template <int NZ, int P, typename C, bool TM = false>
+__global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel_st(ZArgs<3, C> a, PassGeom g) {
   using F = LineFFT<NZ, P>;
   using Rt = RealOf<C>;
-  using S = ZSmem<NZ, P, UV, C>;
+  using S = ZStashSmem<NZ, P, C>;
   constexpr int T = F::T;
   using LM = ZLaneMap<T>;
   constexpr int PW = z_pw<NZ, P, C>();
@@ -920,7 +1044,6 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel(ZArgs<UV ? 6 : 3
   __shared__ uint32_t tm_base_s;  // TMEM address of the CTA's columns (TM)
   const int warp = threadIdx.x >> 5;
   if constexpr (TM) {
-    static_assert(S::TM_OK, "TMEM stash");
     if (warp == 0) tmem_alloc_warp(&tm_base_s, S::TM_COLS);
     tmem_fence_before_sync();
   }
@@ -933,34 +1056,25 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel(ZArgs<UV ? 6 : 3
   }
   int li, t;
   LM::get(li, t);
-  const int side = li & 1;  // 0: the line (x, y), 1: its mirror
-  const int upi = z_pairs(g);
-  const int u = blockIdx.x * (LM::LPC / 2) + (li >> 1);
-  const bool valid = u < upi * nbatch(g);
-  size_t base;      // this thread's line in C, D, E
-  size_t q1, q2;    // the pair's rows in Qh: (x, y), and (x, -y) on a plane that is its own mirror
-  bool both;        // whether q2 is stored too
-  {
-    const int uc = valid ? u : 0;
-    const int inst = uc / upi;
-    int r = uc - inst * upi, x = 0;
-    if (r > g.Ny / 2) {
-      r -= g.Ny / 2 + 1;
-      x = 1 + r / g.Ny;
-      r -= (x - 1) * g.Ny;
-    }
-    const int y = r, xm = x ? g.Nx - x : 0, ym = y ? g.Ny - y : 0;
-    const size_t row0 = (size_t)inst * g.Nx * g.Ny;
-    base = (row0 + (size_t)(side ? xm * g.Ny + ym : x * g.Ny + y)) * g.Zp;
-    q1 = (row0 + (size_t)(x * g.Ny + y)) * g.Mz;
-    q2 = (row0 + (size_t)(x * g.Ny + ym)) * g.Mz;
-    both = valid && xm == x && ym != y;
-  }
+  const int nb = g.Nx * g.Ny;
+  const int b = blockIdx.x * LM::LPC + li;
+  const bool valid = b < nb;
+  const size_t base = (size_t)(valid ? b : 0) * g.Zp;   // C, D, E
+  const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
   C* sbuf = (C*)(dsm + S::SBUF_OFF) + li * F::BUF;
-  const C* sbuf_m = (const C*)(dsm + S::SBUF_OFF) + (li ^ 1) * F::BUF;
   Rt* stash = (Rt*)(dsm + S::ST_OFF) + threadIdx.x;
   const ZRun run{base, g.Zc, valid && t == 0 && z_prefetch(g)};
-  // stash component c: the P values v(s)
+  const C* order[9] = {a.C[0], a.C[1], a.C[2], a.E[2], a.D[2], a.E[0], a.D[0], a.E[1], a.D[1]};
+  auto pf = [&](int i) {
+    if (NS3D_Z_L2PF != 0 && run.ask) prefetch_z_line(order[i], run.base, run.Zc);
+  };
+  if (NS3D_Z_L2PF == 1)
+    for (int i = 0; i < 9; ++i) pf(i);
+  if (NS3D_Z_L2PF == 2) { pf(0); pf(1); }  // C0, C1
+  auto ux = [&](int s) -> Rt& { return stash[(0 * P + s) * kThreads]; };
+  auto uy = [&](int s) -> Rt& { return stash[(1 * P + s) * kThreads]; };
+  auto uz = [&](int s) -> Rt& { return stash[(2 * P + s) * kThreads]; };
+  // stash component c (0 u_x, 1 u_y, 2 u_z): the P values v(s)
   auto park = [&](int c, auto v) {
     if constexpr (TM) {
 #pragma unroll
@@ -980,157 +1094,81 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel(ZArgs<UV ? 6 : 3
       for (int s = 0; s < P; ++s) stash[(c * P + s) * kThreads] = v(s);
     }
   };
-  // hands f(s, values of the NC components from c0 on) every sample
-  auto parked = [&](auto nc, int c0, auto f) {
-    constexpr int NC = decltype(nc)::value;
+  const Rt sc = (Rt)g.inv_vol;
+  const Rt kfz = (Rt)g.kfz;
+  C w[P];
+  Rt q0[P], q1[P];
+  // q[s] = u_x(s) (w[s].x sc) + u_y(s) (w[s].y sc) + u_z(s) q[s]  (calc_vels_nabla_vels)
+  auto product = [&](Rt (&q)[P]) {
     if constexpr (TM) {
 #pragma unroll
       for (int s0 = 0; s0 < P; s0 += 4) {
-        uint32_t r[NC][8];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) tmem_ld8(tm + (uint32_t)((c0 + c) * 2 * P + 2 * s0), r[c]);
+        uint32_t rx[8], ry[8], rz[8];
+        tmem_ld8(tm + (uint32_t)(0 * 2 * P + 2 * s0), rx);
+        tmem_ld8(tm + (uint32_t)(1 * 2 * P + 2 * s0), ry);
+        tmem_ld8(tm + (uint32_t)(2 * 2 * P + 2 * s0), rz);
         tmem_wait_ld();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          Rt v[NC];
-#pragma unroll
-          for (int c = 0; c < NC; ++c)
-            v[c] = __hiloint2double((int)r[c][2 * k + 1], (int)r[c][2 * k]);
-          f(s0 + k, v);
+          const int s = s0 + k;
+          const Rt vx = __hiloint2double((int)rx[2 * k + 1], (int)rx[2 * k]);
+          const Rt vy = __hiloint2double((int)ry[2 * k + 1], (int)ry[2 * k]);
+          const Rt vz = __hiloint2double((int)rz[2 * k + 1], (int)rz[2 * k]);
+          q[s] = vx * (w[s].x * sc) + vy * (w[s].y * sc) + vz * q[s];
         }
       }
     } else {
 #pragma unroll
-      for (int s = 0; s < P; ++s) {
-        Rt v[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) v[c] = stash[((c0 + c) * P + s) * kThreads];
-        f(s, v);
-      }
+      for (int s = 0; s < P; ++s)
+        q[s] = ux(s) * (w[s].x * sc) + uy(s) * (w[s].y * sc) + uz(s) * q[s];
     }
   };
-  using One = std::integral_constant<int, 1>;
-  using Two = std::integral_constant<int, 2>;
-  using Three = std::integral_constant<int, 3>;
-  const Rt sc = (Rt)g.inv_vol;
-  const Rt kfz = (Rt)g.kfz;
-  C w[P];
-  Rt q0[P], qy[P], qz[P];
-  // one paired C2R: (f1, f2), each optionally times i kz
-  auto c2r = [&](auto ik1, auto ik2, const C* f1, const C* f2) {
-    load_pair<NZ, P, decltype(ik1)::value, decltype(ik2)::value>(w, f1, f2, base, t, kfz, run.Zc);
-    F::template run<+1, PW>(w, t, sbuf, tw_s);
-  };
-  constexpr std::false_type plain{};
-  constexpr std::true_type ik{};
-  prefetch_z_pair(a.C[0], a.C[1], run);
-  if constexpr (!UV) {
-    // q[s] = u_x(s) (w[s].x sc) + u_y(s) (w[s].y sc) + u_z(s) q[s]  (calc_vels_nabla_vels)
-    auto product = [&](Rt (&q)[P]) {
-      parked(Three{}, 0, [&](int s, const Rt* v) {
-        q[s] = v[0] * (w[s].x * sc) + v[1] * (w[s].y * sc) + v[2] * q[s];
-      });
-    };
-    prefetch_z_pair(a.C[2], a.C[2], run);
-    c2r(plain, plain, a.C[0], a.C[1]);  // (u_x, u_y)
-    park(0, [&](int s) { return w[s].x * sc; });
-    park(1, [&](int s) { return w[s].y * sc; });
-    prefetch_z_pair(a.E[2], a.D[2], run);
-    c2r(plain, ik, a.C[2], a.C[2]);  // (u_z, d_z u_z)
-    park(2, [&](int s) { return w[s].x * sc; });
+  // (u_x, u_y)
+  if (NS3D_Z_L2PF == 2) pf(2);  // C2
+  load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+  park(0, [&](int s) { return w[s].x * sc; });
+  park(1, [&](int s) { return w[s].y * sc; });
+  // (u_z, d_z u_z); q0 accumulates Q_z first
+  if (NS3D_Z_L2PF == 2) { pf(3); pf(4); }  // E2, D2
+  load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz, run.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+  park(2, [&](int s) { return w[s].x * sc; });
 #pragma unroll
-    for (int s = 0; s < P; ++s) q0[s] = w[s].y * sc;
-    prefetch_z_pair(a.E[0], a.D[0], run);
-    c2r(plain, plain, a.E[2], a.D[2]);  // (d_x u_z, d_y u_z)
-    product(q0);                        // Q_z
-    park(3, [&](int s) { return q0[s]; });
-    c2r(ik, ik, a.C[0], a.C[1]);  // (d_z u_x, d_z u_y)
+  for (int s = 0; s < P; ++s) q0[s] = w[s].y * sc;
+  // Q_z = u_x d_x u_z + u_y d_y u_z + u_z d_z u_z
+  if (NS3D_Z_L2PF == 2) { pf(5); pf(6); }  // E0, D0
+  load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz, run.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+  product(q0);
+  // R2C of Q_z alone
 #pragma unroll
-    for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; qy[s] = w[s].y * sc; }
-    prefetch_z_pair(a.E[1], a.D[1], run);
-    c2r(plain, plain, a.E[0], a.D[0]);
-    product(q0);
-    c2r(plain, plain, a.E[1], a.D[1]);
-    product(qy);
-    parked(One{}, 3, [&](int s, const Rt* v) { qz[s] = v[0]; });
-  } else {
-    // B(u,v)_i = (v.grad) u_i + (u.grad) v_i (convolute_2p3_UV,
-    // Source/advection_2_3.cu:414-466); fields 0..2 are u, 3..5 are v
-    prefetch_z_pair(a.C[2], a.C[3], run);
-    c2r(plain, plain, a.C[0], a.C[1]);
-    park(0, [&](int s) { return w[s].x * sc; });
-    park(1, [&](int s) { return w[s].y * sc; });
-    prefetch_z_pair(a.C[4], a.C[5], run);
-    c2r(plain, plain, a.C[2], a.C[3]);
-    park(2, [&](int s) { return w[s].x * sc; });
-    park(3, [&](int s) { return w[s].y * sc; });
-    prefetch_z_pair(a.E[0], a.D[0], run);
-    c2r(plain, plain, a.C[4], a.C[5]);
-    park(4, [&](int s) { return w[s].x * sc; });
-    park(5, [&](int s) { return w[s].y * sc; });
-    auto component = [&](Rt (&q)[P], int i) {
-      prefetch_z_pair(a.E[3 + i], a.E[3 + i], run);
-      c2r(plain, plain, a.E[i], a.D[i]);  // (d_x u_i, d_y u_i)
-      parked(Two{}, 3, [&](int s, const Rt* v) {
-        q[s] = v[0] * (w[s].x * sc) + v[1] * (w[s].y * sc);
-      });
-      prefetch_z_pair(a.D[3 + i], a.D[3 + i], run);
-      c2r(ik, plain, a.C[i], a.E[3 + i]);  // (d_z u_i, d_x v_i)
-      parked(One{}, 5, [&](int s, const Rt* v) { q[s] = q[s] + v[0] * (w[s].x * sc); });
-      parked(One{}, 0, [&](int s, const Rt* v) { q[s] = q[s] + v[0] * (w[s].y * sc); });
-      if (i < 2) prefetch_z_pair(a.E[i + 1], a.D[i + 1], run);
-      c2r(plain, ik, a.D[3 + i], a.C[3 + i]);  // (d_y v_i, d_z v_i)
-      parked(Two{}, 1, [&](int s, const Rt* v) {
-        q[s] = q[s] + (v[0] * (w[s].x * sc) + v[1] * (w[s].y * sc));
-      });
-    };
-    component(q0, 0);
-    component(qy, 1);
-    component(qz, 2);
-  }
-  // the odd parts: this line's products against the mirror line's at -z
-  line_sync<T>();  // the last transform's readers of sbuf are done
-#pragma unroll
-  for (int s = 0; s < P; ++s)
-    sbuf[spad<PW>(t + T * s)] = side ? mkc<C>(q0[s], qy[s]) : mkc<C>(qz[s], (Rt)0);
-  pair_sync<T>();
-#pragma unroll
-  for (int s = 0; s < P; ++s) {
-    const int k = t + T * s;
-    const C m = sbuf_m[spad<PW>(k == 0 ? 0 : NZ - k)];
-    w[s] = side ? mkc<C>((Rt)0.5 * (qz[s] - m.x), (Rt)0)
-                : mkc<C>((Rt)0.5 * (q0[s] - m.x), (Rt)0.5 * (qy[s] - m.y));
-  }
-  pair_sync<T>();  // the mirror's reads come before this line's exchanges
+  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], (Rt)0);
   F::template run<-1, PW>(w, t, sbuf, tw_s);
-  // side 0: split the packed (q_x, q_y) with the mirror bin W[N - k]; side 1:
-  // q_z of the line (-x, -y) is -conj of the line (x, y)'s
-  line_sync<T>();
-#pragma unroll
-  for (int s = 0; s < P; ++s) sbuf[spad<PW>(t + T * s)] = w[s];
-  line_sync<T>();
   if (valid) {
 #pragma unroll
     for (int s = 0; s < P; ++s) {
       const int k = t + T * s;
-      if (k > NZ / 2) continue;
-      const C v = w[s];
-      if (side == 0) {
-        const C m = sbuf[spad<PW>(k == 0 ? 0 : NZ - k)];
-        const C s1 = mkc<C>((Rt)0.5 * (v.x + m.x), (Rt)0.5 * (v.y - m.y));
-        const C s2 = mkc<C>((Rt)0.5 * (v.y + m.y), (Rt)-0.5 * (v.x - m.x));
-        a.Qh[0][q1 + k] = s1;
-        a.Qh[1][q1 + k] = s2;
-        if (both) {  // the row (x, -y) = -conj of this one
-          a.Qh[0][q2 + k] = mkc<C>(-s1.x, s1.y);
-          a.Qh[1][q2 + k] = mkc<C>(-s2.x, s2.y);
-        }
-      } else {
-        a.Qh[2][q1 + k] = mkc<C>(-v.x, v.y);
-        if (both) a.Qh[2][q2 + k] = v;
-      }
+      if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
     }
   }
+  // (d_z u_x, d_z u_y)
+  load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; q1[s] = w[s].y * sc; }
+  if (NS3D_Z_L2PF == 2) { pf(7); pf(8); }  // E1, D1
+  load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz, run.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+  product(q0);
+  load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz, run.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+  product(q1);
+  // R2C of (Q_x, Q_y) packed
+#pragma unroll
+  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
+  F::template run<-1, PW>(w, t, sbuf, tw_s);
+  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
   if constexpr (TM) {
     // every thread's TMEM reads have completed (waited); free the columns
     tmem_fence_before_sync();
@@ -1141,8 +1179,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel(ZArgs<UV ? 6 : 3
 }
 
 // ---------------------------------------------------------------------------
-// fwd_y: in-place forward transform along y of the 3 product spectra, on the
-// planes x = 0 .. Nx/2 the z pass stores
+// fwd_y: in-place forward transform along y of the 3 product spectra
 // ---------------------------------------------------------------------------
 template <typename Cx = double2>
 struct FwdYArgs {
@@ -1163,8 +1200,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) fwd_y_kernel(FwdYArg
   LM::get(li, t);
   C* sbuf = S::sbuf(dsm, li);
   C* pf = S::pf(dsm);
-  const int hx = g.Nx / 2 + 1;  // planes of an instance
-  const int nb = hx * g.Mz * nbatch(g);
+  const int nb = g.Nx * g.Mz;
   const int groups = (nb + LM::LPC - 1) / LM::LPC;
   const size_t stride = (size_t)g.Mz;
   const GroupRange gr = group_range(groups);
@@ -1174,9 +1210,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) fwd_y_kernel(FwdYArg
   auto line_base = [&](int gidx) -> size_t {
     const int b = gidx * LM::LPC + li;
     const int bc = b < nb ? b : 0;
-    const int pl = bc / g.Mz, z = bc - pl * g.Mz;
-    const int inst = pl / hx;
-    return (size_t)(inst * g.Nx + (pl - inst * hx)) * g.Ny * g.Mz + z;
+    const int x = bc / g.Mz, z = bc - x * g.Mz;
+    return (size_t)x * g.Ny * g.Mz + z;
   };
   issue_line<P, T>(pf, a.Q[0], line_base(grp), stride, t);
   cp_async_commit();
@@ -1420,110 +1455,37 @@ struct FwdXArgs {
   const double2* tw;
 };
 
-// The product spectra along x: G(x) for x = 0 .. N/2, G(-x) = -conj G(x) (the
-// z pass kept the odd part), so H = -i G is Hermitian and its transform real:
-// FFT_x of G is i times it.  Two components' lines share one complex FFT of
-// H_1 + i H_2.  A thread copies its samples x = t + T s below N/2 (half of a
-// slot per component; thread 0 also x = N/2, into a cell behind the slot) and
-// reads the others from the thread that holds their mirror, after a barrier.
-template <int N, int P, int CS, typename E>
-__device__ __forceinline__ void issue_half(E* blk, E* mid, const E* __restrict__ src, size_t off,
-                                           size_t stride, int t) {
-  constexpr int T = N / P;
-#pragma unroll
-  for (int s = 0; s < P / 2; ++s)
-    cp_async_elem(blk + CS * (s * kThreads + threadIdx.x), src + off + (size_t)(t + T * s) * stride,
-                  true);
-  if (t == 0) cp_async_elem(mid, src + off + (size_t)(N / 2) * stride, true);
-}
-
-// H(t + T s) of one component from its half slot; tm: the thread of the same
-// line that holds the mirrors (T - t of this thread's t; itself at t = 0)
-template <int N, int P, int CS, typename C>
-__device__ __forceinline__ C half_sample(const C* blk, const C* mid, int t, int tm, int s) {
-  using Rt = RealOf<C>;
-  if (s < P / 2) {
-    const C v = blk[CS * (s * kThreads + threadIdx.x)];
-    return mkc<C>(v.y, t == 0 && s == 0 ? (Rt)0 : -v.x);  // H(0) is real
-  }
-  // x >= N/2: conj H(N - x); row P - s of thread 0 (x = N/2: its cell), else
-  // row P - 1 - s of thread T - t
-  const C* m = blk + CS * ((t == 0 ? P - s : P - 1 - s) * kThreads + tm);
-  if (s == P / 2 && t == 0) m = mid;
-  const C v = *m;
-  return mkc<C>(v.y, s == P / 2 && t == 0 ? (Rt)0 : v.x);
-}
-// W = H_1 + i H_2 of the packed transform (H_2 = 0 with PAIR false)
-template <int N, int P, int CS, bool PAIR, typename C>
-__device__ __forceinline__ void load_half(C (&w)[P], const C* b1, const C* m1, const C* b2,
-                                          const C* m2, int t, int tm) {
-#pragma unroll
-  for (int s = 0; s < P; ++s) {
-    const C h1 = half_sample<N, P, CS>(b1, m1, t, tm, s);
-    if constexpr (PAIR) {
-      const C h2 = half_sample<N, P, CS>(b2, m2, t, tm, s);
-      w[s] = mkc<C>(h1.x - h2.y, h1.y + h2.x);
-    } else {
-      w[s] = h1;
-    }
-  }
-}
-// the thread of a line's mirrors (LaneMap's layout)
-template <int T>
-__device__ __forceinline__ int mirror_thread(int li, int t) {
-  using LM = LaneMap<T>;
-  const int tt = t == 0 ? 0 : T - t;
-  if constexpr (LM::kSpread) {
-    return tt * LM::LPC + li;
-  } else {
-    return (int)(threadIdx.x & ~31u) + tt * LM::LPW + li % LM::LPW;
-  }
-}
-
 // One line of the forward x pass: FFT_x of the 3 product spectra (from the
 // prefetch slots), then the pointwise update of Source/diffusion.cu.
 template <int NX, int P, int MODE, bool COMBINE, typename C>
-__device__ __forceinline__ void fwd_x_line(const FwdXArgs<C>& a, const PassGeom& g, int li, int t,
-                                           int L, size_t off, int inst, bool valid, C* sbuf,
-                                           const C* tw_s, C* pf, C* mid, int& ub,
+__device__ __forceinline__ void fwd_x_line(const FwdXArgs<C>& a, const PassGeom& g, int t, int L,
+                                           size_t off, int inst, bool valid, C* sbuf,
+                                           const C* tw_s, C* pf, int& ub,
                                            bool more, size_t offn) {
   constexpr int T = NX / P;
   using F = LineFFT<NX, P>;
-  using LM = LaneMap<T>;
   const int nlines = g.Ny * g.Mz;
   const int y = L / g.Mz, z = L - y * g.Mz;
-  const int tm = mirror_thread<T>(li, t);
-  // Re(Qh) is set to zero (set_to_zero_real): only the imaginary part of each
-  // transformed component is needed.  Units: (Q_x, Q_y), then Q_z
+  // Re(Qh) is set to zero (set_to_zero_real), so only the imaginary part of
+  // each transformed component is kept
   double qi[3][P];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
+  for (int c = 0; c < 3; ++c) {
     const C* cur = pf + ub * (P * kThreads);
-    const C* cmid = mid + ub * (2 * LM::LPC);
     C* nxt = pf + (ub ^ 1) * (P * kThreads);
-    C* nmid = mid + (ub ^ 1) * (2 * LM::LPC);
-    if (c == 0) {
-      issue_half<NX, P, 1>(nxt, nmid + li, a.Qh[2], off, (size_t)nlines, t);
+    if (c + 1 < 3) {
+      issue_line<P, T>(nxt, a.Qh[c + 1], off, (size_t)nlines, t);
     } else if (more) {
-      issue_half<NX, P, 1>(nxt, nmid + li, a.Qh[0], offn, (size_t)nlines, t);
-      issue_half<NX, P, 1>(nxt + P / 2 * kThreads, nmid + LM::LPC + li, a.Qh[1], offn,
-                           (size_t)nlines, t);
+      issue_line<P, T>(nxt, a.Qh[0], offn, (size_t)nlines, t);
     }
     cp_async_commit();
     cp_async_wait<1>();
-    line_sync<LM::SW>();  // the line's other threads' copies
     C v[P];
-    if (c == 0)
-      load_half<NX, P, 1, true>(v, cur, cmid + li, cur + P / 2 * kThreads, cmid + LM::LPC + li, t,
-                                tm);
-    else
-      load_half<NX, P, 1, false>(v, cur, cmid + li, cur, cmid, t, tm);
-    F::template run<-1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
 #pragma unroll
-    for (int s = 0; s < P; ++s) {
-      qi[2 * c][s] = (double)v[s].x;
-      if (c == 0) qi[1][s] = (double)v[s].y;
-    }
+    for (int s = 0; s < P; ++s) v[s] = cur[s * kThreads];
+    F::template run<-1, F::PADW, LaneMap<T>::SW>(v, t, sbuf, tw_s);
+#pragma unroll
+    for (int s = 0; s < P; ++s) qi[c][s] = (double)v[s].y;
     ub ^= 1;
   }
   if (!valid) return;
@@ -1645,18 +1607,9 @@ __device__ __forceinline__ void prefetch_update_rows(const FwdXArgs<C>& a, int G
   }
 }
 
-// PassSmem with the x = N/2 cells of the two buffers behind them
-template <int N, int P, typename C>
-struct FwdXSmem : PassSmem<N, P, C, C> {
-  using Base = PassSmem<N, P, C, C>;
-  static constexpr size_t MID_OFF = align16(Base::BYTES);
-  static constexpr size_t BYTES = MID_OFF + (size_t)4 * Base::LPC * sizeof(C);
-  static_assert(BYTES <= 227 * 1024, "shared memory per CTA");
-};
-
 template <int NX, int P, int MODE, bool COMBINE, typename C>
 __global__ void __launch_bounds__(kThreads, kMinCtasFwdX) fwd_x_kernel(FwdXArgs<C> a, PassGeom g) {
-  using S = FwdXSmem<NX, P, C>;
+  using S = PassSmem<NX, P, C, C>;
   using F = typename S::F;
   using LM = typename S::LM;
   constexpr int T = F::T;
@@ -1666,8 +1619,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasFwdX) fwd_x_kernel(FwdXArgs<
   int li, t;
   LM::get(li, t);
   C* sbuf = S::sbuf(dsm, li);
-  C* pf = (C*)(dsm + S::PF_OFF);
-  C* mid = (C*)(dsm + S::MID_OFF);
+  C* pf = S::pf(dsm);
   const int nlines = g.Ny * g.Mz;
   const int tlines = nlines * nbatch(g);
   const int groups = (tlines + LM::LPC - 1) / LM::LPC;
@@ -1681,10 +1633,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasFwdX) fwd_x_kernel(FwdXArgs<
   if (grp >= g_end) return;
   {
     const int G0 = grp * LM::LPC + li;
-    const size_t off0 = line_off(G0 < tlines ? G0 : 0);
-    issue_half<NX, P, 1>(pf, mid + li, a.Qh[0], off0, (size_t)nlines, t);
-    issue_half<NX, P, 1>(pf + P / 2 * kThreads, mid + LM::LPC + li, a.Qh[1], off0, (size_t)nlines,
-                         t);
+    issue_line<P, T>(pf, a.Qh[0], line_off(G0 < tlines ? G0 : 0), (size_t)nlines, t);
     cp_async_commit();
   }
   int ub = 0;
@@ -1697,8 +1646,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtasFwdX) fwd_x_kernel(FwdXArgs<
     const int Gn = gn * LM::LPC + li;
     if constexpr (MODE != kConvOut && !LM::kSpread)
       prefetch_update_rows<NX, LM::LPC, COMBINE>(a, grp * LM::LPC, tlines, nlines, line_off);
-    fwd_x_line<NX, P, MODE, COMBINE, C>(a, g, li, t, Gc - inst * nlines, line_off(Gc), inst,
-                                        valid, sbuf, tw_s, pf, mid, ub, gn < g_end,
+    fwd_x_line<NX, P, MODE, COMBINE, C>(a, g, t, Gc - inst * nlines, line_off(Gc), inst, valid,
+                                     sbuf, tw_s, pf, ub, gn < g_end,
                                      line_off(Gn < tlines ? Gn : 0));
   }
   cp_async_wait<0>();
@@ -1708,9 +1657,9 @@ __global__ void __launch_bounds__(kThreads, kMinCtasFwdX) fwd_x_kernel(FwdXArgs<
 // fwd_x with the update's operands in the prefetch ring.
 //
 // fwd_x_kernel reads the state (and RK partner) samples of its update with
-// plain loads after the transforms, two points at a time: every group
+// plain loads after the three transforms, two points at a time: every group
 // waits several memory round trips with little in flight.  Here the unit
-// sequence of a group is (Qh_x, Qh_y), Qh_z (transformed), then u^s_c (and
+// sequence of a group is Qh_x, Qh_y, Qh_z (transformed), then u^s_c (and
 // u^n_c when combining) for c = x, y, z, and every unit goes through one ring
 // of NSLOT per-thread cp.async slots, issued NSLOT - 1 units ahead.  The
 // update runs component by component as its operands arrive: component c of
@@ -1743,8 +1692,7 @@ struct FxRingSmem {
   static constexpr int STRIDE = line_stride(F::BUF, xy_stride_target<F::T>());
   static constexpr size_t SBUF_OFF = align16((size_t)F::TWLEN * sizeof(C));
   static constexpr size_t RING_OFF = align16(SBUF_OFF + (size_t)LPC * STRIDE * sizeof(C));
-  static constexpr size_t MID = (size_t)P * kThreads * sizeof(double2);  // x = N/2 cells
-  static constexpr size_t SLOT = MID + (size_t)2 * LPC * sizeof(double2);
+  static constexpr size_t SLOT = (size_t)P * kThreads * sizeof(double2);
   static constexpr size_t BYTES = RING_OFF + (size_t)NSLOT * SLOT;
   // CTAs per SM asked of ptxas (registers): as many as the shared memory allows
   static constexpr int MINC =
@@ -1760,8 +1708,7 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
   using LM = typename S::LM;
   constexpr int T = F::T;
   constexpr int NUPD = MODE == kConvOut ? 0 : (COMBINE ? 6 : 3);
-  constexpr int UPG = 2 + NUPD;  // units per group
-  constexpr int CELL = (int)(sizeof(double2) / sizeof(C));  // C elements per cell
+  constexpr int UPG = 3 + NUPD;  // units per group
   static_assert(NSLOT >= 2 && (!COMBINE || NSLOT >= 3), "ring depth");
   extern __shared__ __align__(16) unsigned char dsm[];
   F::load_tw((C*)dsm, a.tw);
@@ -1788,16 +1735,12 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
       const int G = (gr.grp + gi * gr.step) * LM::LPC + li;
       const size_t off = line_off(G < tlines ? G : 0);
       unsigned char* sl = ring + (size_t)(k % NSLOT) * S::SLOT;
-      C* q = (C*)sl;
-      C* mid = (C*)(sl + S::MID) + CELL * li;
-      if (j == 0) {
-        issue_half<NX, P, CELL>(q, mid, a.Qh[0], off, (size_t)nlines, t);
-        issue_half<NX, P, CELL>(q + CELL * (P / 2 * kThreads), mid + CELL * LM::LPC, a.Qh[1], off,
-                                (size_t)nlines, t);
-      } else if (j == 1) {
-        issue_half<NX, P, CELL>(q, mid, a.Qh[2], off, (size_t)nlines, t);
+      if (j < 3) {
+        constexpr int CELL = (int)(sizeof(double2) / sizeof(C));  // C elements per cell
+        issue_line<P, T, CELL * kThreads>((C*)sl + CELL * threadIdx.x, a.Qh[j], off,
+                                          (size_t)nlines, t);
       } else {
-        const int u = j - 2;
+        const int u = j - 3;
         const double2* src = COMBINE ? ((u & 1) ? a.un[u >> 1] : a.us[u >> 1]) : a.us[u];
         issue_line<P, T>((double2*)sl + threadIdx.x, src, off, (size_t)nlines, t);
       }
@@ -1818,26 +1761,20 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
     // transformed products: Re(Qh) is set to zero (set_to_zero_real), so only
     // the imaginary parts are kept; Qh(0,0,0) = 0
     double qi[3][P];
-    const int tm = mirror_thread<T>(li, t);
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
+    for (int c = 0; c < 3; ++c) {
       issue(k + NSLOT - 1);
       cp_async_wait<NSLOT - 1>();
-      line_sync<LM::SW>();  // the line's other threads' copies
-      const C* cur = (const C*)slot(k);
-      const C* mid = (const C*)(slot(k) + S::MID) + CELL * li;
+      constexpr int CELL = (int)(sizeof(double2) / sizeof(C));
+      const C* cur = (const C*)slot(k) + CELL * threadIdx.x;
       C v[P];
-      if (c == 0)
-        load_half<NX, P, CELL, true>(v, cur, mid, cur + CELL * (P / 2 * kThreads),
-                                     mid + CELL * LM::LPC, t, tm);
-      else
-        load_half<NX, P, CELL, false>(v, cur, mid, cur, mid, t, tm);
+#pragma unroll
+      for (int s = 0; s < P; ++s) v[s] = cur[s * CELL * kThreads];
       F::template run<-1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
 #pragma unroll
       for (int s = 0; s < P; ++s) {
         const bool origin = (t + T * s == 0) && (L == 0);
-        qi[2 * c][s] = origin ? 0.0 : (double)v[s].x;
-        if (c == 0) qi[1][s] = origin ? 0.0 : (double)v[s].y;
+        qi[c][s] = origin ? 0.0 : (double)v[s].y;
       }
       ++k;
     }
@@ -1873,7 +1810,7 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
         const double kk = kx * kx + ky * ky + kz * kz;
         kq[s] = kk > 0.0 ? (kx * qi[0][s] + ky * qi[1][s] + kz * qi[2][s]) / kk : 0.0;
       }
-#pragma unroll 1  // one copy of the update's code: three overflow the instruction cache
+#pragma unroll
       for (int c = 0; c < 3; ++c) {
         // issued so far: units 0 .. k + NSLOT - 2; the next issue refills the
         // slot of unit k - 1, consumed already
@@ -1897,8 +1834,7 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
           const double kx = g.kfx * (double)signed_idx(x, NX);
           const double kk = kx * kx + ky * ky + kz * kz;
           // AM.Q - Q, imaginary part only
-          const double qc = c == 0 ? qi[0][s] : (c == 1 ? qi[1][s] : qi[2][s]);
-          const double pc = (c == 0 ? kx : kc) * kq[s] - qc;
+          const double pc = (c == 0 ? kx : kc) * kq[s] - qi[c][s];
           double2 f = make_double2(0.0, 0.0);
           if constexpr (MODE != kImplicit) {
             if (dense_f) {
