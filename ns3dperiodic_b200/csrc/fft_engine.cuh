@@ -225,11 +225,15 @@ __device__ __forceinline__ void line_sync() {
 // shared-memory line buffer index with one pad slot every PADW entries;
 // PADW = 0: no padding, the position inside each row of 16 elements XORed
 // with bits 3..6 of the index (the 8-byte lines of the FP32 z pass, whose
-// Stockham exchanges the padding leaves 2-way bank conflicted)
+// Stockham exchanges the padding leaves 2-way bank conflicted); PADW = -1:
+// likewise with the row's own number (16-byte lines of radix 16: no words lost
+// to padding)
 template <int PADW>
 __device__ __forceinline__ int spad(int p) {
   if constexpr (PADW == 0) {
     return (p & ~15) | ((p & 15) ^ ((p >> 3) & 15));
+  } else if constexpr (PADW < 0) {
+    return p ^ ((p >> 4) & 15);
   } else {
     return p + p / PADW;
   }
@@ -248,6 +252,18 @@ constexpr int line_buf_len() {
 #define NS3D_TW_COMPOSE 1
 #endif
 constexpr bool kComposeTwiddles = NS3D_TW_COMPOSE != 0;
+// The powers a stage of radix R reads from its table: all of them for R <= 4,
+// else w, w^2, w^4, w^8.  The table holds only these rows (64 entries instead
+// of 240 for the second stage of a 256-point line of radix 16).
+__host__ __device__ constexpr bool tw_all(int R) { return !kComposeTwiddles || R <= 4; }
+__host__ __device__ constexpr bool tw_read(int R, int r) {
+  return tw_all(R) || r == 1 || r == 2 || r == 4 || r == 8;
+}
+// table row of power r (r = R: the number of rows), and the power of a row
+__host__ __device__ constexpr int tw_row(int R, int r) {
+  return tw_all(R) ? r - 1 : (r <= 1 ? 0 : (r <= 2 ? 1 : (r <= 4 ? 2 : (r <= 8 ? 3 : 4))));
+}
+__host__ __device__ constexpr int tw_power(int R, int row) { return tw_all(R) ? row + 1 : 1 << row; }
 template <int N, int T, int DIR, int PADW, int SW, int NS, int R, int... Rest>
 struct Stages {
   static constexpr int P = N / T;
@@ -267,15 +283,16 @@ struct Stages {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = x[u + r * U];
       if constexpr (NS > 1) {
-        // stage table [r-1][jm] = w^r, w = exp(2 pi i jm / (NS R)); consecutive
-        // lanes read consecutive entries.  For R > 4 only w, w^2, w^4, w^8 are
-        // read and the other powers composed (at most 3 products deep).
+        // stage table [tw_row(r)][jm] = w^r, w = exp(2 pi i jm / (NS R));
+        // consecutive lanes read consecutive entries.  For R > 4 only w, w^2,
+        // w^4, w^8 are read and the other powers composed (at most 3 products
+        // deep).
         const int jm = b % NS;
         C W[R];
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          if (!kComposeTwiddles || R <= 4 || r == 1 || r == 2 || r == 4 || r == 8) {
-            W[r] = tw[(r - 1) * NS + jm];
+          if (tw_read(R, r)) {
+            W[r] = tw[tw_row(R, r) * NS + jm];
           } else {
             // r = hi + lo with hi the largest of 8, 4, 2 below r (lo >= 1)
             const int hi = r > 8 ? 8 : (r > 4 ? 4 : 2);
@@ -300,7 +317,7 @@ struct Stages {
 #pragma unroll
       for (int s = 0; s < P; ++s) x[s] = sbuf[spad<PADW>(t + T * s)];
       Stages<N, T, DIR, PADW, SW, NS * R, Rest...>::run(x, t, sbuf,
-                                                    NS > 1 ? tw + (R - 1) * NS : tw);
+                                                    NS > 1 ? tw + tw_row(R, R) * NS : tw);
     }
   }
 };
@@ -362,7 +379,7 @@ struct FirstRadix<RadixList<R0, Rs...>> {
 };
 
 // Per-stage twiddle tables of a plan, stage after stage (stages with NS > 1):
-// entry (r-1)*NS + jm of a stage = exp(2 pi i jm r step / N), step = N/(NS R).
+// entry tw_row(r)*NS + jm of a stage = exp(2 pi i jm r step / N), step = N/(NS R).
 template <int N, int NS, typename L>
 struct StageTw;
 template <int N, int NS>
@@ -373,7 +390,7 @@ struct StageTw<N, NS, RadixList<>> {
 };
 template <int N, int NS, int R, int... Rest>
 struct StageTw<N, NS, RadixList<R, Rest...>> {
-  static constexpr int own = NS > 1 ? (R - 1) * NS : 0;
+  static constexpr int own = NS > 1 ? tw_row(R, R) * NS : 0;
   using Next = StageTw<N, NS * R, RadixList<Rest...>>;
   static constexpr int len = own + Next::len;
   template <typename C>
@@ -381,7 +398,8 @@ struct StageTw<N, NS, RadixList<R, Rest...>> {
     if constexpr (NS > 1) {
       constexpr int step = N / (NS * R);
       for (int e = threadIdx.x; e < own; e += blockDim.x) {
-        const int r = e / NS + 1, jm = e - (r - 1) * NS;
+        const int row = e / NS, jm = e - row * NS;
+        const int r = tw_power(R, row);
         tws[e] = cvt<C>(tw_g[jm * r * step]);  // FP64 table, rounded for FP32 lines
       }
     }
@@ -423,7 +441,7 @@ struct LineFFT {
   using L = typename PlanV<N, P, V>::L;
   static constexpr int PADW = FirstRadix<L>::value < 4 ? 4 : FirstRadix<L>::value;
   static constexpr int BUF = line_buf_len<N, PADW>();
-  // shared-memory twiddle words the plan needs (N - first radix), at least 1
+  // shared-memory twiddle words the plan needs, at least 1
   static constexpr int TWLEN = StageTw<N, 1, L>::len > 0 ? StageTw<N, 1, L>::len : 1;
   // fills the per-stage table from the global table tw_g[e] = exp(2 pi i e / N);
   // ends with a CTA barrier

@@ -5,10 +5,10 @@
 namespace ns3d {
 
 cudaError_t run_z(const ZArgs<3>& a, const PassGeom& g, cudaStream_t st) {
-  return launch_z<false, double2>(a, g, st);
+  return launch_z(a, g, st);
 }
 cudaError_t run_z(const ZArgs<6>& a, const PassGeom& g, cudaStream_t st) {
-  return launch_z<true, double2>(a, g, st);
+  return launch_z(a, g, st);
 }
 
 }  // namespace ns3d

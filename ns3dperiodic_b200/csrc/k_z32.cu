@@ -5,10 +5,10 @@
 namespace ns3d {
 
 cudaError_t run_z(const ZArgs<3, float2>& a, const PassGeom& g, cudaStream_t st) {
-  return launch_z<false, float2>(a, g, st);
+  return launch_z(a, g, st);
 }
 cudaError_t run_z(const ZArgs<6, float2>& a, const PassGeom& g, cudaStream_t st) {
-  return launch_z<true, float2>(a, g, st);
+  return launch_z(a, g, st);
 }
 
 }  // namespace ns3d

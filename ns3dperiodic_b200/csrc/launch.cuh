@@ -19,9 +19,6 @@ namespace ns3d {
 #ifndef NS3D_PXY
 #define NS3D_PXY 16
 #endif
-#ifndef NS3D_PZ
-#define NS3D_PZ 8
-#endif
 #ifndef NS3D_PFX
 #define NS3D_PFX 16
 #endif
@@ -30,27 +27,18 @@ namespace ns3d {
 // the z / fwd_x passes that hold several fields per thread at once.
 constexpr int p_pow2(int n, int p) { return p > n ? n : p; }
 constexpr int p_xy(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PXY); }
-constexpr int p_z(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PZ); }
 constexpr int p_fx(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PFX); }
-// the tangent z pass keeps u, v and the three products live: fewer points
-constexpr int p_zuv(int n) { return n % 3 == 0 ? 6 : 4; }
-// The nonlinear term's z pass with the velocities stashed in shared memory
-// (z_kernel_st): 16 points per thread for powers of two (one Stockham
-// exchange per 256-point transform instead of two), 12 for multiples of 3.
-// NS3D_Z_STASH 0 keeps z_kernel with p_z points per thread.
-#ifndef NS3D_Z_STASH
-#define NS3D_Z_STASH 1
-#endif
+// The nonlinear term's z pass: 16 points per thread for powers of two (one
+// Stockham exchange per 256-point transform instead of two), 12 for multiples
+// of 3; the tangent form, with twice the velocities parked: 8.
 #ifndef NS3D_PZST
 #define NS3D_PZST 16
 #endif
-constexpr int p_zst(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PZST); }
-// FP32 lines of the nonlinear term's z pass: half the registers per point,
-// so 16 points per thread fit without the stash (one exchange per transform)
-#ifndef NS3D_PZ32
-#define NS3D_PZ32 16
+constexpr int p_z(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PZST); }
+#ifndef NS3D_PZUV
+#define NS3D_PZUV 8
 #endif
-constexpr int p_z32(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PZ32); }
+constexpr int p_zuv(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PZUV); }
 // points per thread of the plain line passes (8 measured slower than 16 at 256^3 and 512^3)
 #ifndef NS3D_PLINE
 #define NS3D_PLINE 16
@@ -313,33 +301,27 @@ cudaError_t launch_inv_y(const InvYArgs<NF, C>& a, const PassGeom& gi, cudaStrea
   }
 }
 
-template <int N, typename C>
-cudaError_t launch_z_stash(const ZArgs<3, C>& a, const PassGeom& g, cudaStream_t st) {
-  constexpr int P = p_zst(N);
-  using S = ZStashSmem<N, P, C>;
-  constexpr bool TM = z_tmem(N);
-  constexpr size_t bytes = TM ? S::TM_BYTES : S::BYTES;
-  const long long lines = (long long)g.Nx * g.Ny;
-  const unsigned grid = persistent_grid<KTag<40, N, P, prec_tag<C>()>>(
-      z_kernel_st<N, P, C, TM>, bytes, blocks_for(lines, lines_per_cta_z<N, P>()));
-  z_kernel_st<N, P, C, TM><<<grid, kThreads, bytes, st>>>(a, g);
-  return cudaGetLastError();
-}
-
-template <bool UV, typename C>
-cudaError_t launch_z(const ZArgs<UV ? 6 : 3, C>& a, const PassGeom& gi, cudaStream_t st) {
+template <typename C, int NF>
+cudaError_t launch_z(const ZArgs<NF, C>& a, const PassGeom& gi, cudaStream_t st) {
   const PassGeom g = planes_geom(gi);
   const long long lines = (long long)g.Nx * g.Ny;
   switch (g.Nz) {
-#define NS3D_CASE(N)                                                               \
-  case N: {                                                                        \
-    if constexpr (!UV && NS3D_Z_STASH && sizeof(C) == 16) {                        \
-      return launch_z_stash<N, C>(a, g, st);                                       \
-    }                                                                              \
-    constexpr int P = UV ? p_zuv(N) : (sizeof(C) == 8 ? p_z32(N) : p_z(N));        \
-    z_kernel<N, P, UV, C><<<blocks_for(lines, lines_per_cta_z<N, P>()),           \
-                         kWarpsPerCta * 32, 0, st>>>(a, g);                        \
-    return cudaGetLastError();                                                     \
+#define NS3D_CASE(N)                                                                  \
+  case N: {                                                                           \
+    constexpr bool UV = NF == 6;                                                      \
+    constexpr int P = UV ? p_zuv(N) : p_z(N);                                         \
+    using S = ZSmem<N, P, UV, C>;                                                     \
+    const unsigned groups = blocks_for(lines, S::LM::LPC);                            \
+    if constexpr (UV) {                                                               \
+      const unsigned grid = persistent_grid<KTag<41, N, P, prec_tag<C>()>>(           \
+          z_uv_kernel<N, P, C>, S::BYTES, groups);                                    \
+      z_uv_kernel<N, P, C><<<grid, kThreads, S::BYTES, st>>>(a, g);                   \
+    } else {                                                                          \
+      const unsigned grid = persistent_grid<KTag<40, N, P, prec_tag<C>()>>(           \
+          z_kernel<N, P, C>, S::BYTES, groups);                                       \
+      z_kernel<N, P, C><<<grid, kThreads, S::BYTES, st>>>(a, g);                      \
+    }                                                                                 \
+    return cudaGetLastError();                                                        \
   }
     NS3D_FOR_EACH_EXTENT(NS3D_CASE)
 #undef NS3D_CASE

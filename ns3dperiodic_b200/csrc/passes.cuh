@@ -664,7 +664,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
 
 // ---------------------------------------------------------------------------
 // z pass: lines along z (contiguous), batch b = x*Ny + y; input at b*Zp of the
-// compact scratch, product spectra at b*Mz
+// compact scratch, product spectra at b*Mz (arguments and loads; the kernel
+// follows)
 // ---------------------------------------------------------------------------
 template <int NF, typename Cx = double2>
 struct ZArgs {
@@ -674,6 +675,7 @@ struct ZArgs {
   const Cx* E[NF];  // IFFT_xy(i kx M u_i)
   Cx* Qh[3];        // R2C_z of the products (x, y still physical)
   const double2* tw;
+  int* err = nullptr;  // error flag of the bounded waits on the staged rows
 };
 
 // L2 prefetch of one contiguous run (16-byte aligned, a multiple of 16 bytes)
@@ -682,47 +684,11 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void* p, unsigned bytes) 
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// L2 prefetch of the z pass's input (NS3D_Z_L2PF): 0 none; 1 the CTA's nine
-// input runs (one contiguous run of LPC lines per field) at kernel start, in
-// the order the transforms read them; 2 each transform's two runs one
-// transform ahead (the bulk-copy unit fetches them while the current
-// transform runs, and the loads then hit L2).  Measured on a B200 (z pass per
-// launch, 256^3 / 128^3 FP64): none 503 / 80.4 us, 1: 462 / 81 us, 2: 439 /
-// 67.5 us (two repeats each, within 0.5%).
-#ifndef NS3D_Z_L2PF
-#define NS3D_Z_L2PF 2
-#endif
-
-// L2 prefetch of one z line's kept modes (elements base .. base + Zc - 1),
-// trimmed to 16-byte boundaries (FP32 rows of an odd Mz start at 8-byte
-// offsets).  One run per line and field: a run over the CTA's consecutive
-// lines would also fetch the masked third of every line.
+// L2 prefetch of a row of n elements, trimmed to 16-byte boundaries
 template <typename C>
-__device__ __forceinline__ void prefetch_z_line(const C* f, size_t base, int Zc) {
-  const uintptr_t a = (uintptr_t)(f + base) & ~(uintptr_t)15;
-  const uintptr_t e = (uintptr_t)(f + base + (size_t)Zc) & ~(uintptr_t)15;
-  if (e > a) prefetch_l2_bulk((const void*)a, (unsigned)(e - a));
-}
-
-// One z line of a CTA's thread: its first element, the kept modes, and
-// whether this thread asks for the line's prefetches (the line's t = 0).
-struct ZRun {
-  size_t base;
-  int Zc;
-  bool ask;
-};
-// Whether the pass's nine FP64 fields are larger than what L2 keeps of them
-// between inv_y and this pass (126 MB): below, the prefetches only cost issue
-// slots (32^3: 18.6 us a launch without them, 24.4 us with).
-__device__ __forceinline__ bool z_prefetch(const PassGeom& g) {
-  return (size_t)g.Nx * g.Ny * g.Zp * (9 * sizeof(double2)) > ((size_t)64 << 20);
-}
-// the next transform's two input lines
-template <typename C>
-__device__ __forceinline__ void prefetch_z_pair(const C* f1, const C* f2, const ZRun& r) {
-  if (NS3D_Z_L2PF == 0 || !r.ask) return;
-  prefetch_z_line(f1, r.base, r.Zc);
-  if (f2 != f1) prefetch_z_line(f2, r.base, r.Zc);
+__device__ __forceinline__ void prefetch_z_line(const C* row, int n) {
+  const uintptr_t b = (uintptr_t)row & ~(uintptr_t)15, e = (uintptr_t)(row + n) & ~(uintptr_t)15;
+  if (e > b) prefetch_l2_bulk((const void*)b, (unsigned)(e - b));
 }
 
 // whether every thread's sample s (k = t + T s) is a kept mode
@@ -745,10 +711,10 @@ __host__ __device__ constexpr bool z_dead(int s) {
 
 // Load W[k] = H(X1)[k] + i H(X2)[k] for positions k = t + T s, where H is the
 // Hermitian extension of a z half-line (H[0], H[N/2] keep only real parts),
-// X = line (optionally times i kz).  Modes from Zc up are zero (the mask).
-template <int NZ, int P, bool IK1, bool IK2, typename C>
-__device__ __forceinline__ void load_pair(C (&w)[P], const C* __restrict__ f1,
-                                          const C* __restrict__ f2, size_t base, int t,
+// X = line (times i kz where IK1, IK2).  Modes from Zc up are zero (the mask).
+// STAGED: the rows are in shared memory, else in global memory.
+template <int NZ, int P, bool IK1, bool IK2, bool STAGED, typename C>
+__device__ __forceinline__ void load_pair(C (&w)[P], const C* f1, const C* f2, int t,
                                           RealOf<C> kfz, int Zc) {
   using Rt = RealOf<C>;
   constexpr int T = NZ / P;
@@ -763,8 +729,8 @@ __device__ __forceinline__ void load_pair(C (&w)[P], const C* __restrict__ f1,
     const int q = upper ? NZ - k : k;
     C c1 = mkc<C>((Rt)0, (Rt)0), c2 = c1;
     if (z_live<NZ, T>(s) || q < Zc) {
-      c1 = __ldg(f1 + base + q);
-      c2 = __ldg(f2 + base + q);
+      c1 = STAGED ? f1[q] : __ldg(f1 + q);
+      c2 = STAGED ? f2[q] : __ldg(f2 + q);
     }
     const Rt kz = kfz * (Rt)q;
     if constexpr (IK1) c1 = mkc<C>(-c1.y * kz, c1.x * kz);
@@ -785,11 +751,14 @@ __device__ __forceinline__ void load_pair(C (&w)[P], const C* __restrict__ f1,
 // W[N-k] (exchanged through shared memory) and store the half spectra
 // Q1h[k], Q2h[k] for k = 0..N/2.
 // Line-buffer index scheme of the z pass: the XOR swizzle for FP32 lines of
-// 128 points and more (fewer shared-memory wavefronts), the padding else.
+// 128 points and more (fewer shared-memory wavefronts); for FP64 lines of 512
+// points the swizzle by rows, as free of conflicts as the padding and without
+// its words (three CTAs then fit an SM); the padding else.
 template <int NZ, int P, typename C>
 __host__ __device__ constexpr int z_pw() {
-  return (sizeof(C) == 8 && P == 8 && (NZ & (NZ - 1)) == 0 && NZ >= 128)
-             ? 0 : LineFFT<NZ, P>::PADW;
+  return (sizeof(C) == 8 && P == 8 && (NZ & (NZ - 1)) == 0 && NZ >= 128) ? 0
+         : (sizeof(C) == 16 && P == 16 && NZ == 512)                     ? -1
+                                                     : LineFFT<NZ, P>::PADW;
 }
 
 template <int NZ, int P, typename C>
@@ -832,217 +801,160 @@ struct ZLaneMap {  // lanes of one line are adjacent: the line is contiguous in 
   }
 };
 
-// One component of B(u,v)_i = (v.grad) u_i + (u.grad) v_i in the z pass
-// (convolute_2p3_UV, Source/advection_2_3.cu:414-466); 3 paired C2R lines.
-template <int NZ, int P, typename C, typename Rt = RealOf<C>>
-__device__ __forceinline__ void uv_component(Rt (&q)[P], int i, const ZArgs<6, C>& a, size_t base,
-                                             int t, Rt kfz, Rt sc, C* sbuf,
-                                             const C* tw_s, const Rt (&ux)[P],
-                                             const Rt (&uy)[P], const Rt (&uz)[P],
-                                             const Rt (&vx)[P], const Rt (&vy)[P],
-                                             const Rt (&vz)[P], const ZRun& run) {
-  using F = LineFFT<NZ, P>;
-  C w[P];
-  // (d_x u_i, d_y u_i)
-  prefetch_z_pair(a.C[i], a.E[3 + i], run);
-  load_pair<NZ, P, false, false>(w, a.E[i], a.D[i], base, t, kfz, run.Zc);
-  F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-  for (int s = 0; s < P; ++s) q[s] = vx[s] * (w[s].x * sc) + vy[s] * (w[s].y * sc);
-  // (d_z u_i, d_x v_i)
-  prefetch_z_pair(a.D[3 + i], a.C[3 + i], run);
-  load_pair<NZ, P, true, false>(w, a.C[i], a.E[3 + i], base, t, kfz, run.Zc);
-  F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-  for (int s = 0; s < P; ++s) {
-    q[s] = q[s] + vz[s] * (w[s].x * sc);
-    q[s] = q[s] + ux[s] * (w[s].y * sc);
-  }
-  // (d_y v_i, d_z v_i)
-  if (i < 2) prefetch_z_pair(a.E[i + 1], a.D[i + 1], run);
-  load_pair<NZ, P, false, true>(w, a.D[3 + i], a.C[3 + i], base, t, kfz, run.Zc);
-  F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-  for (int s = 0; s < P; ++s) q[s] = q[s] + (uy[s] * (w[s].x * sc) + uz[s] * (w[s].y * sc));
-}
+// ---------------------------------------------------------------------------
+// z pass: C2R along z of the paired rows, the products, R2C along z.
+//
+// What bounds it is its line transforms: the FP64 pipe and the shared memory the
+// exchanges and rows pass through (59% and 66% busy at 256^3 FP64).  Each
+// Stockham exchange moves the whole line through shared memory, so 16 points
+// per thread (one exchange at 256) beat 8 (two): 503 against 534 us per launch.
+// The rest of the form gets 12 warps per SM to run at 16 points per thread:
+//  * the velocities and the d_z terms wait in tensor memory (tcgen05.st / ld;
+//    each thread parks its own samples, no other thread reads them, so no
+//    barrier), the fifth component in a private shared-memory slot
+//    ([component][s][thread], conflict-free): 168 registers, 3 CTAs per SM.
+//    FP32 lines park the velocities in shared memory and keep the rest.
+//  * the rows a transform reads are staged by bulk copies (cp.async.bulk, one
+//    per field for a warp's consecutive rows, completed on an mbarrier), the
+//    next transform's while this one runs (96 to 384 points; ZSmem::STAGE).
+//  * the six inverse transforms are one loop: unrolled, the eight transforms
+//    outgrow the instruction cache (435 us against 379, a third of all stalls
+//    waiting for instructions).
+// Per launch on a B200 (plain loads behind L2 prefetches, unrolled, stash in
+// shared memory, 8 warps per SM -> this form): FP64 256^3 403 -> 379 us, 128^3
+// 62.4 -> 56.5; FP32 275 -> 229, 47.1 -> 37.9.
+//
+// The tangent form (z_uv_kernel) parks six velocities, keeps its products in
+// registers and stages its rows two transforms deep, 8 points per thread (12
+// for multiples of 3).  The linearised product, 4 (6) points and plain loads ->
+// this form: 128^3 495 -> 388 us, 96^3 251 -> 206.
+// ---------------------------------------------------------------------------
+// CTAs per SM the FP32 lines ask for (they take half the registers)
+#ifndef NS3D_MINCTA_Z32
+#define NS3D_MINCTA_Z32 4
+#endif
+// ... and the nonlinear term's FP64 lines, 168 registers at 3
+#ifndef NS3D_MINCTA_Z64
+#define NS3D_MINCTA_Z64 3
+#endif
 
 template <int NZ, int P, bool UV, typename C>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_kernel(ZArgs<UV ? 6 : 3, C> a, PassGeom g) {
-  using F = LineFFT<NZ, P>;
-  using Rt = RealOf<C>;
-  constexpr int T = F::T;
-  using LM = ZLaneMap<T>;
-  __shared__ C tw_s[F::TWLEN];
-  __shared__ C sbuf_all[LM::LPC][F::BUF];
-  F::load_tw(tw_s, a.tw);
-  int li, t;
-  LM::get(li, t);
-  const int nb = g.Nx * g.Ny;
-  const int b = blockIdx.x * LM::LPC + li;
-  const bool valid = b < nb;
-  const size_t base = (size_t)(valid ? b : 0) * g.Zp;   // C, D, E
-  const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
-  C* sbuf = sbuf_all[li];
-  const Rt sc = (Rt)g.inv_vol;
-  const Rt kfz = (Rt)g.kfz;
-  const ZRun run{base, g.Zc, valid && t == 0 && z_prefetch(g)};  // one transform ahead into L2
-  C w[P];
-  Rt ux[P], uy[P], uz[P], q0[P], q1[P], q2[P];
-  if constexpr (!UV) {
-    // Q_z first, so at most five real lines (u_x, u_y, u_z and two products)
-    // are live at any time.
-    // (u_x, u_y)
-    prefetch_z_pair(a.C[2], a.C[2], run);
-    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s) { ux[s] = w[s].x * sc; uy[s] = w[s].y * sc; }
-    // (u_z, d_z u_z) from one field
-    prefetch_z_pair(a.E[2], a.D[2], run);
-    load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s) { uz[s] = w[s].x * sc; q2[s] = w[s].y * sc; }
-    // Q_z = u_x d_x u_z + u_y d_y u_z + u_z d_z u_z  (calc_vels_nabla_vels)
-    prefetch_z_pair(a.E[0], a.D[0], run);
-    load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s)
-      q2[s] = ux[s] * (w[s].x * sc) + uy[s] * (w[s].y * sc) + uz[s] * q2[s];
-    // R2C of Q_z alone
-#pragma unroll
-    for (int s = 0; s < P; ++s) w[s] = mkc<C>(q2[s], (Rt)0);
-    F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-    if (valid) {
-#pragma unroll
-      for (int s = 0; s < P; ++s) {
-        const int k = t + T * s;
-        if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
-      }
-    }
-    // (d_z u_x, d_z u_y)
-    load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; q1[s] = w[s].y * sc; }
-    prefetch_z_pair(a.E[1], a.D[1], run);
-    load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s)
-      q0[s] = ux[s] * (w[s].x * sc) + uy[s] * (w[s].y * sc) + uz[s] * q0[s];
-    load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s)
-      q1[s] = ux[s] * (w[s].x * sc) + uy[s] * (w[s].y * sc) + uz[s] * q1[s];
-    // R2C of (Q_x, Q_y) packed
-#pragma unroll
-    for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
-    F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-    store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
-    return;
-  } else {
-    // B(u,v)_i = (v.grad) u_i + (u.grad) v_i; fields 0..2 are u, 3..5 are v
-    Rt vx[P], vy[P], vz[P];
-    prefetch_z_pair(a.C[2], a.C[3], run);
-    load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s) { ux[s] = w[s].x * sc; uy[s] = w[s].y * sc; }
-    prefetch_z_pair(a.C[4], a.C[5], run);
-    load_pair<NZ, P, false, false>(w, a.C[2], a.C[3], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s) { uz[s] = w[s].x * sc; vx[s] = w[s].y * sc; }
-    prefetch_z_pair(a.E[0], a.D[0], run);
-    load_pair<NZ, P, false, false>(w, a.C[4], a.C[5], base, t, kfz, run.Zc);
-    F::template run<+1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-#pragma unroll
-    for (int s = 0; s < P; ++s) { vy[s] = w[s].x * sc; vz[s] = w[s].y * sc; }
-    uv_component<NZ, P>(q0, 0, a, base, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, run);
-    uv_component<NZ, P>(q1, 1, a, base, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, run);
-    uv_component<NZ, P>(q2, 2, a, base, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, run);
-  }
-  // forward R2C along z: (Q0, Q1) packed, then Q2 alone
-#pragma unroll
-  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
-  F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
-#pragma unroll
-  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q2[s], (Rt)0);
-  F::template run<-1, z_pw<NZ, P, C>()>(w, t, sbuf, tw_s);
-  if (valid) {
-#pragma unroll
-    for (int s = 0; s < P; ++s) {
-      const int k = t + T * s;
-      if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// z pass with the physical velocities stashed in shared memory (the nonlinear
-// term; the tangent form keeps z_kernel).
-//
-// The line transforms are what bound the z pass: each Stockham exchange moves
-// the whole line through shared memory, so at 8 points per thread a 256-point
-// line takes two exchanges per transform (16 per line and pass) and the
-// shared-memory pipe, not HBM, sets the pace.  With 16 points per thread the
-// same transform needs one exchange, but u_x, u_y, u_z, two products and the
-// line no longer fit in registers.  Here each thread parks its own P samples
-// of u_x, u_y, u_z in a private shared-memory slot ([component][s][thread]:
-// the lanes of a warp touch consecutive words, conflict-free) right after
-// their transforms and reads them back for each product; no other thread
-// reads them, so no barrier is needed.  The arithmetic of every product is
-// the one z_kernel does.
-// ---------------------------------------------------------------------------
-template <int NZ, int P, typename C>
-struct ZStashSmem {
+struct ZSmem {
   using F = LineFFT<NZ, P>;
   using LM = ZLaneMap<F::T>;
   using Rt = RealOf<C>;
+  // the stash: in tensor memory for FP64 lines (the nonlinear term's fifth
+  // component, beyond 128 columns, in shared memory), in shared memory for FP32
+  static constexpr bool TM = sizeof(C) == 16 && (UV || NZ > 64);
+  // rows staged by bulk copies; else (short lines, whose transforms are over
+  // before a copy is) read where they are used
+  static constexpr bool STAGE = UV || NZ > 64;
+  static constexpr int NTM = TM ? (UV ? 6 : 4) : 0;
+  static constexpr int NST = TM ? (UV ? 0 : 1) : (UV ? 6 : 3);
+  static constexpr int NSLOT = UV ? 2 : (STAGE ? 1 : 0);  // staging slots
+  // a group: the lines of a warp, or a line of several warps
+  static constexpr int GT = F::T > 32 ? F::T : 32;  // its threads
+  static constexpr int GL = GT / F::T;              // its lines
+  static constexpr int NG = kThreads / GT;
+  // a staged row: Zp elements, at most zc_max rounded up to whole blocks of 8;
+  // only the Zc kept ones where a row is copied by itself (FP64)
+  static constexpr bool KEPT = GL == 1 && sizeof(C) == 16;
+  static constexpr int ROW = KEPT ? zc_max(NZ) : (zc_max(NZ) + 7) / 8 * 8;
+  static constexpr size_t SLOT = (size_t)2 * GL * ROW * sizeof(C);  // two fields of a group
+  // line buffers: the spare word behind a line only staggers the banks of
+  // lines that share a quarter warp (fewer than 4 threads each)
+  static constexpr int BUF =
+      z_pw<NZ, P, C>() < 0 ? NZ : (F::T >= 4 ? F::BUF - 1 : F::BUF);
   static constexpr size_t SBUF_OFF = align16((size_t)F::TWLEN * sizeof(C));
-  static constexpr size_t ST_OFF = align16(SBUF_OFF + (size_t)LM::LPC * F::BUF * sizeof(C));
-  static constexpr size_t BYTES = ST_OFF + (size_t)3 * P * kThreads * sizeof(Rt);
-  static_assert(BYTES <= 113 * 1024, "two CTAs per SM");
-  // The TMEM form (NS3D_Z_TMEM) keeps the stash in tensor memory instead:
-  // TM_COLS columns per CTA (3 P doubles per thread = 6 P words, rounded up
-  // to a power of two).  Its launch asks for at least TM_BYTES of shared
-  // memory, which caps the CTAs per SM that hold columns at
-  // kTmemColsPerSm / TM_COLS, so an allocation never waits for good.
-  static constexpr uint32_t TM_COLS = 6 * P <= 32 ? 32 : (6 * P <= 64 ? 64 : (6 * P <= 128 ? 128 : 256));
+  static constexpr size_t SLOT_OFF = align16(SBUF_OFF + (size_t)LM::LPC * BUF * sizeof(C));
+  static constexpr size_t ST_OFF = SLOT_OFF + NSLOT * NG * SLOT;
+  static constexpr size_t BAR_OFF = ST_OFF + (size_t)NST * P * kThreads * sizeof(Rt);
+  static constexpr size_t BAD_OFF = BAR_OFF + (size_t)NSLOT * NG * 8;
+  static constexpr size_t USED = STAGE ? BAD_OFF + 8 : BAR_OFF;
+  // Tensor memory: TM_COLS columns per CTA (2 NTM P words per thread, rounded
+  // up to a power of two).  The launch asks for at least enough shared memory
+  // to cap the CTAs per SM that hold columns at kTmemColsPerSm / TM_COLS; an
+  // allocation can then only wait for CTAs of another launch, which end by
+  // themselves.
+  static constexpr int W = 2 * NTM * P;
+  static constexpr uint32_t TM_COLS = W <= 32 ? 32 : (W <= 64 ? 64 : (W <= 128 ? 128 : 256));
   static constexpr int TM_MAXCTAS = (int)(kTmemColsPerSm / TM_COLS);
-  static constexpr size_t TM_BYTES =
-      BYTES > (228 * 1024) / (TM_MAXCTAS + 1) + 1 ? BYTES : (228 * 1024) / (TM_MAXCTAS + 1) + 1;
-  static_assert(sizeof(Rt) == 8, "the TMEM form holds FP64 stash words in pairs");
-  static_assert(P % 4 == 0 && 6 * P <= 256, "TMEM stash columns");
-  static_assert((TM_BYTES + 1024) * (TM_MAXCTAS + 1) > 228 * 1024, "CTAs per SM bound");
+  static constexpr size_t TM_MIN = (228 * 1024) / (TM_MAXCTAS + 1) + 1;
+  static constexpr size_t BYTES = TM && USED < TM_MIN ? TM_MIN : USED;
+  static_assert(!TM || (P % 4 == 0 && W <= 256), "tensor-memory columns");
+  static_assert(!TM || (BYTES + 1024) * (TM_MAXCTAS + 1) > 228 * 1024, "CTAs per SM bound");
+  static_assert(BYTES <= 113 * 1024, "two CTAs per SM");
+  // CTAs per SM asked of ptxas: as many as wanted where the shared memory fits
+  static constexpr int WANT = sizeof(C) == 8 ? NS3D_MINCTA_Z32 : (UV ? (P <= 8 ? 3 : 2) : (TM ? NS3D_MINCTA_Z64 : kMinCtasZ));
+  static constexpr int fit(int n) {
+    return n <= kMinCtasZ || (BYTES + 1024) * n <= 228 * 1024 ? n : fit(n - 1);
+  }
+  static constexpr int MINC = fit(WANT);
 };
 
-// Where the nonlinear term's z pass keeps its velocity stash: 0 in shared
-// memory, 1 in tensor memory, 2 in tensor memory for z extents from 512.
-// Measured on a B200 (z pass per launch, shared / tensor memory): 128^3
-// 69.4 / 71.5 us, 256^3 453.5 / 457 us, 512^3 4553 / 4453 us.
-#ifndef NS3D_Z_TMEM
-#define NS3D_Z_TMEM 2
-#endif
-__host__ __device__ constexpr bool z_tmem(int nz) {
-  return NS3D_Z_TMEM == 1 || (NS3D_Z_TMEM == 2 && nz >= 512);
+// a stage number known at compile time
+template <int K>
+struct Stage {
+  __host__ __device__ constexpr operator int() const { return K; }
+};
+
+// bulk copy of `bytes` (a multiple of 16) from 16-byte aligned global memory,
+// completing on `bar`
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes,
+                                          uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
 }
 
-template <int NZ, int P, typename C, bool TM = false>
-__global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel_st(ZArgs<3, C> a, PassGeom g) {
+template <int NZ, int P, typename C>
+__global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, false, C>::MINC))
+    z_kernel(const __grid_constant__ ZArgs<3, C> a, PassGeom g) {
   using F = LineFFT<NZ, P>;
   using Rt = RealOf<C>;
-  using S = ZStashSmem<NZ, P, C>;
+  using S = ZSmem<NZ, P, false, C>;
+  constexpr bool TM = S::TM, STAGE = S::STAGE;
   constexpr int T = F::T;
   using LM = ZLaneMap<T>;
   constexpr int PW = z_pw<NZ, P, C>();
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ uint32_t tm_base_s;  // TMEM address of the CTA's columns (TM)
   const int warp = threadIdx.x >> 5;
+  int li, t;
+  LM::get(li, t);
+  const int nb = g.Nx * g.Ny;
+  const int b = blockIdx.x * LM::LPC + li;
+  const bool valid = b < nb;
+  const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
+  // staging: this thread's group of GL consecutive lines and its slot
+  constexpr int GL = S::GL;
+  const int grp = threadIdx.x / S::GT;
+  const int gt = threadIdx.x % S::GT;
+  const int row = li % GL;
+  const int b0 = blockIdx.x * LM::LPC + (li - row);  // the group's first line
+  const int nrow = nb - b0 < GL ? (nb - b0 > 0 ? nb - b0 : 0) : GL;
+  C* slot = (C*)(dsm + S::SLOT_OFF) + (size_t)grp * (S::SLOT / sizeof(C));
+  uint64_t* bar = (uint64_t*)(dsm + S::BAR_OFF) + grp;
+  volatile int* bad = (volatile int*)(dsm + S::BAD_OFF);  // a wait of this CTA gave up
+  if (STAGE && threadIdx.x == 0) *bad = 0;
+  const size_t field2 = S::KEPT ? (size_t)S::ROW : (size_t)GL * g.Zp;  // the second field's rows
+  // copies the rows of one transform (the group's first thread)
+  auto stage = [&](const C* f1, const C* f2) {
+    const uint32_t bytes = (uint32_t)(nrow * (S::KEPT ? g.Zc : g.Zp)) * (uint32_t)sizeof(C);
+    const size_t off = (size_t)b0 * g.Zp;
+    mbar_expect_tx(bar, f1 != f2 ? 2 * bytes : bytes);
+    if (bytes) {
+      bulk_load(slot, f1 + off, bytes, bar);
+      if (f1 != f2) bulk_load(slot + field2, f2 + off, bytes, bar);
+    }
+  };
+  if (STAGE && gt == 0) {
+    mbar_init(bar, 1);
+    mbar_init_fence();
+    stage(a.C[0], a.C[1]);  // in flight while the twiddles are read
+  }
   if constexpr (TM) {
     if (warp == 0) tmem_alloc_warp(&tm_base_s, S::TM_COLS);
     tmem_fence_before_sync();
@@ -1054,27 +966,274 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel_st(ZArgs<3, C> a
     tmem_fence_after_sync();
     tm = tmem_addr(tm_base_s, 32 * (warp & 3), 0);
   }
+  C* sbuf = (C*)(dsm + S::SBUF_OFF) + li * S::BUF;
+  Rt* stash = (Rt*)(dsm + S::ST_OFF) + threadIdx.x;
+  const size_t base = (size_t)(valid ? b : 0) * g.Zp;  // this line's row
+  auto next = [&](const C* f1, const C* f2) {
+    if constexpr (GL == 1) line_sync<T>(); else __syncwarp();  // the group has read the slot
+    if (gt == 0 && !*bad) {
+      fence_proxy_async_smem();
+      stage(f1, f2);
+    }
+  };
+  // stash component c: the P values v(s)
+  auto park = [&](int c, auto v) {
+    if (c < S::NTM) {
+#pragma unroll
+      for (int s0 = 0; s0 < P; s0 += 4) {
+        uint32_t r[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double d = v(s0 + k);
+          r[2 * k] = (uint32_t)__double2loint(d);
+          r[2 * k + 1] = (uint32_t)__double2hiint(d);
+        }
+        tmem_st8(tm + (uint32_t)(c * 2 * P + 2 * s0), r);
+      }
+      tmem_wait_st();
+    } else {
+#pragma unroll
+      for (int s = 0; s < P; ++s) stash[((c - S::NTM) * P + s) * kThreads] = v(s);
+    }
+  };
+  // hands f(s, value) every sample of component c
+  auto parked = [&](int c, auto f) {
+    if (c < S::NTM) {
+#pragma unroll
+      for (int s0 = 0; s0 < P; s0 += 4) {
+        uint32_t r[8];
+        tmem_ld8(tm + (uint32_t)(c * 2 * P + 2 * s0), r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          f(s0 + k, (Rt)__hiloint2double((int)r[2 * k + 1], (int)r[2 * k]));
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < P; ++s) f(s, stash[((c - S::NTM) * P + s) * kThreads]);
+    }
+  };
+  const Rt sc = (Rt)g.inv_vol;
+  const Rt kfz = (Rt)g.kfz;
+  C w[P];
+  Rt q0[P], q1[P];
+  // q[s] = u_x(s) (w[s].x sc) + u_y(s) (w[s].y sc) + u_z(s) q[s]  (calc_vels_nabla_vels),
+  // q's d_z term parked as component cq where the stash is in tensor memory
+  auto product = [&](Rt (&q)[P], int cq) {
+    if constexpr (TM) {
+#pragma unroll
+      for (int s0 = 0; s0 < P; s0 += 4) {
+        uint32_t rx[8], ry[8], rz[8], rq[8];
+        tmem_ld8(tm + (uint32_t)(0 * 2 * P + 2 * s0), rx);
+        tmem_ld8(tm + (uint32_t)(1 * 2 * P + 2 * s0), ry);
+        tmem_ld8(tm + (uint32_t)(2 * 2 * P + 2 * s0), rz);
+        if (cq < S::NTM) tmem_ld8(tm + (uint32_t)(cq * 2 * P + 2 * s0), rq);
+        tmem_wait_ld();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int s = s0 + k;
+          const Rt vx = __hiloint2double((int)rx[2 * k + 1], (int)rx[2 * k]);
+          const Rt vy = __hiloint2double((int)ry[2 * k + 1], (int)ry[2 * k]);
+          const Rt vz = __hiloint2double((int)rz[2 * k + 1], (int)rz[2 * k]);
+          const Rt dz = cq < S::NTM ? __hiloint2double((int)rq[2 * k + 1], (int)rq[2 * k])
+                                    : stash[((cq - S::NTM) * P + s) * kThreads];
+          q[s] = vx * (w[s].x * sc) + vy * (w[s].y * sc) + vz * dz;
+        }
+      }
+    } else {
+      auto u = [&](int c, int s) -> Rt { return stash[(c * P + s) * kThreads]; };
+#pragma unroll
+      for (int s = 0; s < P; ++s)
+        q[s] = u(0, s) * (w[s].x * sc) + u(1, s) * (w[s].y * sc) + u(2, s) * q[s];
+    }
+  };
+  // rows read where they are used: worth an L2 prefetch where the nine fields
+  // are larger than what L2 keeps of them between inv_y and this pass
+  const bool ask = !STAGE && valid && t == 0 &&
+                   (size_t)nb * g.Zp * (9 * sizeof(C)) > ((size_t)64 << 20);
+  auto transform = [&](auto k) {
+    // stage k's fields: (C_0, C_1), (C_2, C_2), (E_2, D_2), (C_0, C_1), (E_0, D_0), (E_1, D_1)
+    auto f1 = [&](int n) { return n == 0 || n == 3 ? a.C[0] : (n == 1 ? a.C[2] : a.E[n < 3 ? 2 : n - 4]); };
+    auto f2 = [&](int n) { return n == 0 || n == 3 ? a.C[1] : (n == 1 ? a.C[2] : a.D[n < 3 ? 2 : n - 4]); };
+    auto load = [&](const C* r1, const C* r2) {
+      if (k == 1) {
+        load_pair<NZ, P, false, true, STAGE>(w, r1, r1, t, kfz, g.Zc);
+      } else if (k == 3) {
+        load_pair<NZ, P, true, true, STAGE>(w, r1, r2, t, kfz, g.Zc);
+      } else {
+        load_pair<NZ, P, false, false, STAGE>(w, r1, r2, t, kfz, g.Zc);
+      }
+    };
+    if constexpr (STAGE) {
+      mbar_wait(bar, (uint32_t)(k & 1), a.err, bad);
+      const C* r1 = slot + (size_t)row * g.Zp;
+      load(r1, r1 + field2);
+      // the next stage's copies into the same slot run under this transform
+      // and its product
+      if (k < 5) next(f1(k + 1), f2(k + 1));
+    } else {
+      if (ask && k < 5) {  // the next stage's rows into L2
+        prefetch_z_line(f1(k + 1) + base, g.Zc);
+        prefetch_z_line(f2(k + 1) + base, g.Zc);
+      }
+      load(f1(k) + base, f2(k) + base);
+    }
+    F::template run<+1, PW>(w, t, sbuf, tw_s);
+    if (k == 0) {  // (u_x, u_y)
+      park(0, [&](int s) { return w[s].x * sc; });
+      park(1, [&](int s) { return w[s].y * sc; });
+    } else if (k == 1) {  // (u_z, d_z u_z)
+      park(2, [&](int s) { return w[s].x * sc; });
+      if constexpr (TM) {
+        park(3, [&](int s) { return w[s].y * sc; });
+      } else {
+#pragma unroll
+        for (int s = 0; s < P; ++s) q0[s] = w[s].y * sc;
+      }
+    } else if (k == 2) {  // (d_x u_z, d_y u_z): Q_z and its R2C
+      product(q0, 3);
+#pragma unroll
+      for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], (Rt)0);
+      F::template run<-1, PW>(w, t, sbuf, tw_s);
+      if (valid) {
+#pragma unroll
+        for (int s = 0; s < P; ++s) {
+          const int kz = t + T * s;
+          if (kz <= NZ / 2) a.Qh[2][qbase + kz] = w[s];
+        }
+      }
+    } else if (k == 3) {  // (d_z u_x, d_z u_y)
+      if constexpr (TM) {
+        park(3, [&](int s) { return w[s].x * sc; });
+        park(4, [&](int s) { return w[s].y * sc; });
+      } else {
+#pragma unroll
+        for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; q1[s] = w[s].y * sc; }
+      }
+    } else if (k == 4) {  // (d_x u_x, d_y u_x)
+      product(q0, 3);
+      if constexpr (TM) park(3, [&](int s) { return q0[s]; });  // Q_x, until Q_y joins it
+    } else {  // (d_x u_y, d_y u_y)
+      product(q1, 4);
+    }
+  };
+  // Short lines stay written out: a transform of 64 points is small, and where
+  // one thread holds a line (NZ = P) a loop would part the first butterflies
+  // from the i kz products they fuse with.
+  if constexpr (NZ <= 64) {
+    transform(Stage<0>{});
+    transform(Stage<1>{});
+    transform(Stage<2>{});
+    transform(Stage<3>{});
+    transform(Stage<4>{});
+    transform(Stage<5>{});
+  } else {
+#pragma unroll 1
+    for (int k = 0; k < 6; ++k) transform(k);
+  }
+  if (STAGE && gt == 0 && *bad) mbar_drain(bar, 1);  // a broken ring: the last copies may be in flight
+  if constexpr (TM) parked(3, [&](int s, Rt v) { q0[s] = v; });
+  // R2C of (Q_x, Q_y) packed
+#pragma unroll
+  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
+  F::template run<-1, PW>(w, t, sbuf, tw_s);
+  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
+  if constexpr (TM) {
+    // every thread's TMEM reads have completed (waited); free the columns
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    if (warp == 0) tmem_dealloc_warp(tm_base_s, S::TM_COLS);
+  }
+}
+
+// Stage k of the tangent z pass: the two rows it transforms.  The six
+// velocities in pairs, then per component i (d_x u_i, d_y u_i), (d_z u_i,
+// d_x v_i) with the first row times i kz, (d_y v_i, d_z v_i) with the second.
+template <typename C>
+struct ZStage {
+  static constexpr int N = 12;
+  const C* f1;
+  const C* f2;
+  int j;  // -1: velocities; else the place in a component's three
+  __device__ __forceinline__ ZStage(const ZArgs<6, C>& a, int k) {
+    if (k < 3) {
+      f1 = a.C[2 * k], f2 = a.C[2 * k + 1];
+      j = -1;
+    } else {
+      const int i = (k - 3) / 3;
+      j = k - 3 - 3 * i;
+      f1 = j == 0 ? a.E[i] : (j == 1 ? a.C[i] : a.D[3 + i]);
+      f2 = j == 0 ? a.D[i] : (j == 1 ? a.E[3 + i] : a.C[3 + i]);
+    }
+  }
+};
+
+template <int NZ, int P, typename C>
+__global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, true, C>::MINC))
+    z_uv_kernel(const __grid_constant__ ZArgs<6, C> a, PassGeom g) {
+  using F = LineFFT<NZ, P>;
+  using Rt = RealOf<C>;
+  using S = ZSmem<NZ, P, true, C>;
+  using St = ZStage<C>;
+  constexpr int T = F::T;
+  constexpr bool TM = S::TM;
+  using LM = ZLaneMap<T>;
+  constexpr int PW = z_pw<NZ, P, C>();
+  extern __shared__ __align__(16) unsigned char dsm[];
+  __shared__ uint32_t tm_base_s;  // TMEM address of the CTA's columns (TM)
+  const int warp = threadIdx.x >> 5;
   int li, t;
   LM::get(li, t);
   const int nb = g.Nx * g.Ny;
   const int b = blockIdx.x * LM::LPC + li;
   const bool valid = b < nb;
-  const size_t base = (size_t)(valid ? b : 0) * g.Zp;   // C, D, E
   const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
-  C* sbuf = (C*)(dsm + S::SBUF_OFF) + li * F::BUF;
-  Rt* stash = (Rt*)(dsm + S::ST_OFF) + threadIdx.x;
-  const ZRun run{base, g.Zc, valid && t == 0 && z_prefetch(g)};
-  const C* order[9] = {a.C[0], a.C[1], a.C[2], a.E[2], a.D[2], a.E[0], a.D[0], a.E[1], a.D[1]};
-  auto pf = [&](int i) {
-    if (NS3D_Z_L2PF != 0 && run.ask) prefetch_z_line(order[i], run.base, run.Zc);
+  // staging: this thread's group of GL consecutive lines, its place in it, and
+  // the group's ring of two slots
+  constexpr int GL = S::GL;
+  const int grp = threadIdx.x / S::GT;
+  const int gt = threadIdx.x % S::GT;
+  const int row = li % GL;
+  const int b0 = blockIdx.x * LM::LPC + (li - row);  // the group's first line
+  const int nrow = nb - b0 < GL ? (nb - b0 > 0 ? nb - b0 : 0) : GL;
+  C* slots = (C*)(dsm + S::SLOT_OFF) + (size_t)grp * 2 * (S::SLOT / sizeof(C));
+  uint64_t* bar = (uint64_t*)(dsm + S::BAR_OFF) + 2 * grp;
+  volatile int* bad = (volatile int*)(dsm + S::BAD_OFF);  // a wait of this CTA gave up
+  if (threadIdx.x == 0) *bad = 0;
+  if (gt == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init_fence();
+  }
+  const size_t field2 = S::KEPT ? (size_t)S::ROW : (size_t)GL * g.Zp;  // the second field's rows
+  // copies the rows of stage k into its slot (the group's first thread)
+  auto stage = [&](int k) {
+    const St s(a, k);
+    C* dst = slots + (k & 1) * (S::SLOT / sizeof(C));
+    const uint32_t bytes = (uint32_t)(nrow * (S::KEPT ? g.Zc : g.Zp)) * (uint32_t)sizeof(C);
+    const size_t off = (size_t)b0 * g.Zp;
+    mbar_expect_tx(&bar[k & 1], 2 * bytes);
+    if (bytes) {
+      bulk_load(dst, s.f1 + off, bytes, &bar[k & 1]);
+      bulk_load(dst + field2, s.f2 + off, bytes, &bar[k & 1]);
+    }
   };
-  if (NS3D_Z_L2PF == 1)
-    for (int i = 0; i < 9; ++i) pf(i);
-  if (NS3D_Z_L2PF == 2) { pf(0); pf(1); }  // C0, C1
-  auto ux = [&](int s) -> Rt& { return stash[(0 * P + s) * kThreads]; };
-  auto uy = [&](int s) -> Rt& { return stash[(1 * P + s) * kThreads]; };
-  auto uz = [&](int s) -> Rt& { return stash[(2 * P + s) * kThreads]; };
-  // stash component c (0 u_x, 1 u_y, 2 u_z): the P values v(s)
+  if (gt == 0) stage(0);  // in flight while the twiddles are read
+  if constexpr (TM) {
+    if (warp == 0) tmem_alloc_warp(&tm_base_s, S::TM_COLS);
+    tmem_fence_before_sync();
+  }
+  C* tw_s = (C*)dsm;
+  F::load_tw(tw_s, a.tw);  // ends with a CTA barrier: the TMEM address is published
+  uint32_t tm = 0;         // this warp's lane quarter, column 0
+  if constexpr (TM) {
+    tmem_fence_after_sync();
+    tm = tmem_addr(tm_base_s, 32 * (warp & 3), 0);
+  }
+  C* sbuf = (C*)(dsm + S::SBUF_OFF) + li * S::BUF;
+  Rt* stash = (Rt*)(dsm + S::ST_OFF) + threadIdx.x;
+  // stash component c: the P values v(s)
   auto park = [&](int c, auto v) {
     if constexpr (TM) {
 #pragma unroll
@@ -1094,81 +1253,104 @@ __global__ void __launch_bounds__(kThreads, kMinCtasZ) z_kernel_st(ZArgs<3, C> a
       for (int s = 0; s < P; ++s) stash[(c * P + s) * kThreads] = v(s);
     }
   };
-  const Rt sc = (Rt)g.inv_vol;
-  const Rt kfz = (Rt)g.kfz;
-  C w[P];
-  Rt q0[P], q1[P];
-  // q[s] = u_x(s) (w[s].x sc) + u_y(s) (w[s].y sc) + u_z(s) q[s]  (calc_vels_nabla_vels)
-  auto product = [&](Rt (&q)[P]) {
+  // hands f(s, values of the NC components from c0 on) every sample
+  auto parked = [&](auto nc, int c0, auto f) {
+    constexpr int NC = decltype(nc)::value;
     if constexpr (TM) {
 #pragma unroll
       for (int s0 = 0; s0 < P; s0 += 4) {
-        uint32_t rx[8], ry[8], rz[8];
-        tmem_ld8(tm + (uint32_t)(0 * 2 * P + 2 * s0), rx);
-        tmem_ld8(tm + (uint32_t)(1 * 2 * P + 2 * s0), ry);
-        tmem_ld8(tm + (uint32_t)(2 * 2 * P + 2 * s0), rz);
+        uint32_t r[NC][8];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) tmem_ld8(tm + (uint32_t)((c0 + c) * 2 * P + 2 * s0), r[c]);
         tmem_wait_ld();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const int s = s0 + k;
-          const Rt vx = __hiloint2double((int)rx[2 * k + 1], (int)rx[2 * k]);
-          const Rt vy = __hiloint2double((int)ry[2 * k + 1], (int)ry[2 * k]);
-          const Rt vz = __hiloint2double((int)rz[2 * k + 1], (int)rz[2 * k]);
-          q[s] = vx * (w[s].x * sc) + vy * (w[s].y * sc) + vz * q[s];
+          Rt v[NC];
+#pragma unroll
+          for (int c = 0; c < NC; ++c)
+            v[c] = __hiloint2double((int)r[c][2 * k + 1], (int)r[c][2 * k]);
+          f(s0 + k, v);
         }
       }
     } else {
 #pragma unroll
-      for (int s = 0; s < P; ++s)
-        q[s] = ux(s) * (w[s].x * sc) + uy(s) * (w[s].y * sc) + uz(s) * q[s];
+      for (int s = 0; s < P; ++s) {
+        Rt v[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) v[c] = stash[((c0 + c) * P + s) * kThreads];
+        f(s, v);
+      }
     }
   };
-  // (u_x, u_y)
-  if (NS3D_Z_L2PF == 2) pf(2);  // C2
-  load_pair<NZ, P, false, false>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
-  F::template run<+1, PW>(w, t, sbuf, tw_s);
-  park(0, [&](int s) { return w[s].x * sc; });
-  park(1, [&](int s) { return w[s].y * sc; });
-  // (u_z, d_z u_z); q0 accumulates Q_z first
-  if (NS3D_Z_L2PF == 2) { pf(3); pf(4); }  // E2, D2
-  load_pair<NZ, P, false, true>(w, a.C[2], a.C[2], base, t, kfz, run.Zc);
-  F::template run<+1, PW>(w, t, sbuf, tw_s);
-  park(2, [&](int s) { return w[s].x * sc; });
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, 2>;
+  const Rt sc = (Rt)g.inv_vol;
+  const Rt kfz = (Rt)g.kfz;
+  C w[P];
+  Rt q0[P], qy[P], qz[P];
+#pragma unroll 1
+  for (int k = 0; k < St::N; ++k) {
+    // the next stage's rows, into the slot of stage k - 1: the group's threads
+    // have read it (they have passed a barrier of its transform)
+    if constexpr (T == 1) __syncwarp();  // (one-stage transforms have none)
+    if (gt == 0 && k + 1 < St::N && !*bad) {
+      fence_proxy_async_smem();
+      stage(k + 1);
+    }
+    mbar_wait(&bar[k & 1], (uint32_t)((k >> 1) & 1), a.err, bad);
+    {
+      const St st(a, k);
+      const C* f1 = slots + (k & 1) * (S::SLOT / sizeof(C)) + (size_t)row * g.Zp;  // (row 0 where GL = 1)
+      const C* f2 = f1 + field2;
+      if (st.j < 1)
+        load_pair<NZ, P, false, false, true>(w, f1, f2, t, kfz, g.Zc);
+      else if (st.j == 1)
+        load_pair<NZ, P, true, false, true>(w, f1, f2, t, kfz, g.Zc);
+      else
+        load_pair<NZ, P, false, true, true>(w, f1, f2, t, kfz, g.Zc);
+    }
+    F::template run<+1, PW>(w, t, sbuf, tw_s);
+    // B(u,v)_i = (v.grad) u_i + (u.grad) v_i (convolute_2p3_UV,
+    // Source/advection_2_3.cu:414-466); fields 0..2 are u, 3..5 are v
+    const int j = k < 3 ? -1 : (k - 3) % 3;
+    if (k < 3) {
+      park(2 * k, [&](int s) { return w[s].x * sc; });
+      park(2 * k + 1, [&](int s) { return w[s].y * sc; });
+    } else if (j == 0) {  // (d_x u_i, d_y u_i); the previous component moves on
 #pragma unroll
-  for (int s = 0; s < P; ++s) q0[s] = w[s].y * sc;
-  // Q_z = u_x d_x u_z + u_y d_y u_z + u_z d_z u_z
-  if (NS3D_Z_L2PF == 2) { pf(5); pf(6); }  // E0, D0
-  load_pair<NZ, P, false, false>(w, a.E[2], a.D[2], base, t, kfz, run.Zc);
-  F::template run<+1, PW>(w, t, sbuf, tw_s);
-  product(q0);
-  // R2C of Q_z alone
-#pragma unroll
-  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], (Rt)0);
-  F::template run<-1, PW>(w, t, sbuf, tw_s);
-  if (valid) {
-#pragma unroll
-    for (int s = 0; s < P; ++s) {
-      const int k = t + T * s;
-      if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
+      for (int s = 0; s < P; ++s) { q0[s] = qy[s]; qy[s] = qz[s]; }
+      parked(Two{}, 3, [&](int s, const Rt* v) {
+        qz[s] = v[0] * (w[s].x * sc) + v[1] * (w[s].y * sc);
+      });
+    } else if (j == 1) {  // (d_z u_i, d_x v_i)
+      parked(One{}, 5, [&](int s, const Rt* v) { qz[s] = qz[s] + v[0] * (w[s].x * sc); });
+      parked(One{}, 0, [&](int s, const Rt* v) { qz[s] = qz[s] + v[0] * (w[s].y * sc); });
+    } else {  // (d_y v_i, d_z v_i)
+      parked(Two{}, 1, [&](int s, const Rt* v) {
+        qz[s] = qz[s] + (v[0] * (w[s].x * sc) + v[1] * (w[s].y * sc));
+      });
     }
   }
-  // (d_z u_x, d_z u_y)
-  load_pair<NZ, P, true, true>(w, a.C[0], a.C[1], base, t, kfz, run.Zc);
-  F::template run<+1, PW>(w, t, sbuf, tw_s);
+  if (gt == 0 && *bad) {  // a broken ring: the last copies may still be in flight
+    mbar_drain(&bar[0], (uint32_t)(((St::N - 2) >> 1) & 1));
+    mbar_drain(&bar[1], (uint32_t)(((St::N - 1) >> 1) & 1));
+  }
+  // forward R2C along z: (Q_x, Q_y) packed, then Q_z alone
+#pragma unroll 1
+  for (int r = 0; r < 2; ++r) {
 #pragma unroll
-  for (int s = 0; s < P; ++s) { q0[s] = w[s].x * sc; q1[s] = w[s].y * sc; }
-  if (NS3D_Z_L2PF == 2) { pf(7); pf(8); }  // E1, D1
-  load_pair<NZ, P, false, false>(w, a.E[0], a.D[0], base, t, kfz, run.Zc);
-  F::template run<+1, PW>(w, t, sbuf, tw_s);
-  product(q0);
-  load_pair<NZ, P, false, false>(w, a.E[1], a.D[1], base, t, kfz, run.Zc);
-  F::template run<+1, PW>(w, t, sbuf, tw_s);
-  product(q1);
-  // R2C of (Q_x, Q_y) packed
+    for (int s = 0; s < P; ++s) w[s] = r == 0 ? mkc<C>(q0[s], qy[s]) : mkc<C>(qz[s], (Rt)0);
+    F::template run<-1, PW>(w, t, sbuf, tw_s);
+    if (r == 0) {
+      store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
+    } else if (valid) {
 #pragma unroll
-  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
-  F::template run<-1, PW>(w, t, sbuf, tw_s);
-  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
+      for (int s = 0; s < P; ++s) {
+        const int k = t + T * s;
+        if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
+      }
+    }
+  }
   if constexpr (TM) {
     // every thread's TMEM reads have completed (waited); free the columns
     tmem_fence_before_sync();

@@ -161,6 +161,7 @@ ns3d_status conv_front_t(ns3d_solver* h, const double2* const u[3],
     ax.qcut = h->qcut; ax.tw = h->tw[0];
     ay.tw = h->tw[1];
     az.tw = h->tw[2];
+    az.err = h->dev_err;
     if (sizeof(C) == 16 && g.tile[ns3d::kTileInvY] == 2) {  // FP64: the bulk-copy form
       ay.maps = h->ymaps;
       ay.err = h->dev_err;
@@ -185,6 +186,7 @@ ns3d_status conv_front_t(ns3d_solver* h, const double2* const u[3],
     ax.qcut = h->qcut; ax.tw = h->tw[0];
     ay.tw = h->tw[1];
     az.tw = h->tw[2];
+    az.err = h->dev_err;
     NS3D_CHECK(h, ns3d::run_inv_x(ax, g, st), "inv_x(uv)");
     NS3D_CHECK(h, ns3d::run_inv_y(ay, g, st), "inv_y(uv)");
     NS3D_CHECK(h, ns3d::run_z(az, g, st), "z(uv)");
@@ -1340,7 +1342,7 @@ ns3d_status profile_passes_t(ns3d_solver* h, const ns3d_complex* ux, const ns3d_
     fx.fd[i] = h->f_dense[0] ? h->f_dense[i] : nullptr;
   }
   ax.qcut = h->qcut; ax.tw = h->tw[0];
-  ay.tw = h->tw[1]; az.tw = h->tw[2]; fy.tw = h->tw[1]; fx.tw = h->tw[0];
+  ay.tw = h->tw[1]; az.tw = h->tw[2]; az.err = h->dev_err; fy.tw = h->tw[1]; fx.tw = h->tw[0];
   if (sizeof(C) == 16 && g.tile[ns3d::kTileInvY] == 2) {  // as conv_front
     ay.maps = h->ymaps;
     ay.err = h->dev_err;
