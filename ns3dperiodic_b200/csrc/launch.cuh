@@ -343,33 +343,21 @@ cudaError_t launch_fwd_x_p(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t
   return cudaGetLastError();
 }
 
-// fwd_x with the update operands in the prefetch ring (fwd_x_ring_kernel):
-// 8 points per thread for powers of two, 12 for multiples of 3, and as many
-// slots as two CTAs per SM leave room for; used where a line fits in a warp
-// (to 256 and 384 points).  At 512 points the ring's lines would spread over
-// the CTA two at a time (32-byte rows): measured 4.69 ms per launch
-// there against 3.42 ms for fwd_x_kernel with 16 points per thread.
-#ifndef NS3D_FX_RING
-#define NS3D_FX_RING 1
-#endif
-#ifndef NS3D_FX_RING32
-#define NS3D_FX_RING32 1
-#endif
+// fwd_x with the update operands in the prefetch ring (fwd_x_ring_kernel), at
+// 8 points per thread where a line then fills a warp (256) or its wider tile
+// would stay inside a warp (to 64), 16 at 128 and 512, whose lines interleaved
+// over the CTA read wider rows that way (per plain launch at 512^3: 16 points
+// 3.42 ms, 8 points 4.69), 12 for multiples of 3.  The 12-point lines spread
+// over the CTA (96, 192) keep fwd_x_kernel: 25.8 against 26.7 us at 96^3 (FP32
+// lines 22.5 against 25.8).
 #ifndef NS3D_PFXR
 #define NS3D_PFXR 8
 #endif
-constexpr int p_fxr(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PFXR); }
-constexpr int nslot_fxr(int p) { return p > 8 ? 3 : NS3D_FX_SLOTS; }
-// The ring where its lines are a warp wide (64-byte rows over the CTA), or
-// where fwd_x_kernel's own lines would stay inside their warps; elsewhere
-// fwd_x_kernel's lines, interleaved over the CTA, read wider rows than the
-// ring's.  Per plain launch on a B200: 256^3 ring 295 us, fwd_x_kernel (16
-// points) 383 us; 128^3 ring 65.5 us, fwd_x_kernel 61.7 us.
-template <int N, typename C>
-constexpr bool fx_use_ring() {
-  return NS3D_FX_RING && N / p_fxr(N) <= 32 && (NS3D_FX_RING32 || sizeof(C) == 16) &&
-         (N / p_fxr(N) == 32 || N / p_fx(N) < NS3D_SPREAD_T);
+constexpr int p_fxr(int n) {
+  return n % 3 == 0 ? 12 : (n == 128 || n == 512) ? 16 : p_pow2(n, NS3D_PFXR);
 }
+constexpr int nslot_fxr(int p) { return p > 12 ? 2 : (p > 8 ? 3 : NS3D_FX_SLOTS); }
+constexpr bool fx_use_ring(int n) { return n % 3 != 0 || n / 12 < NS3D_SPREAD_T || n / 12 >= 32; }
 
 template <int N, int P, int MODE, bool COMBINE, typename C>
 cudaError_t launch_fwd_x_ring(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t st,
@@ -396,7 +384,7 @@ cudaError_t launch_fwd_x(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t s
       if (g.tile[kTileFwdX])                                                          \
         return launch_fwd_x_p<N, p_alt(N), MODE, COMBINE, C>(a, g, st, prepare_only); \
     }                                                                                 \
-    if constexpr (fx_use_ring<N, C>())                                                \
+    if constexpr (fx_use_ring(N))                                                \
       return launch_fwd_x_ring<N, p_fxr(N), MODE, COMBINE, C>(a, g, st, prepare_only); \
     return launch_fwd_x_p<N, p_fx(N), MODE, COMBINE, C>(a, g, st, prepare_only);
     NS3D_FOR_EACH_EXTENT(NS3D_CASE)

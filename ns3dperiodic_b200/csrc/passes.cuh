@@ -1838,27 +1838,32 @@ __global__ void __launch_bounds__(kThreads, kMinCtasFwdX) fwd_x_kernel(FwdXArgs<
 // ---------------------------------------------------------------------------
 // fwd_x with the update's operands in the prefetch ring.
 //
-// fwd_x_kernel reads the state (and RK partner) samples of its update with
-// plain loads after the three transforms, two points at a time: every group
-// waits several memory round trips with little in flight.  Here the unit
-// sequence of a group is Qh_x, Qh_y, Qh_z (transformed), then u^s_c (and
-// u^n_c when combining) for c = x, y, z, and every unit goes through one ring
-// of NSLOT per-thread cp.async slots, issued NSLOT - 1 units ahead.  The
-// update runs component by component as its operands arrive: component c of
-// the update needs only u^s_c (u^n_c) and the three transformed products,
-// whose Leray term k (k.Q)/|k|^2 is formed once per point.  Slots hold one
-// 16-byte cell per sample and thread (the state is FP64 in both precisions):
-// an FP32 product sample sits in the first half of its thread's cell, so a
-// slot stays private to each thread whichever kind of unit it holds (with
-// 8-byte product cells a thread's cell would overlap another warp's, and a
-// warp that runs ahead would overwrite samples not yet read).  Arithmetic
-// per point as in fwd_x_line.
+// What bounds it is the latency of its 9 (12) streams.  fwd_x_kernel reads the
+// state (and RK partner) samples of its update with plain loads after the three
+// transforms, two points at a time: every group waits several memory round
+// trips with little in flight.  Here the unit sequence of a group of lines is
+// Qh_x, Qh_y, Qh_z (transformed), then the update's operands for c = x, y, z:
+// u^s_c, or, when combining, u^s_c and u^n_c for half of the points at a time.
+// Every unit fills one slot of P 16-byte cells per thread (private to the
+// thread; the state is FP64 in both precisions, an FP32 product sample takes
+// half of its cell), and units are issued NSLOT - 1 ahead, so the copies of one
+// unit run under the work on the others.  The update runs component by
+// component as its operands arrive; the Leray term k (k.Q)/|k|^2 is formed once
+// per point.  FP64 lines do not unroll the loop over the components: three
+// copies of the update's code stall on instruction fetches (2.1 of 10 stall
+// cycles per issue at 256^3); FP32 lines of 8 and 12 points, whose transforms
+// are shorter, gain from the unrolled form (256^3: 278 against 299 us).  An in-place update is
+// safe: every element is copied once, by the thread that later writes it,
+// before it writes it.  Per plain FP64 launch on a B200 (unrolled, separate
+// units for u^n; 128^3 and 512^3: fwd_x_kernel -> this form): 128^3 56 -> 49
+// us, 256^3 277 -> 248, 512^3 3157 -> 2854, 384 x 48 x 192 131 -> 87.
 // ---------------------------------------------------------------------------
 // Ring depth of the 8-point lines and the CTAs per SM requested from ptxas:
 // 3 slots at 3 CTAs per SM (168 registers) measured 292 us per plain launch
 // at 256^3 against 399 us with 4 slots at 2 CTAs per SM.  Lines of 12 points
-// keep 3 slots; shapes whose shared memory does not fit 3 CTAs per SM (12
-// points, or the many short lines of 8-point extents) ask for 2.
+// keep 3 slots, 16 points 2 (32 KB each); shapes whose shared memory does not
+// fit 3 CTAs per SM (12 and 16 points, or the many short lines of 8-point
+// extents) ask for 2.
 #ifndef NS3D_FX_SLOTS
 #define NS3D_FX_SLOTS 3
 #endif
@@ -1891,7 +1896,10 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
   constexpr int T = F::T;
   constexpr int NUPD = MODE == kConvOut ? 0 : (COMBINE ? 6 : 3);
   constexpr int UPG = 3 + NUPD;  // units per group
-  static_assert(NSLOT >= 2 && (!COMBINE || NSLOT >= 3), "ring depth");
+  // The 16-point extents ran fwd_x_kernel before: its compiled form's choice of
+  // fused multiply-adds is written out for them, so their results keep every bit.
+  constexpr bool FUSED = P == 16;
+  static_assert(NSLOT >= 2 && P % 2 == 0, "ring depth, halves of a combining unit");
   extern __shared__ __align__(16) unsigned char dsm[];
   F::load_tw((C*)dsm, a.tw);
   const C* tw_s = (const C*)dsm;
@@ -1923,8 +1931,14 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
                                           (size_t)nlines, t);
       } else {
         const int u = j - 3;
-        const double2* src = COMBINE ? ((u & 1) ? a.un[u >> 1] : a.us[u >> 1]) : a.us[u];
-        issue_line<P, T>((double2*)sl + threadIdx.x, src, off, (size_t)nlines, t);
+        double2* cell = (double2*)sl + threadIdx.x;
+        if constexpr (COMBINE) {  // points (u & 1) P/2 ..: the state, then its partner
+          const size_t oh = off + (size_t)((u & 1) * (P / 2) * T) * nlines;
+          issue_line<P / 2, T>(cell, a.us[u >> 1], oh, (size_t)nlines, t);
+          issue_line<P / 2, T>(cell + P / 2 * kThreads, a.un[u >> 1], oh, (size_t)nlines, t);
+        } else {
+          issue_line<P, T>(cell, a.us[u], off, (size_t)nlines, t);
+        }
       }
     }
     cp_async_commit();
@@ -1990,65 +2004,67 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
       for (int s = 0; s < P; ++s) {
         const double kx = g.kfx * (double)signed_idx(t + T * s, NX);
         const double kk = kx * kx + ky * ky + kz * kz;
-        kq[s] = kk > 0.0 ? (kx * qi[0][s] + ky * qi[1][s] + kz * qi[2][s]) / kk : 0.0;
+        const double kQ = FUSED ? __fma_rn(kz, qi[2][s], __fma_rn(ky, qi[1][s], __dmul_rn(kx, qi[0][s])))
+                                : kx * qi[0][s] + ky * qi[1][s] + kz * qi[2][s];
+        kq[s] = kk > 0.0 ? kQ / kk : 0.0;
       }
-#pragma unroll
+      constexpr int UNROLL_C = sizeof(C) == 8 && P <= 12 ? 3 : 1;
+#pragma unroll UNROLL_C
       for (int c = 0; c < 3; ++c) {
-        // issued so far: units 0 .. k + NSLOT - 2; the next issue refills the
-        // slot of unit k - 1, consumed already
-        issue(k + NSLOT - 1);
-        // the combining form reads two units (u^s_c, u^n_c) at once: wait for
-        // both, and refill the first one's slot only after the update below
-        if constexpr (COMBINE) {
-          cp_async_wait<NSLOT - 2>();
-        } else {
-          cp_async_wait<NSLOT - 1>();
-        }
-        const double2* us = (const double2*)slot(k) + threadIdx.x;
-        const double2* un = COMBINE ? (const double2*)slot(k + 1) + threadIdx.x : us;
         const double kc = c == 0 ? 0.0 : (c == 1 ? ky : kz);
-        if (valid) {
+        constexpr int NH = COMBINE ? 2 : 1;  // units of a component
+        constexpr int PU = P / NH;           // points of a unit
 #pragma unroll
-        for (int s = 0; s < P; ++s) {
-          const int x = t + T * s;
-          const size_t fi = (size_t)x * nlines + L;  // index inside the instance (forcing)
-          const size_t idx = off + (size_t)x * nlines;
-          const double kx = g.kfx * (double)signed_idx(x, NX);
-          const double kk = kx * kx + ky * ky + kz * kz;
-          // AM.Q - Q, imaginary part only
-          const double pc = (c == 0 ? kx : kc) * kq[s] - qi[c][s];
-          double2 f = make_double2(0.0, 0.0);
-          if constexpr (MODE != kImplicit) {
-            if (dense_f) {
-              f = __ldg(a.fd[c] + fi);
-            } else if (line_f) {
-              for (int e = 0; e < a.fnnz; ++e)
-                if (__ldg(a.fidx + e) == (int)fi) f = cadd(f, __ldg(a.fval + 3 * e + c));
-            }
-          }
-          const double2 u = us[s * kThreads];
-          double2 r;
-          if constexpr (MODE == kExplicit) {
-            const double Gf = 1.0 - kk * dt / Re;
-            r = make_double2(Gf * u.x + dt * f.x, dt * pc + Gf * u.y + dt * f.y);
-          } else if constexpr (MODE == kRhs) {
-            const double Gf = -kk / Re;
-            r = make_double2(Gf * u.x + f.x, pc + Gf * u.y + f.y);
-          } else {
-            const double Gf = 1.0 + kk * dt / Re;
-            r = make_double2(u.x / Gf, (dt * pc + u.y) / Gf);
-          }
-          if constexpr (COMBINE) {
-            const double2 n = un[s * kThreads];
-            r = make_double2(a.ca * n.x + a.cb * r.x, a.ca * n.y + a.cb * r.y);
-          }
-          a.out[c][idx] = r;
-        }
-        }
-        ++k;
-        if constexpr (COMBINE) {
-          issue(k + NSLOT - 1);  // into the slot of u^s_c, read above
+        for (int h = 0; h < NH; ++h) {
+          // the next unit refills the slot of unit k - 1, consumed already
+          issue(k + NSLOT - 1);
+          cp_async_wait<NSLOT - 1>();
+          const double2* us = (const double2*)slot(k) + threadIdx.x;
+          const double2* un = us + PU * kThreads;  // COMBINE
           ++k;
+          if (!valid) continue;
+#pragma unroll
+          for (int i = 0; i < PU; ++i) {
+            const int s = h * PU + i;
+            const int x = t + T * s;
+            const size_t fi = (size_t)x * nlines + L;  // index inside the instance (forcing)
+            const size_t idx = off + (size_t)x * nlines;
+            const double kx = g.kfx * (double)signed_idx(x, NX);
+            const double kk = kx * kx + ky * ky + kz * kz;
+            // AM.Q - Q, imaginary part only
+            const double qc = c == 0 ? qi[0][s] : (c == 1 ? qi[1][s] : qi[2][s]);
+            const double pc = (c == 0 ? kx : kc) * kq[s] - qc;
+            double2 f = make_double2(0.0, 0.0);
+            if constexpr (MODE != kImplicit) {
+              if (dense_f) {
+                f = __ldg(a.fd[c] + fi);
+              } else if (line_f) {
+                for (int e = 0; e < a.fnnz; ++e)
+                  if (__ldg(a.fidx + e) == (int)fi) f = cadd(f, __ldg(a.fval + 3 * e + c));
+              }
+            }
+            const double2 u = us[i * kThreads];
+            double2 r;
+            if constexpr (MODE == kExplicit) {
+              const double Gf = 1.0 - kk * dt / Re;
+              r = FUSED ? make_double2(__fma_rn(Gf, u.x, __dmul_rn(dt, f.x)),
+                                       __fma_rn(dt, f.y, __fma_rn(Gf, u.y, __dmul_rn(dt, pc))))
+                        : make_double2(Gf * u.x + dt * f.x, dt * pc + Gf * u.y + dt * f.y);
+            } else if constexpr (MODE == kRhs) {
+              const double Gf = -kk / Re;
+              r = make_double2(Gf * u.x + f.x, pc + Gf * u.y + f.y);
+            } else {
+              const double Gf = 1.0 + kk * dt / Re;
+              r = make_double2(u.x / Gf, (dt * pc + u.y) / Gf);
+            }
+            if constexpr (COMBINE) {
+              const double2 n = un[i * kThreads];
+              r = FUSED ? make_double2(__fma_rn(a.ca, n.x, __dmul_rn(a.cb, r.x)),
+                                       __fma_rn(a.ca, n.y, __dmul_rn(a.cb, r.y)))
+                        : make_double2(a.ca * n.x + a.cb * r.x, a.ca * n.y + a.cb * r.y);
+            }
+            a.out[c][idx] = r;
+          }
         }
       }
     }
