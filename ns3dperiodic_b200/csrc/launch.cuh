@@ -154,6 +154,15 @@ inline unsigned persistent_grid(Kern kern, size_t smem, long long groups) {
   return (unsigned)(groups < cap ? (groups > 0 ? groups : 1) : cap);
 }
 
+// Whether the inv_x, inv_y and fwd_y passes give each CTA one field instead of
+// all of them: where the groups of lines alone leave SMs idle, the chain of
+// transforms a CTA runs one after the other is then a third (sixth) as long.
+// With more groups than SMs the CTAs' start (twiddles, tables) costs more than
+// the shorter chain gives.  The RK3 step on a B200, all fields / one per CTA:
+// 32^3 (16 to 18 groups) 144 / 109 us, 64^3 (48 to 66) 149 / 116; 96^3 (192 to
+// 294) 350 / 372.
+inline bool one_field_per_cta(long long groups) { return groups < 148; }
+
 // KTag's last argument separates the FP64 and FP32 instantiations.
 template <typename C>
 constexpr int prec_tag() { return sizeof(C) == 16 ? 0 : 100; }
@@ -163,10 +172,16 @@ cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStre
                            bool prepare_only) {
   const long long lines = 8LL * g.nlive * nbatch(g);
   using S = PassSmem<N, P, C, double2, V>;
+  const long long groups = (lines + S::LPC - 1) / S::LPC;
   const unsigned grid = persistent_grid<KTag<0, N, P, NF + prec_tag<C>() + 1000 * V>>(
-      inv_x_kernel<N, P, NF, C, V>, S::BYTES, (lines + S::LPC - 1) / S::LPC);
+      inv_x_kernel<N, P, NF, C, V>, S::BYTES, groups);
+  const unsigned grid1 = persistent_grid<KTag<60, N, P, NF + prec_tag<C>() + 1000 * V>>(
+      inv_x_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
   if (prepare_only) return cudaGetLastError();
-  inv_x_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
+  if (one_field_per_cta(groups))
+    inv_x_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);
+  else
+    inv_x_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
   return cudaGetLastError();
 }
 
@@ -259,10 +274,16 @@ cudaError_t launch_inv_y_p(const InvYArgs<NF, C>& a, const PassGeom& g, cudaStre
   }
   const long long lines = (long long)g.Nx * g.Zp;
   using S = PassSmem<N, P, C, C, V>;
+  const long long groups = (lines + S::LPC - 1) / S::LPC;
   const unsigned grid = persistent_grid<KTag<1, N, P, NF + prec_tag<C>() + 1000 * V>>(
-      inv_y_kernel<N, P, NF, C, V>, S::BYTES, (lines + S::LPC - 1) / S::LPC);
+      inv_y_kernel<N, P, NF, C, V>, S::BYTES, groups);
+  const unsigned grid1 = persistent_grid<KTag<61, N, P, NF + prec_tag<C>() + 1000 * V>>(
+      inv_y_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
   if (prepare_only) return cudaGetLastError();
-  inv_y_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
+  if (one_field_per_cta(groups))
+    inv_y_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);
+  else
+    inv_y_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
   return cudaGetLastError();
 }
 
@@ -399,10 +420,16 @@ cudaError_t launch_fwd_y_p(const FwdYArgs<C>& a, const PassGeom& g, cudaStream_t
                            bool prepare_only) {
   const long long lines = (long long)g.Nx * g.Mz;
   using S = PassSmem<N, P, C, C, V>;
+  const long long groups = (lines + S::LPC - 1) / S::LPC;
   const unsigned grid = persistent_grid<KTag<20, N, P, prec_tag<C>() + 1000 * V>>(
-      fwd_y_kernel<N, P, C, V>, S::BYTES, (lines + S::LPC - 1) / S::LPC);
+      fwd_y_kernel<N, P, C, V>, S::BYTES, groups);
+  const unsigned grid1 = persistent_grid<KTag<62, N, P, prec_tag<C>() + 1000 * V>>(
+      fwd_y_kernel<N, P, C, V, 1>, S::BYTES, groups);
   if (prepare_only) return cudaGetLastError();
-  fwd_y_kernel<N, P, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
+  if (one_field_per_cta(groups))
+    fwd_y_kernel<N, P, C, V, 1><<<dim3(grid1, 3), kThreads, S::BYTES, st>>>(a, g);
+  else
+    fwd_y_kernel<N, P, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
   return cudaGetLastError();
 }
 

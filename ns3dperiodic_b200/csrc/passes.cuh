@@ -276,8 +276,11 @@ struct InvXArgs {
   const double2* tw;
 };
 
-template <int NX, int P, int NF, typename C, int V = 0>
-__global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_x_kernel(InvXArgs<NF, C> a, PassGeom g) {
+// FPC: fields of a CTA (NF, or 1 with blockIdx.y the field; fields_per_cta)
+template <int NX, int P, int NF, typename C, int V = 0, int FPC = NF>
+__global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
+    inv_x_kernel(const __grid_constant__ InvXArgs<NF, C> a, PassGeom g) {
+  const int f0 = FPC == NF ? 0 : blockIdx.y * FPC;
   using S = PassSmem<NX, P, C, double2, V>;
   using F = typename S::F;
   using LM = typename S::LM;
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_x_kernel(InvXArg
   uint32_t keep;             // bit s: mode (t + T s, y, z) survives the 2/3 mask
   size_t off, out;           // the line's elements at x = 0
   bool valid = line(grp * LM::LPC + li, off, out, keep);
-  issue_line<P, T>(pf, a.in[0], off, (size_t)nlines, t, keep);
+  issue_line<P, T>(pf, a.in[f0], off, (size_t)nlines, t, keep);
   cp_async_commit();
   int ub = 0;
   for (; grp < g_end; grp += gr.step) {
@@ -329,13 +332,14 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_x_kernel(InvXArg
     bool valid_next = false;
     if (gn < g_end) valid_next = line(gn * LM::LPC + li, off_next, out_next, keep_next);
 #pragma unroll
-    for (int f = 0; f < NF; ++f) {
+    for (int i = 0; i < FPC; ++i) {
+      const int f = f0 + i;
       const double2* cur = pf + ub * (P * kThreads);
       double2* nxt = pf + (ub ^ 1) * (P * kThreads);
-      if (f + 1 < NF) {
+      if (i + 1 < FPC) {
         issue_line<P, T>(nxt, a.in[f + 1], off, (size_t)nlines, t, keep);
       } else if (gn < g_end) {
-        issue_line<P, T>(nxt, a.in[0], off_next, (size_t)nlines, t, keep_next);
+        issue_line<P, T>(nxt, a.in[f0], off_next, (size_t)nlines, t, keep_next);
       }
       cp_async_commit();
       cp_async_wait<1>();
@@ -397,8 +401,10 @@ struct InvYArgs {
   int* err = nullptr;  // error flag of the bulk-copy form's bounded waits
 };
 
-template <int NY, int P, int NF, typename C, int V = 0>
-__global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArgs<NF, C> a, PassGeom g) {
+template <int NY, int P, int NF, typename C, int V = 0, int FPC = NF>
+__global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
+    inv_y_kernel(const __grid_constant__ InvYArgs<NF, C> a, PassGeom g) {
+  const int f0 = FPC == NF ? 0 : blockIdx.y * FPC;
   using S = PassSmem<NY, P, C, C, V>;
   using F = typename S::F;
   using LM = typename S::LM;
@@ -428,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArg
   };
   uint32_t keep, keep_next = 0;  // rows inside the mask
   size_t base = line_base(grp, keep), basen = 0;
-  issue_line<P, T>(pf, a.A[0], base, stride, t, keep);
+  issue_line<P, T>(pf, a.A[f0], base, stride, t, keep);
   cp_async_commit();
   int ub = 0;
   for (; grp < g_end; grp += gr.step) {
@@ -436,7 +442,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArg
     const int gn = grp + gr.step;
     if (gn < g_end) basen = line_base(gn, keep_next);
 #pragma unroll 1  // one copy of the three transforms: nine (18) outgrow the instruction cache
-    for (int f = 0; f < NF; ++f) {
+    for (int i = 0; i < FPC; ++i) {
+      const int f = f0 + i;
       // unit A[f] -> C[f] = IFFT_y A, D[f] = IFFT_y(i ky A)
       {
         const C* cur = pf + ub * (P * kThreads);
@@ -469,10 +476,10 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) inv_y_kernel(InvYArg
       {
         const C* cur = pf + ub * (P * kThreads);
         C* nxt = pf + (ub ^ 1) * (P * kThreads);
-        if (f + 1 < NF) {
+        if (i + 1 < FPC) {
           issue_line<P, T>(nxt, a.A[f + 1], base, stride, t, keep);
         } else if (gn < g_end) {
-          issue_line<P, T>(nxt, a.A[0], basen, stride, t, keep_next);
+          issue_line<P, T>(nxt, a.A[f0], basen, stride, t, keep_next);
         }
         cp_async_commit();
         cp_async_wait<1>();
@@ -1369,8 +1376,10 @@ struct FwdYArgs {
   const double2* tw;
 };
 
-template <int NY, int P, typename C, int V = 0>
-__global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) fwd_y_kernel(FwdYArgs<C> a, PassGeom g) {
+template <int NY, int P, typename C, int V = 0, int FPC = 3>
+__global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
+    fwd_y_kernel(const __grid_constant__ FwdYArgs<C> a, PassGeom g) {
+  const int f0 = FPC == 3 ? 0 : blockIdx.y * FPC;
   using S = PassSmem<NY, P, C, C, V>;
   using F = typename S::F;
   using LM = typename S::LM;
@@ -1395,7 +1404,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) fwd_y_kernel(FwdYArg
     const int x = bc / g.Mz, z = bc - x * g.Mz;
     return (size_t)x * g.Ny * g.Mz + z;
   };
-  issue_line<P, T>(pf, a.Q[0], line_base(grp), stride, t);
+  issue_line<P, T>(pf, a.Q[f0], line_base(grp), stride, t);
   cp_async_commit();
   int ub = 0;
   for (; grp < g_end; grp += gr.step) {
@@ -1404,13 +1413,14 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P)) fwd_y_kernel(FwdYArg
     const int gn = grp + gr.step;
     const size_t basen = line_base(gn < g_end ? gn : grp);
 #pragma unroll
-    for (int f = 0; f < 3; ++f) {
+    for (int i = 0; i < FPC; ++i) {
+      const int f = f0 + i;
       const C* cur = pf + ub * (P * kThreads);
       C* nxt = pf + (ub ^ 1) * (P * kThreads);
-      if (f + 1 < 3) {
+      if (i + 1 < FPC) {
         issue_line<P, T>(nxt, a.Q[f + 1], base, stride, t);
       } else if (gn < g_end) {
-        issue_line<P, T>(nxt, a.Q[0], basen, stride, t);
+        issue_line<P, T>(nxt, a.Q[f0], basen, stride, t);
       }
       cp_async_commit();
       cp_async_wait<1>();
