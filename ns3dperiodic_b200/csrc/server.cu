@@ -201,7 +201,7 @@ ns3d_status jvp_step_active(ns3d_solver* h, double2* const u[3], double2* const 
   const double2* v1c[3] = {h->v1[0], h->v1[1], h->v1[2]};
   NS3D_TRY(conv_front(h, uc, vc));
   NS3D_TRY(finish(h, ns3d::kExplicit, false, vc, h->v1, nullptr, 0.0, 1.0, 0.0, 0.0));
-  NS3D_TRY(rk3_launches(h, u, 0.0, 0.0));
+  NS3D_TRY(rk3_launches(h, u, 0.0, 0.0, true));  // at the u the tangent transformed
   NS3D_TRY(conv_front(h, uc, v1c));
   NS3D_TRY(finish(h, ns3d::kExplicit, false, v1c, v, vc, 0.5, 0.5, 0.0, 0.0));
   return NS3D_OK;

@@ -139,68 +139,73 @@ ns3d_status ensure_uv_pool(ns3d_solver* h) {
   return NS3D_OK;
 }
 
-// inv_x -> inv_y -> z -> fwd_y: leaves the y,z-transformed products in A[0..2]
-// (FP64 scratch, or FP32 scratch in the precision mode).
-template <typename C>
-ns3d_status conv_front_t(ns3d_solver* h, const double2* const u[3],
-                         const double2* const v[3]) {
+// inv_x -> inv_y of NF fields into A .. E from field `at` on.
+template <int NF, typename C>
+ns3d_status transform_t(ns3d_solver* h, const double2* const* u, int at) {
   auto sc = [](double2* p) { return reinterpret_cast<C*>(p); };
   const PassGeom& g = h->geom;
-  cudaStream_t st = h->stream;
-  if (!v) {
-    InvXArgs<3, C> ax{};
-    InvYArgs<3, C> ay{};
-    ZArgs<3, C> az{};
-    for (int i = 0; i < 3; ++i) {
-      ax.in[i] = u[i]; ax.A[i] = sc(h->A[i]); ax.B[i] = sc(h->B[i]);
-      ay.A[i] = sc(h->A[i]); ay.B[i] = sc(h->B[i]);
-      ay.C[i] = sc(h->C[i]); ay.D[i] = sc(h->D[i]); ay.E[i] = sc(h->E[i]);
-      az.C[i] = sc(h->C[i]); az.D[i] = sc(h->D[i]); az.E[i] = sc(h->E[i]);
-      az.Qh[i] = sc(h->A[i]);
-    }
-    ax.qcut = h->qcut; ax.tw = h->tw[0];
-    ay.tw = h->tw[1];
-    az.tw = h->tw[2];
-    az.err = h->dev_err;
-    if (sizeof(C) == 16 && g.tile[ns3d::kTileInvY] == 2) {  // FP64: the bulk-copy form
-      ay.maps = h->ymaps;
-      ay.err = h->dev_err;
-    }
-    NS3D_CHECK(h, ns3d::run_inv_x(ax, g, st), "inv_x");
-    NS3D_CHECK(h, ns3d::run_inv_y(ay, g, st), "inv_y");
-    NS3D_CHECK(h, ns3d::run_z(az, g, st), "z");
-  } else {
-    ns3d_status s = ensure_uv_pool(h);
-    if (s != NS3D_OK) return s;
-    InvXArgs<6, C> ax{};
-    InvYArgs<6, C> ay{};
-    ZArgs<6, C> az{};
-    for (int i = 0; i < 6; ++i) {
-      ax.in[i] = i < 3 ? u[i] : v[i - 3];
-      ax.A[i] = sc(h->A[i]); ax.B[i] = sc(h->B[i]);
-      ay.A[i] = sc(h->A[i]); ay.B[i] = sc(h->B[i]);
-      ay.C[i] = sc(h->C[i]); ay.D[i] = sc(h->D[i]); ay.E[i] = sc(h->E[i]);
-      az.C[i] = sc(h->C[i]); az.D[i] = sc(h->D[i]); az.E[i] = sc(h->E[i]);
-    }
-    for (int i = 0; i < 3; ++i) az.Qh[i] = sc(h->A[i]);
-    ax.qcut = h->qcut; ax.tw = h->tw[0];
-    ay.tw = h->tw[1];
-    az.tw = h->tw[2];
-    az.err = h->dev_err;
-    NS3D_CHECK(h, ns3d::run_inv_x(ax, g, st), "inv_x(uv)");
-    NS3D_CHECK(h, ns3d::run_inv_y(ay, g, st), "inv_y(uv)");
-    NS3D_CHECK(h, ns3d::run_z(az, g, st), "z(uv)");
+  InvXArgs<NF, C> ax{};
+  InvYArgs<NF, C> ay{};
+  for (int i = 0; i < NF; ++i) {
+    const int f = at + i;
+    ax.in[i] = u[i]; ax.A[i] = sc(h->A[f]); ax.B[i] = sc(h->B[f]);
+    ay.A[i] = sc(h->A[f]); ay.B[i] = sc(h->B[f]);
+    ay.C[i] = sc(h->C[f]); ay.D[i] = sc(h->D[f]); ay.E[i] = sc(h->E[f]);
   }
-  FwdYArgs<C> fy{};
-  for (int i = 0; i < 3; ++i) fy.Q[i] = sc(h->A[i]);
-  fy.tw = h->tw[1];
-  NS3D_CHECK(h, ns3d::run_fwd_y(fy, g, st), "fwd_y");
+  ax.qcut = h->qcut; ax.tw = h->tw[0];
+  ay.tw = h->tw[1];
+  if (NF == 3 && at == 0 && sizeof(C) == 16 && g.tile[ns3d::kTileInvY] == 2) {
+    ay.maps = h->ymaps;  // the bulk-copy form (its tensor maps cover A, B of u)
+    ay.err = h->dev_err;
+  }
+  NS3D_CHECK(h, ns3d::run_inv_x(ax, g, h->stream), "inv_x");
+  NS3D_CHECK(h, ns3d::run_inv_y(ay, g, h->stream), "inv_y");
   return NS3D_OK;
 }
 
-ns3d_status conv_front(ns3d_solver* h, const double2* const u[3], const double2* const v[3]) {
-  return h->precision == NS3D_PRECISION_FP32 ? conv_front_t<float2>(h, u, v)
-                                             : conv_front_t<double2>(h, u, v);
+// z -> fwd_y of the nonlinear term (NF = 3) or B(u,v) (6) from C, D, E.
+template <int NF, typename C>
+ns3d_status products_t(ns3d_solver* h) {
+  auto sc = [](double2* p) { return reinterpret_cast<C*>(p); };
+  ZArgs<NF, C> az{};
+  for (int i = 0; i < NF; ++i) {
+    az.C[i] = sc(h->C[i]); az.D[i] = sc(h->D[i]); az.E[i] = sc(h->E[i]);
+  }
+  FwdYArgs<C> fy{};
+  for (int i = 0; i < 3; ++i) az.Qh[i] = fy.Q[i] = sc(h->A[i]);
+  az.tw = h->tw[2];
+  az.err = h->dev_err;
+  fy.tw = h->tw[1];
+  NS3D_CHECK(h, ns3d::run_z(az, h->geom, h->stream), "z");
+  NS3D_CHECK(h, ns3d::run_fwd_y(fy, h->geom, h->stream), "fwd_y");
+  return NS3D_OK;
+}
+
+// inv_x -> inv_y -> z -> fwd_y: leaves the y,z-transformed products in A[0..2]
+// (FP64 scratch, or FP32 scratch in the precision mode).  held: C, D, E hold
+// u's transforms already (the fields 0..2 of an earlier evaluation at this u,
+// with no other evaluation since), so only v's, if any, are made.
+template <typename C>
+ns3d_status conv_front_t(ns3d_solver* h, const double2* const u[3],
+                         const double2* const v[3], bool held) {
+  if (v) NS3D_TRY(ensure_uv_pool(h));
+  if (!v) {
+    if (!held) NS3D_TRY((transform_t<3, C>(h, u, 0)));
+    return products_t<3, C>(h);
+  }
+  if (held) {
+    NS3D_TRY((transform_t<3, C>(h, v, 3)));
+  } else {
+    const double2* uv[6] = {u[0], u[1], u[2], v[0], v[1], v[2]};
+    NS3D_TRY((transform_t<6, C>(h, uv, 0)));
+  }
+  return products_t<6, C>(h);
+}
+
+ns3d_status conv_front(ns3d_solver* h, const double2* const u[3], const double2* const v[3],
+                       bool held) {
+  return h->precision == NS3D_PRECISION_FP32 ? conv_front_t<float2>(h, u, v, held)
+                                             : conv_front_t<double2>(h, u, v, held);
 }
 
 // fwd_x + pointwise update on the products left by conv_front.
@@ -240,11 +245,11 @@ ns3d_status finish(ns3d_solver* h, int mode, bool forcing, const double2* const 
 
 // RK3_SSP (Source/RK_time_step.cu:310-327) with every stage fused:
 //   u1 = u + dt L(u); u2 = 3/4 u + 1/4 (u1 + dt L(u1)); u = 1/3 u + 2/3 (u2 + dt L(u2))
-ns3d_status rk3_launches(ns3d_solver* h, double2* const u[3], double dt, double Re) {
+ns3d_status rk3_launches(ns3d_solver* h, double2* const u[3], double dt, double Re, bool held) {
   const double2* uc[3] = {u[0], u[1], u[2]};
   const double2* u1c[3] = {h->u1[0], h->u1[1], h->u1[2]};
   const double2* u2c[3] = {h->u2[0], h->u2[1], h->u2[2]};
-  NS3D_TRY(conv_front(h, uc, nullptr));
+  NS3D_TRY(conv_front(h, uc, nullptr, held));
   NS3D_TRY(finish(h, ns3d::kExplicit, true, uc, h->u1, nullptr, 0.0, 1.0, dt, Re));
   NS3D_TRY(conv_front(h, u1c, nullptr));
   NS3D_TRY(finish(h, ns3d::kExplicit, true, u1c, h->u2, uc, 3.0 / 4.0, 1.0 / 4.0, dt, Re));
@@ -272,8 +277,10 @@ ns3d_status check_step(ns3d_solver* h, double dt, double Re) {
 void drop_graph(ns3d_solver* h) {
   if (h->rk3_exec) cudaGraphExecDestroy(h->rk3_exec);
   h->rk3_exec = nullptr;
-  if (h->jvp_exec) cudaGraphExecDestroy(h->jvp_exec);
-  h->jvp_exec = nullptr;
+  for (auto& e : h->jvp_exec) {
+    if (e) cudaGraphExecDestroy(e);
+    e = nullptr;
+  }
 }
 
 }  // namespace
@@ -896,54 +903,63 @@ ns3d_status ns3d_jvp_steps(ns3d_solver* h, ns3d_complex* ux, ns3d_complex* uy, n
   const double2* uc[3] = {u[0], u[1], u[2]};
   const double2* vc[3] = {v[0], v[1], v[2]};
   const double2* v1c[3] = {h->v1[0], h->v1[1], h->v1[2]};
-  // the 25 launches of one step
-  auto one = [&]() -> ns3d_status {
-    NS3D_TRY(conv_front(h, uc, vc));
+  // The 23 launches of one step.  u's transforms serve both the tangent and the
+  // first RK3 stage; a step after the first of a call finds them made by the
+  // second tangent evaluation of the step before (held), at the same u.
+  auto one = [&](bool held) -> ns3d_status {
+    NS3D_TRY(conv_front(h, uc, vc, held));
     NS3D_TRY(finish(h, ns3d::kExplicit, false, vc, h->v1, nullptr, 0.0, 1.0, dt, Re));
-    NS3D_TRY(rk3_launches(h, u, dt, Re));
+    NS3D_TRY(rk3_launches(h, u, dt, Re, true));
     NS3D_TRY(conv_front(h, uc, v1c));
     return finish(h, ns3d::kExplicit, false, v1c, v, vc, 0.5, 0.5, dt, Re);
   };
   if (nsteps == 0) return NS3D_OK;
+  bool apart = true;  // v's update leaves u as the second evaluation transformed it
+  for (int i = 0; i < 9; ++i) apart = apart && u[i / 3] != v[i % 3];
   // As for the RK3 steps: replay a captured step where the stream allows it
   // (the legacy default stream cannot be captured).
   if (h->stream != nullptr && !h->graphs_off) {
     const void* key[6] = {ux, uy, uz, vx, vy, vz};
-    bool hit = h->jvp_exec && h->jvp_dt == dt && h->jvp_Re == Re &&
+    bool hit = h->jvp_exec[0] && h->jvp_dt == dt && h->jvp_Re == Re &&
                h->jvp_stream == h->stream && h->jvp_fversion == h->f_version;
     for (int i = 0; i < 6 && hit; ++i) hit = h->jvp_key[i] == key[i];
     if (!hit) {
-      if (h->jvp_exec) cudaGraphExecDestroy(h->jvp_exec);
-      h->jvp_exec = nullptr;
+      for (auto& e : h->jvp_exec) {
+        if (e) cudaGraphExecDestroy(e);
+        e = nullptr;
+      }
+    }
+    // [0] the first step of a call, [1] the later ones
+    for (int k = 0; k < (nsteps > 1 && apart ? 2 : 1) && !h->graphs_off; ++k) {
+      if (h->jvp_exec[k]) continue;
       cudaGraph_t graph = nullptr;
       cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
-        ns3d_status s = one();
+        ns3d_status s = one(k == 1);
         e = cudaStreamEndCapture(h->stream, &graph);
         if (s != NS3D_OK) {
           if (graph) cudaGraphDestroy(graph);
           return s;
         }
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&h->jvp_exec, graph, 0);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&h->jvp_exec[k], graph, 0);
         if (graph) cudaGraphDestroy(graph);
       }
       if (e != cudaSuccess) {
         cudaGetLastError();
-        h->jvp_exec = nullptr;
+        drop_graph(h);
         h->graphs_off = true;
-      } else {
-        for (int i = 0; i < 6; ++i) h->jvp_key[i] = key[i];
-        h->jvp_dt = dt; h->jvp_Re = Re; h->jvp_stream = h->stream;
-        h->jvp_fversion = h->f_version;
       }
     }
     if (!h->graphs_off) {
+      for (int i = 0; i < 6; ++i) h->jvp_key[i] = key[i];
+      h->jvp_dt = dt; h->jvp_Re = Re; h->jvp_stream = h->stream;
+      h->jvp_fversion = h->f_version;
       for (int s = 0; s < nsteps; ++s)
-        NS3D_CHECK(h, cudaGraphLaunch(h->jvp_exec, h->stream), "graph launch");
+        NS3D_CHECK(h, cudaGraphLaunch(h->jvp_exec[s > 0 && apart], h->stream), "graph launch");
       return NS3D_OK;
     }
   }
-  for (int s = 0; s < nsteps; ++s) NS3D_TRY(one());
+  for (int s = 0; s < nsteps; ++s) NS3D_TRY(one(s > 0 && apart));
   return NS3D_OK;
 }
 

@@ -66,7 +66,7 @@ struct ns3d_solver {
   int f_version = 0, rk3_fversion = -1;
   bool graphs_off = false;
   // the captured tangent step (RK3_SSP_UV) of ns3d_jvp_steps and its key
-  cudaGraphExec_t jvp_exec = nullptr;
+  cudaGraphExec_t jvp_exec[2] = {};  // the first step of a call, the later ones
   const void* jvp_key[6] = {};
   double jvp_dt = 0.0, jvp_Re = 0.0;
   cudaStream_t jvp_stream = nullptr;
@@ -100,14 +100,19 @@ ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double L
                           ns3d_solver** out);
 // the tangent scratch (B(u,v) fields and v1), for the whole batch
 ns3d_status ensure_uv_pool(ns3d_solver* h);
-// inv_x -> inv_y -> z -> fwd_y (v null: the nonlinear term; else B(u, v))
-ns3d_status conv_front(ns3d_solver* h, const double2* const u[3], const double2* const v[3]);
+// inv_x -> inv_y -> z -> fwd_y (v null: the nonlinear term; else B(u, v)).
+// held: u's transforms are in the scratch already, from the latest evaluation
+// that made them, at this same u
+ns3d_status conv_front(ns3d_solver* h, const double2* const u[3], const double2* const v[3],
+                       bool held = false);
 // fwd_x with the pointwise update of `mode` (ns3d::UpdateMode)
 ns3d_status finish(ns3d_solver* h, int mode, bool forcing, const double2* const us[3],
                    double2* const out[3], const double2* const un[3], double ca, double cb,
                    double dt, double Re);
-// one RK3_SSP step of the state u (all instances of a batch)
-ns3d_status rk3_launches(ns3d_solver* h, double2* const u[3], double dt, double Re);
+// one RK3_SSP step of the state u (all instances of a batch); held: as for
+// conv_front, of the first stage
+ns3d_status rk3_launches(ns3d_solver* h, double2* const u[3], double dt, double Re,
+                         bool held = false);
 
 }  // namespace ns3d_detail
 
