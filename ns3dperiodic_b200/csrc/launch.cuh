@@ -130,6 +130,18 @@ inline unsigned blocks_for(long long lines, int lpc) { return (unsigned)((lines 
 template <int KIND, int N, int P, int X>
 struct KTag {};
 
+// Passes that run resident CTAs, the groups of lines dealt round robin, so that
+// a CTA reads its twiddles once and its copy pipeline runs on from group to
+// group: the FP32 lines and the plain transforms' passes, whose groups are
+// short (FP32) or a single unit (plain).  FP64 lines keep one CTA per group:
+// their neighbouring groups then run side by side.  Per launch on a B200 at
+// 256^3, one CTA per group / resident CTAs: FP32 inv_x 134 / 125 us, inv_y 149 /
+// 141, fwd_y 102 / 95, fwd_x 278 / 260; FP64 170 / 175, 265 / 268, 150 / 165,
+// 248 / 249; a plain R2C and C2R 359 / 297 us.  FP32 lines of 512 points, four
+// to a CTA, lose: inv_x 1.39 / 1.52 ms, fwd_x 2.76 / 3.16.
+template <typename C, int N>
+constexpr bool cap_grid() { return NS3D_SCHED != 0 || (sizeof(C) == 8 && N < 512); }
+
 // The caches are atomics: host threads that launch on the same device may
 // race to fill them, and each writes the same values.
 // kCap: cap the grid at the resident CTAs whatever NS3D_SCHED says (kernels
@@ -173,9 +185,9 @@ cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStre
   const long long lines = 8LL * g.nlive * nbatch(g);
   using S = PassSmem<N, P, C, double2, V>;
   const long long groups = (lines + S::LPC - 1) / S::LPC;
-  const unsigned grid = persistent_grid<KTag<0, N, P, NF + prec_tag<C>() + 1000 * V>>(
+  const unsigned grid = persistent_grid<KTag<0, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_x_kernel<N, P, NF, C, V>, S::BYTES, groups);
-  const unsigned grid1 = persistent_grid<KTag<60, N, P, NF + prec_tag<C>() + 1000 * V>>(
+  const unsigned grid1 = persistent_grid<KTag<60, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_x_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
   if (prepare_only) return cudaGetLastError();
   if (one_field_per_cta(groups))
@@ -275,9 +287,9 @@ cudaError_t launch_inv_y_p(const InvYArgs<NF, C>& a, const PassGeom& g, cudaStre
   const long long lines = (long long)g.Nx * g.Zp;
   using S = PassSmem<N, P, C, C, V>;
   const long long groups = (lines + S::LPC - 1) / S::LPC;
-  const unsigned grid = persistent_grid<KTag<1, N, P, NF + prec_tag<C>() + 1000 * V>>(
+  const unsigned grid = persistent_grid<KTag<1, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_y_kernel<N, P, NF, C, V>, S::BYTES, groups);
-  const unsigned grid1 = persistent_grid<KTag<61, N, P, NF + prec_tag<C>() + 1000 * V>>(
+  const unsigned grid1 = persistent_grid<KTag<61, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_y_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
   if (prepare_only) return cudaGetLastError();
   if (one_field_per_cta(groups))
@@ -357,7 +369,7 @@ cudaError_t launch_fwd_x_p(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t
   const long long lines = (long long)g.Ny * g.Mz * nbatch(g);
   using S = PassSmem<N, P, C, C>;
   const unsigned grid =
-      persistent_grid<KTag<2 + 2 * MODE + (COMBINE ? 1 : 0), N, P, prec_tag<C>()>>(
+      persistent_grid<KTag<2 + 2 * MODE + (COMBINE ? 1 : 0), N, P, prec_tag<C>()>, cap_grid<C, N>()>(
           fwd_x_kernel<N, P, MODE, COMBINE, C>, S::BYTES, (lines + S::LPC - 1) / S::LPC);
   if (prepare_only) return cudaGetLastError();
   fwd_x_kernel<N, P, MODE, COMBINE, C><<<grid, kThreads, S::BYTES, st>>>(a, g);
@@ -387,7 +399,7 @@ cudaError_t launch_fwd_x_ring(const FwdXArgs<C>& a, const PassGeom& g, cudaStrea
   const long long lines = (long long)g.Ny * g.Mz * nbatch(g);
   using S = FxRingSmem<N, P, NSLOT, C>;
   const unsigned grid =
-      persistent_grid<KTag<50 + 2 * MODE + (COMBINE ? 1 : 0), N, P, prec_tag<C>()>>(
+      persistent_grid<KTag<50 + 2 * MODE + (COMBINE ? 1 : 0), N, P, prec_tag<C>()>, cap_grid<C, N>()>(
           fwd_x_ring_kernel<N, P, MODE, COMBINE, NSLOT, C>, S::BYTES,
           (lines + S::LPC - 1) / S::LPC);
   if (prepare_only) return cudaGetLastError();
@@ -421,9 +433,9 @@ cudaError_t launch_fwd_y_p(const FwdYArgs<C>& a, const PassGeom& g, cudaStream_t
   const long long lines = (long long)g.Nx * g.Mz;
   using S = PassSmem<N, P, C, C, V>;
   const long long groups = (lines + S::LPC - 1) / S::LPC;
-  const unsigned grid = persistent_grid<KTag<20, N, P, prec_tag<C>() + 1000 * V>>(
+  const unsigned grid = persistent_grid<KTag<20, N, P, prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       fwd_y_kernel<N, P, C, V>, S::BYTES, groups);
-  const unsigned grid1 = persistent_grid<KTag<62, N, P, prec_tag<C>() + 1000 * V>>(
+  const unsigned grid1 = persistent_grid<KTag<62, N, P, prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       fwd_y_kernel<N, P, C, V, 1>, S::BYTES, groups);
   if (prepare_only) return cudaGetLastError();
   if (one_field_per_cta(groups))
@@ -471,7 +483,7 @@ cudaError_t launch_line(const LineArgs& a, const PassGeom& g, cudaStream_t st,
   case N: {                                                                             \
     constexpr int P = p_line(N);                                                           \
     using S = PassSmem<N, P>;                                                           \
-    const unsigned grid = persistent_grid<KTag<30 + 2 * AXIS + (DIR > 0 ? 1 : 0), N, P, 0>>( \
+    const unsigned grid = persistent_grid<KTag<30 + 2 * AXIS + (DIR > 0 ? 1 : 0), N, P, 0>, true>( \
         line_kernel<N, P, AXIS, DIR>, S::BYTES, (lines + S::LPC - 1) / S::LPC);         \
     if (prepare_only) return cudaGetLastError();                                        \
     line_kernel<N, P, AXIS, DIR><<<grid, kThreads, S::BYTES, st>>>(a, g);                \
