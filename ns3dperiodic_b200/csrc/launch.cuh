@@ -174,6 +174,16 @@ inline unsigned persistent_grid(Kern kern, size_t smem, long long groups) {
 // 32^3 (16 to 18 groups) 144 / 109 us, 64^3 (48 to 66) 149 / 116; 96^3 (192 to
 // 294) 350 / 372.
 inline bool one_field_per_cta(long long groups) { return groups < 148; }
+// Whether larger grids too run one field per CTA, with one prefetch buffer and
+// three CTAs per SM instead of two: then 12 warps per SM hide what 8 with a
+// deeper pipeline cannot.  FP64 lines of 12 and 16 points only (the others have
+// three CTAs already, or live on L1); lines of 32 threads, four to a CTA, and
+// inv_x's plain form from 16 threads a line keep two.  Per launch on a B200, two /
+// three CTAs: inv_y 96^3 26.6 / 23.3 us, 128^3 44 / 37, 256^3 265 / 218, 512^3
+// 2274 / 2454; inv_x 96^3 22.8 / 22.4, 128^3 36 / 31, 256^3 170 / 178; the tangent
+// step (six fields) at 128^3 1205 / 1074.
+template <int P, typename C>
+constexpr bool dense_ctas(bool wide) { return sizeof(C) == 16 && P > 8 && !wide; }
 
 // KTag's last argument separates the FP64 and FP32 instantiations.
 template <typename C>
@@ -189,6 +199,17 @@ cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStre
       inv_x_kernel<N, P, NF, C, V>, S::BYTES, groups);
   const unsigned grid1 = persistent_grid<KTag<60, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_x_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
+  constexpr bool DENSE = dense_ctas<P, C>(NF == 3 && N / P >= 16);
+  if constexpr (DENSE) {
+    using S1 = PassSmem<N, P, C, double2, V, 1>;
+    const unsigned gridd = persistent_grid<KTag<70, N, P, NF + prec_tag<C>() + 1000 * V>>(
+        inv_x_kernel<N, P, NF, C, V, 1, 1>, S1::BYTES, groups);
+    if (prepare_only) return cudaGetLastError();
+    if (!one_field_per_cta(groups)) {
+      inv_x_kernel<N, P, NF, C, V, 1, 1><<<dim3(gridd, NF), kThreads, S1::BYTES, st>>>(a, g);
+      return cudaGetLastError();
+    }
+  }
   if (prepare_only) return cudaGetLastError();
   if (one_field_per_cta(groups))
     inv_x_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);
@@ -291,6 +312,17 @@ cudaError_t launch_inv_y_p(const InvYArgs<NF, C>& a, const PassGeom& g, cudaStre
       inv_y_kernel<N, P, NF, C, V>, S::BYTES, groups);
   const unsigned grid1 = persistent_grid<KTag<61, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_y_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
+  constexpr bool DENSE = dense_ctas<P, C>(N / P >= 32);
+  if constexpr (DENSE) {
+    using S1 = PassSmem<N, P, C, C, V, 1>;
+    const unsigned gridd = persistent_grid<KTag<71, N, P, NF + prec_tag<C>() + 1000 * V>>(
+        inv_y_kernel<N, P, NF, C, V, 1, 1>, S1::BYTES, groups);
+    if (prepare_only) return cudaGetLastError();
+    if (!one_field_per_cta(groups)) {
+      inv_y_kernel<N, P, NF, C, V, 1, 1><<<dim3(gridd, NF), kThreads, S1::BYTES, st>>>(a, g);
+      return cudaGetLastError();
+    }
+  }
   if (prepare_only) return cudaGetLastError();
   if (one_field_per_cta(groups))
     inv_y_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);

@@ -232,7 +232,14 @@ constexpr size_t align16(size_t b) { return (b + 15) / 16 * 16; }
 // buffers in the line precision C, then each thread's double buffer of
 // prefetched elements of type E (the pass's input, FP64 state or scratch).
 // V: the radix schedule (PlanV).
-template <int N, int P, typename C = double2, typename E = C, int V = 0>
+// CTAs per SM asked of ptxas by a form of the x / y passes with NB prefetch
+// buffers: the one-buffer form's shared memory leaves room for three
+// (168 registers).
+__host__ __device__ constexpr int xy_ctas(int p, int nb) { return nb == 1 ? 3 : min_ctas_xy(p); }
+
+// NB: prefetch buffers (2: the next unit's copies run under this unit; 1: the
+// buffer is refilled once its samples are in registers).
+template <int N, int P, typename C = double2, typename E = C, int V = 0, int NB = 2>
 struct PassSmem {
   using F = LineFFT<N, P, V>;
   using LM = LaneMap<F::T>;
@@ -240,7 +247,7 @@ struct PassSmem {
   static constexpr int STRIDE = line_stride(F::BUF, xy_stride_target<F::T>());
   static constexpr size_t SBUF_OFF = align16((size_t)F::TWLEN * sizeof(C));
   static constexpr size_t PF_OFF = align16(SBUF_OFF + (size_t)LPC * STRIDE * sizeof(C));
-  static constexpr size_t BYTES = PF_OFF + (size_t)2 * P * kThreads * sizeof(E);
+  static constexpr size_t BYTES = PF_OFF + (size_t)NB * P * kThreads * sizeof(E);
   static_assert(BYTES <= 227 * 1024, "shared memory per CTA");
   __device__ __forceinline__ static C* tw(unsigned char* base) { return (C*)base; }
   __device__ __forceinline__ static C* sbuf(unsigned char* base, int li) {
@@ -276,12 +283,12 @@ struct InvXArgs {
   const double2* tw;
 };
 
-// FPC: fields of a CTA (NF, or 1 with blockIdx.y the field; fields_per_cta)
-template <int NX, int P, int NF, typename C, int V = 0, int FPC = NF>
-__global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
+// FPC: fields of a CTA (NF, or 1 with blockIdx.y the field)
+template <int NX, int P, int NF, typename C, int V = 0, int FPC = NF, int NB = 2>
+__global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
     inv_x_kernel(const __grid_constant__ InvXArgs<NF, C> a, PassGeom g) {
   const int f0 = FPC == NF ? 0 : blockIdx.y * FPC;
-  using S = PassSmem<NX, P, C, double2, V>;
+  using S = PassSmem<NX, P, C, double2, V, NB>;
   using F = typename S::F;
   using LM = typename S::LM;
   using Rt = RealOf<C>;
@@ -331,18 +338,24 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
     size_t off_next = 0, out_next = 0;
     bool valid_next = false;
     if (gn < g_end) valid_next = line(gn * LM::LPC + li, off_next, out_next, keep_next);
+    auto issue_next = [&](int i, double2* dst) {  // the unit after field f0 + i
+      if (i + 1 < FPC) {
+        issue_line<P, T>(dst, a.in[f0 + i + 1], off, (size_t)nlines, t, keep);
+      } else if (gn < g_end) {
+        issue_line<P, T>(dst, a.in[f0], off_next, (size_t)nlines, t, keep_next);
+      }
+      cp_async_commit();
+    };
 #pragma unroll
     for (int i = 0; i < FPC; ++i) {
       const int f = f0 + i;
       const double2* cur = pf + ub * (P * kThreads);
-      double2* nxt = pf + (ub ^ 1) * (P * kThreads);
-      if (i + 1 < FPC) {
-        issue_line<P, T>(nxt, a.in[f + 1], off, (size_t)nlines, t, keep);
-      } else if (gn < g_end) {
-        issue_line<P, T>(nxt, a.in[f0], off_next, (size_t)nlines, t, keep_next);
+      if constexpr (NB == 2) {
+        issue_next(i, pf + (ub ^ 1) * (P * kThreads));
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
       }
-      cp_async_commit();
-      cp_async_wait<1>();
       // X (masked) then i kx X, both from the prefetched samples
       C v[P];
 #pragma unroll
@@ -358,12 +371,13 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
         const Rt kx = (Rt)(g.kfx * (double)signed_idx(t + T * s, NX));
         v[s] = mkc<C>(-u.y * kx, u.x * kx);  // i kx u (build_ders_device)
       }
+      if constexpr (NB == 1) issue_next(i, pf);
       F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
       if (valid) {
 #pragma unroll
         for (int s = 0; s < P; ++s) a.B[f][out + (size_t)(t + T * s) * olines] = v[s];
       }
-      ub ^= 1;
+      if constexpr (NB == 2) ub ^= 1;
     }
     keep = keep_next;
     off = off_next;
@@ -401,11 +415,11 @@ struct InvYArgs {
   int* err = nullptr;  // error flag of the bulk-copy form's bounded waits
 };
 
-template <int NY, int P, int NF, typename C, int V = 0, int FPC = NF>
-__global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
+template <int NY, int P, int NF, typename C, int V = 0, int FPC = NF, int NB = 2>
+__global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
     inv_y_kernel(const __grid_constant__ InvYArgs<NF, C> a, PassGeom g) {
   const int f0 = FPC == NF ? 0 : blockIdx.y * FPC;
-  using S = PassSmem<NY, P, C, C, V>;
+  using S = PassSmem<NY, P, C, C, V, NB>;
   using F = typename S::F;
   using LM = typename S::LM;
   using Rt = RealOf<C>;
@@ -441,16 +455,30 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
     const bool valid = grp * LM::LPC + li < nb;
     const int gn = grp + gr.step;
     if (gn < g_end) basen = line_base(gn, keep_next);
+    auto issue_b = [&](int f, C* dst) {
+      issue_line<P, T>(dst, a.B[f], base, stride, t, keep);
+      cp_async_commit();
+    };
+    auto issue_a = [&](int i, C* dst) {  // the unit after B of field f0 + i
+      if (i + 1 < FPC) {
+        issue_line<P, T>(dst, a.A[f0 + i + 1], base, stride, t, keep);
+      } else if (gn < g_end) {
+        issue_line<P, T>(dst, a.A[f0], basen, stride, t, keep_next);
+      }
+      cp_async_commit();
+    };
 #pragma unroll 1  // one copy of the three transforms: nine (18) outgrow the instruction cache
     for (int i = 0; i < FPC; ++i) {
       const int f = f0 + i;
       // unit A[f] -> C[f] = IFFT_y A, D[f] = IFFT_y(i ky A)
       {
         const C* cur = pf + ub * (P * kThreads);
-        C* nxt = pf + (ub ^ 1) * (P * kThreads);
-        issue_line<P, T>(nxt, a.B[f], base, stride, t, keep);
-        cp_async_commit();
-        cp_async_wait<1>();
+        if constexpr (NB == 2) {
+          issue_b(f, pf + (ub ^ 1) * (P * kThreads));
+          cp_async_wait<1>();
+        } else {
+          cp_async_wait<0>();
+        }
         C v[P];
 #pragma unroll
         for (int s = 0; s < P; ++s) v[s] = cur[s * kThreads];
@@ -465,33 +493,33 @@ __global__ void __launch_bounds__(kThreads, min_ctas_xy(P))
           const Rt ky = (Rt)(g.kfy * (double)signed_idx(t + T * s, NY));
           v[s] = mkc<C>(-u.y * ky, u.x * ky);
         }
+        if constexpr (NB == 1) issue_b(f, pf);
         F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
         if (valid) {
 #pragma unroll
           for (int s = 0; s < P; ++s) a.D[f][base + (size_t)(t + T * s) * stride] = v[s];
         }
-        ub ^= 1;
+        if constexpr (NB == 2) ub ^= 1;
       }
       // unit B[f] -> E[f] = IFFT_y B
       {
         const C* cur = pf + ub * (P * kThreads);
-        C* nxt = pf + (ub ^ 1) * (P * kThreads);
-        if (i + 1 < FPC) {
-          issue_line<P, T>(nxt, a.A[f + 1], base, stride, t, keep);
-        } else if (gn < g_end) {
-          issue_line<P, T>(nxt, a.A[f0], basen, stride, t, keep_next);
+        if constexpr (NB == 2) {
+          issue_a(i, pf + (ub ^ 1) * (P * kThreads));
+          cp_async_wait<1>();
+        } else {
+          cp_async_wait<0>();
         }
-        cp_async_commit();
-        cp_async_wait<1>();
         C v[P];
 #pragma unroll
         for (int s = 0; s < P; ++s) v[s] = cur[s * kThreads];
+        if constexpr (NB == 1) issue_a(i, pf);
         F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
         if (valid) {
 #pragma unroll
           for (int s = 0; s < P; ++s) a.E[f][base + (size_t)(t + T * s) * stride] = v[s];
         }
-        ub ^= 1;
+        if constexpr (NB == 2) ub ^= 1;
       }
     }
     base = basen;
