@@ -181,7 +181,8 @@ inline bool one_field_per_cta(long long groups) { return groups < 148; }
 // inv_x's plain form from 16 threads a line keep two.  Per launch on a B200, two /
 // three CTAs: inv_y 96^3 26.6 / 23.3 us, 128^3 44 / 37, 256^3 265 / 218, 512^3
 // 2274 / 2454; inv_x 96^3 22.8 / 22.4, 128^3 36 / 31, 256^3 170 / 178; the tangent
-// step (six fields) at 128^3 1205 / 1074.
+// step (six fields) at 128^3 1205 / 1074.  FP32 lines: inv_x so at four CTAs,
+// 128^3 28.7 / 25.1 us, 256^3 127 / 120; their inv_y does not (142 / 155-167).
 template <int P, typename C>
 constexpr bool dense_ctas(bool wide) { return sizeof(C) == 16 && P > 8 && !wide; }
 
@@ -199,10 +200,11 @@ cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStre
       inv_x_kernel<N, P, NF, C, V>, S::BYTES, groups);
   const unsigned grid1 = persistent_grid<KTag<60, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_x_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
-  constexpr bool DENSE = dense_ctas<P, C>(NF == 3 && N / P >= 16);
+  constexpr bool DENSE = sizeof(C) == 8 ? P > 8 && N / P < 32
+                                        : dense_ctas<P, C>(NF == 3 && N / P >= 16);
   if constexpr (DENSE) {
     using S1 = PassSmem<N, P, C, double2, V, 1>;
-    const unsigned gridd = persistent_grid<KTag<70, N, P, NF + prec_tag<C>() + 1000 * V>>(
+    const unsigned gridd = persistent_grid<KTag<70, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
         inv_x_kernel<N, P, NF, C, V, 1, 1>, S1::BYTES, groups);
     if (prepare_only) return cudaGetLastError();
     if (!one_field_per_cta(groups)) {

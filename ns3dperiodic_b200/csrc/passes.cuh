@@ -192,6 +192,34 @@ __device__ __forceinline__ void issue_line(E* slot, const E* __restrict__ src,
                   (keep >> s) & 1u);
 }
 
+// The same for FP32 lines, whose samples are 8 bytes: two neighbouring lines
+// (2k, 2k + 1 of the CTA, threads of one warp, adjacent in memory from a 16-byte
+// boundary) share 16-byte copies, the even line's thread making those of the
+// even samples and the odd line's those of the odd ones.  Half as many copies,
+// and they bypass L1 (an 8-byte copy goes through it, and the lines it
+// allocates in flight bound the pass, most where another stream's kernels, with
+// a larger shared-memory carve-out, run beside it: three 256^3 FP32 solvers in
+// turn 3.10 -> 2.83 ms a step, one alone 2.66 -> 2.62).  A thread reads cells its partner
+// copied: __syncwarp after the wait.  two: samples both lines keep, one: those
+// the even line alone keeps (the odd line's cell is zero-filled).  `slot` is
+// the buffer without the thread's offset, base2 the even line's base.
+template <int P, int T>
+__device__ __forceinline__ void issue_line_pair(float2* slot, const float2* __restrict__ src,
+                                                size_t base2, size_t stride, int t, uint32_t two,
+                                                uint32_t one) {
+  const int par = threadIdx.x & 1;
+  float2* dst = slot + (threadIdx.x & ~1u);
+#pragma unroll
+  for (int s2 = 0; s2 < P; s2 += 2) {
+    const int s = s2 + par;
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst + s * kThreads);
+    const int n = (two >> s) & 1u ? 16 : ((one >> s) & 1u ? 8 : 0);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d),
+                 "l"(src + base2 + (size_t)(t + T * s) * stride), "r"(n)
+                 : "memory");
+  }
+}
+
 // Smallest line-buffer stride >= len whose residue mod 8 (16-byte slots; one
 // shared-memory wavefront is 8 slots) is `target`, 0 meaning any.
 constexpr int line_stride(int len, int target) {
@@ -234,8 +262,11 @@ constexpr size_t align16(size_t b) { return (b + 15) / 16 * 16; }
 // V: the radix schedule (PlanV).
 // CTAs per SM asked of ptxas by a form of the x / y passes with NB prefetch
 // buffers: the one-buffer form's shared memory leaves room for three
-// (168 registers).
-__host__ __device__ constexpr int xy_ctas(int p, int nb) { return nb == 1 ? 3 : min_ctas_xy(p); }
+// (168 registers), four for FP32 lines (128 registers).
+template <typename C>
+__host__ __device__ constexpr int xy_ctas(int p, int nb) {
+  return nb == 1 ? (sizeof(C) == 8 ? 4 : 3) : min_ctas_xy(p);
+}
 
 // NB: prefetch buffers (2: the next unit's copies run under this unit; 1: the
 // buffer is refilled once its samples are in registers).
@@ -285,7 +316,7 @@ struct InvXArgs {
 
 // FPC: fields of a CTA (NF, or 1 with blockIdx.y the field)
 template <int NX, int P, int NF, typename C, int V = 0, int FPC = NF, int NB = 2>
-__global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
+__global__ void __launch_bounds__(kThreads, xy_ctas<C>(P, NB))
     inv_x_kernel(const __grid_constant__ InvXArgs<NF, C> a, PassGeom g) {
   const int f0 = FPC == NF ? 0 : blockIdx.y * FPC;
   using S = PassSmem<NX, P, C, double2, V, NB>;
@@ -416,7 +447,7 @@ struct InvYArgs {
 };
 
 template <int NY, int P, int NF, typename C, int V = 0, int FPC = NF, int NB = 2>
-__global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
+__global__ void __launch_bounds__(kThreads, xy_ctas<C>(P, NB))
     inv_y_kernel(const __grid_constant__ InvYArgs<NF, C> a, PassGeom g) {
   const int f0 = FPC == NF ? 0 : blockIdx.y * FPC;
   using S = PassSmem<NY, P, C, C, V, NB>;
@@ -424,6 +455,8 @@ __global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
   using LM = typename S::LM;
   using Rt = RealOf<C>;
   constexpr int T = F::T;
+  constexpr bool PAIRS = sizeof(C) == 8;
+  static_assert(!PAIRS || (NB == 2 && P % 2 == 0 && LM::LPC % 2 == 0), "pairs of lines");
   extern __shared__ __align__(16) unsigned char dsm[];
   F::load_tw(S::tw(dsm), a.tw);
   const C* tw_s = S::tw(dsm);
@@ -438,32 +471,48 @@ __global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
   const int g_end = gr.end;
   int grp = gr.grp;
   if (grp >= g_end) return;
-  auto line_base = [&](int gidx, uint32_t& keep) -> size_t {
+  auto line_base = [&](int gidx, auto& keep) -> size_t {
     const int b = gidx * LM::LPC + li;
     const bool valid = b < nb;
     const int bc = valid ? b : 0;
     const int x = bc / g.Zp, z = bc - x * g.Zp;
-    keep = row_bits(g.ycut, z, valid, t, T, P);
-    return (size_t)x * g.Ny * g.Zp + z;
+    if constexpr (PAIRS) {  // rows the pair's lines keep (z even: the first one's)
+      keep.two = row_bits(g.ycut, z | 1, valid, t, T, P);
+      keep.one = row_bits(g.ycut, z & ~1, valid, t, T, P);
+      return (size_t)x * g.Ny * g.Zp + (z & ~1);
+    } else {
+      keep.two = row_bits(g.ycut, z, valid, t, T, P);
+      return (size_t)x * g.Ny * g.Zp + z;
+    }
   };
-  uint32_t keep, keep_next = 0;  // rows inside the mask
+  struct Keep {
+    uint32_t two = 0, one = 0;
+  };
+  Keep keep, keep_next;  // rows inside the mask
   size_t base = line_base(grp, keep), basen = 0;
-  issue_line<P, T>(pf, a.A[f0], base, stride, t, keep);
+  auto issue = [&](int buf, const C* src, size_t at, const Keep& k) {
+    if constexpr (PAIRS)
+      issue_line_pair<P, T>(pf - threadIdx.x + buf * (P * kThreads), src, at, stride, t, k.two, k.one);
+    else
+      issue_line<P, T>(pf + buf * (P * kThreads), src, at, stride, t, k.two);
+  };
+  const size_t own = PAIRS ? (size_t)(threadIdx.x & 1) : 0;  // this line past its pair's base
+  issue(0, a.A[f0], base, keep);
   cp_async_commit();
   int ub = 0;
   for (; grp < g_end; grp += gr.step) {
     const bool valid = grp * LM::LPC + li < nb;
     const int gn = grp + gr.step;
     if (gn < g_end) basen = line_base(gn, keep_next);
-    auto issue_b = [&](int f, C* dst) {
-      issue_line<P, T>(dst, a.B[f], base, stride, t, keep);
+    auto issue_b = [&](int f, int buf) {
+      issue(buf, a.B[f], base, keep);
       cp_async_commit();
     };
-    auto issue_a = [&](int i, C* dst) {  // the unit after B of field f0 + i
+    auto issue_a = [&](int i, int buf) {  // the unit after B of field f0 + i
       if (i + 1 < FPC) {
-        issue_line<P, T>(dst, a.A[f0 + i + 1], base, stride, t, keep);
+        issue(buf, a.A[f0 + i + 1], base, keep);
       } else if (gn < g_end) {
-        issue_line<P, T>(dst, a.A[f0], basen, stride, t, keep_next);
+        issue(buf, a.A[f0], basen, keep_next);
       }
       cp_async_commit();
     };
@@ -474,18 +523,19 @@ __global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
       {
         const C* cur = pf + ub * (P * kThreads);
         if constexpr (NB == 2) {
-          issue_b(f, pf + (ub ^ 1) * (P * kThreads));
+          issue_b(f, ub ^ 1);
           cp_async_wait<1>();
         } else {
           cp_async_wait<0>();
         }
+        if constexpr (PAIRS) __syncwarp();  // the partner's copies
         C v[P];
 #pragma unroll
         for (int s = 0; s < P; ++s) v[s] = cur[s * kThreads];
         F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
         if (valid) {
 #pragma unroll
-          for (int s = 0; s < P; ++s) a.C[f][base + (size_t)(t + T * s) * stride] = v[s];
+          for (int s = 0; s < P; ++s) a.C[f][base + own + (size_t)(t + T * s) * stride] = v[s];
         }
 #pragma unroll
         for (int s = 0; s < P; ++s) {
@@ -493,11 +543,11 @@ __global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
           const Rt ky = (Rt)(g.kfy * (double)signed_idx(t + T * s, NY));
           v[s] = mkc<C>(-u.y * ky, u.x * ky);
         }
-        if constexpr (NB == 1) issue_b(f, pf);
+        if constexpr (NB == 1) issue_b(f, 0);
         F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
         if (valid) {
 #pragma unroll
-          for (int s = 0; s < P; ++s) a.D[f][base + (size_t)(t + T * s) * stride] = v[s];
+          for (int s = 0; s < P; ++s) a.D[f][base + own + (size_t)(t + T * s) * stride] = v[s];
         }
         if constexpr (NB == 2) ub ^= 1;
       }
@@ -505,23 +555,25 @@ __global__ void __launch_bounds__(kThreads, xy_ctas(P, NB))
       {
         const C* cur = pf + ub * (P * kThreads);
         if constexpr (NB == 2) {
-          issue_a(i, pf + (ub ^ 1) * (P * kThreads));
+          issue_a(i, ub ^ 1);
           cp_async_wait<1>();
         } else {
           cp_async_wait<0>();
         }
+        if constexpr (PAIRS) __syncwarp();  // the partner's copies
         C v[P];
 #pragma unroll
         for (int s = 0; s < P; ++s) v[s] = cur[s * kThreads];
-        if constexpr (NB == 1) issue_a(i, pf);
+        if constexpr (NB == 1) issue_a(i, 0);
         F::template run<+1, F::PADW, LM::SW>(v, t, sbuf, tw_s);
         if (valid) {
 #pragma unroll
-          for (int s = 0; s < P; ++s) a.E[f][base + (size_t)(t + T * s) * stride] = v[s];
+          for (int s = 0; s < P; ++s) a.E[f][base + own + (size_t)(t + T * s) * stride] = v[s];
         }
         if constexpr (NB == 2) ub ^= 1;
       }
     }
+    if constexpr (PAIRS && T == 1) __syncwarp();  // (a one-thread line has no barrier of its own)
     base = basen;
     keep = keep_next;
   }
