@@ -140,8 +140,8 @@ struct LaneMap {
 
 // ---------------------------------------------------------------------------
 // Software-pipelined x / y passes.  A CTA handles groups of LPC lines (one
-// group per CTA by default, see NS3D_SCHED); every thread owns a private
-// double buffer in shared memory and, while the current line of field f is
+// group per CTA by default, see NS3D_SCHED); every thread owns one or two
+// private buffers in shared memory and, while the current line of field f is
 // transformed, prefetches with cp.async the P samples it will need for the
 // next unit (the next field of the same lines, or the first field of the
 // next group).
@@ -257,7 +257,7 @@ __device__ __forceinline__ GroupRange group_range(int groups) {
 constexpr size_t align16(size_t b) { return (b + 15) / 16 * 16; }
 
 // Dynamic shared memory of a pipelined pass: the stage twiddles and the line
-// buffers in the line precision C, then each thread's double buffer of
+// buffers in the line precision C, then each thread's NB buffers of
 // prefetched elements of type E (the pass's input, FP64 state or scratch).
 // V: the radix schedule (PlanV).
 // CTAs per SM asked of ptxas by a form of the x / y passes with NB prefetch
@@ -491,6 +491,9 @@ __global__ void __launch_bounds__(kThreads, xy_ctas<C>(P, NB))
   Keep keep, keep_next;  // rows inside the mask
   size_t base = line_base(grp, keep), basen = 0;
   auto issue = [&](int buf, const C* src, size_t at, const Keep& k) {
+    // the partner has read the buffer: longer lines passed a barrier of their
+    // transform since, a one-thread line has none
+    if constexpr (PAIRS && T == 1) __syncwarp();
     if constexpr (PAIRS)
       issue_line_pair<P, T>(pf - threadIdx.x + buf * (P * kThreads), src, at, stride, t, k.two, k.one);
     else
@@ -573,7 +576,6 @@ __global__ void __launch_bounds__(kThreads, xy_ctas<C>(P, NB))
         if constexpr (NB == 2) ub ^= 1;
       }
     }
-    if constexpr (PAIRS && T == 1) __syncwarp();  // (a one-thread line has no barrier of its own)
     base = basen;
     keep = keep_next;
   }
