@@ -123,6 +123,7 @@ extern "C" ns3d_status ns3d_convolution_noalloc(int Nx, int Ny, int Nz, double L
     }
     if (cap != cudaStreamCaptureStatusNone) return NS3D_ERR_BAD_ARG;
     if (ns3d_mask_cutoff(Nx, Ny, Nz, Lx, Ly, Lz, g_host_qcut) != NS3D_OK) return NS3D_ERR_BAD_ARG;
+    slot.Nx = 0;  // no grid's tables until all are uploaded
     const int ext[3] = {Nx, Ny, Nz};
     for (int d = 0; d < 3; ++d) {
       if (ns3d_twiddles(ext[d], g_host_tw[d]) != NS3D_OK) return NS3D_ERR_BAD_ARG;
