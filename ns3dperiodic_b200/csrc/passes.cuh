@@ -1535,8 +1535,13 @@ struct LineArgs {
   const double2* tw;
 };
 
+// what the plain transforms need of PassGeom
+struct PlainGeom {
+  int Nx, Ny, Mz;
+};
+
 template <int N, int P, int AXIS, int DIR>
-__global__ void __launch_bounds__(kThreads, kMinCtasXY) line_kernel(LineArgs a, PassGeom g) {
+__global__ void __launch_bounds__(kThreads, kMinCtasXY) line_kernel(LineArgs a, PlainGeom g) {
   using S = PassSmem<N, P>;
   using F = typename S::F;
   using LM = typename S::LM;
@@ -1602,7 +1607,7 @@ struct ZPlainArgs {
 // cufftExecZ2D does with the non-Hermitian planes the reference produces).
 template <int NZ, int P>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_c2r_kernel(ZPlainArgs a,
-                                                                              PassGeom g) {
+                                                                              PlainGeom g) {
   using F = LineFFT<NZ, P>;
   constexpr int T = F::T;
   using LM = ZLaneMap<T>;
@@ -1649,7 +1654,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_c2r_kernel(ZPl
 // R2C along z (unnormalised), the half spectra k = 0..Nz/2.
 template <int NZ, int P>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, kMinCtasZ) z_r2c_kernel(ZPlainArgs a,
-                                                                              PassGeom g) {
+                                                                              PlainGeom g) {
   using F = LineFFT<NZ, P>;
   constexpr int T = F::T;
   using LM = ZLaneMap<T>;
