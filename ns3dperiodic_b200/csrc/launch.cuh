@@ -30,15 +30,12 @@ constexpr int p_xy(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PXY); }
 constexpr int p_fx(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PFX); }
 // The nonlinear term's z pass: 16 points per thread for powers of two (one
 // Stockham exchange per 256-point transform instead of two), 12 for multiples
-// of 3; the tangent form, with twice the velocities parked: 8.
+// of 3; the tangent form, six velocities and three products in registers: 4 (6).
 #ifndef NS3D_PZST
 #define NS3D_PZST 16
 #endif
 constexpr int p_z(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PZST); }
-#ifndef NS3D_PZUV
-#define NS3D_PZUV 8
-#endif
-constexpr int p_zuv(int n) { return n % 3 == 0 ? 12 : p_pow2(n, NS3D_PZUV); }
+constexpr int p_zuv(int n) { return n % 3 == 0 ? 6 : 4; }
 // points per thread of the plain line passes (8 measured slower than 16 at 256^3 and 512^3)
 #ifndef NS3D_PLINE
 #define NS3D_PLINE 16
@@ -377,13 +374,12 @@ cudaError_t launch_z(const ZArgs<NF, C>& a, const PassGeom& gi, cudaStream_t st)
   case N: {                                                                           \
     constexpr bool UV = NF == 6;                                                      \
     constexpr int P = UV ? p_zuv(N) : p_z(N);                                         \
-    using S = ZSmem<N, P, UV, C>;                                                     \
-    const unsigned groups = blocks_for(lines, S::LM::LPC);                            \
     if constexpr (UV) {                                                               \
-      const unsigned grid = persistent_grid<KTag<41, N, P, prec_tag<C>()>>(           \
-          z_uv_kernel<N, P, C>, S::BYTES, groups);                                    \
-      z_uv_kernel<N, P, C><<<grid, kThreads, S::BYTES, st>>>(a, g);                   \
+      z_uv_kernel<N, P, C>                                                            \
+          <<<blocks_for(lines, lines_per_cta_z<N, P>()), kThreads, 0, st>>>(a, g);    \
     } else {                                                                          \
+      using S = ZSmem<N, P, C>;                                                       \
+      const unsigned groups = blocks_for(lines, S::LM::LPC);                          \
       const unsigned grid = persistent_grid<KTag<40, N, P, prec_tag<C>()>>(           \
           z_kernel<N, P, C>, S::BYTES, groups);                                       \
       z_kernel<N, P, C><<<grid, kThreads, S::BYTES, st>>>(a, g);                      \

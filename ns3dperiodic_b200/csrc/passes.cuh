@@ -912,11 +912,6 @@ struct ZLaneMap {  // lanes of one line are adjacent: the line is contiguous in 
 // Per launch on a B200 (plain loads behind L2 prefetches, unrolled, stash in
 // shared memory, 8 warps per SM -> this form): FP64 256^3 403 -> 379 us, 128^3
 // 62.4 -> 56.5; FP32 275 -> 229, 47.1 -> 37.9.
-//
-// The tangent form (z_uv_kernel) parks six velocities, keeps its products in
-// registers and stages its rows two transforms deep, 8 points per thread (12
-// for multiples of 3).  The linearised product, 4 (6) points and plain loads ->
-// this form: 128^3 495 -> 388 us, 96^3 251 -> 206.
 // ---------------------------------------------------------------------------
 // CTAs per SM the FP32 lines ask for (they take half the registers)
 #ifndef NS3D_MINCTA_Z32
@@ -927,20 +922,20 @@ struct ZLaneMap {  // lanes of one line are adjacent: the line is contiguous in 
 #define NS3D_MINCTA_Z64 3
 #endif
 
-template <int NZ, int P, bool UV, typename C>
+template <int NZ, int P, typename C>
 struct ZSmem {
   using F = LineFFT<NZ, P>;
   using LM = ZLaneMap<F::T>;
   using Rt = RealOf<C>;
-  // the stash: in tensor memory for FP64 lines (the nonlinear term's fifth
-  // component, beyond 128 columns, in shared memory), in shared memory for FP32
-  static constexpr bool TM = sizeof(C) == 16 && (UV || NZ > 64);
+  // the stash: in tensor memory for FP64 lines (its fifth component, beyond 128
+  // columns, in shared memory), in shared memory for FP32
+  static constexpr bool TM = sizeof(C) == 16 && NZ > 64;
   // rows staged by bulk copies; else (short lines, whose transforms are over
   // before a copy is) read where they are used
-  static constexpr bool STAGE = UV || NZ > 64;
-  static constexpr int NTM = TM ? (UV ? 6 : 4) : 0;
-  static constexpr int NST = TM ? (UV ? 0 : 1) : (UV ? 6 : 3);
-  static constexpr int NSLOT = UV ? 2 : (STAGE ? 1 : 0);  // staging slots
+  static constexpr bool STAGE = NZ > 64;
+  static constexpr int NTM = TM ? 4 : 0;
+  static constexpr int NST = TM ? 1 : 3;
+  static constexpr int NSLOT = STAGE ? 1 : 0;  // staging slots
   // a group: the lines of a warp, or a line of several warps
   static constexpr int GT = F::T > 32 ? F::T : 32;  // its threads
   static constexpr int GL = GT / F::T;              // its lines
@@ -974,7 +969,7 @@ struct ZSmem {
   static_assert(!TM || (BYTES + 1024) * (TM_MAXCTAS + 1) > 228 * 1024, "CTAs per SM bound");
   static_assert(BYTES <= 113 * 1024, "two CTAs per SM");
   // CTAs per SM asked of ptxas: as many as wanted where the shared memory fits
-  static constexpr int WANT = sizeof(C) == 8 ? NS3D_MINCTA_Z32 : (UV ? (P <= 8 ? 3 : 2) : (TM ? NS3D_MINCTA_Z64 : kMinCtasZ));
+  static constexpr int WANT = sizeof(C) == 8 ? NS3D_MINCTA_Z32 : (TM ? NS3D_MINCTA_Z64 : kMinCtasZ);
   static constexpr int fit(int n) {
     return n <= kMinCtasZ || (BYTES + 1024) * n <= 228 * 1024 ? n : fit(n - 1);
   }
@@ -999,11 +994,11 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 
 template <int NZ, int P, typename C>
-__global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, false, C>::MINC))
+__global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C>::MINC))
     z_kernel(const __grid_constant__ ZArgs<3, C> a, PassGeom g) {
   using F = LineFFT<NZ, P>;
   using Rt = RealOf<C>;
-  using S = ZSmem<NZ, P, false, C>;
+  using S = ZSmem<NZ, P, C>;
   constexpr bool TM = S::TM, STAGE = S::STAGE;
   constexpr int T = F::T;
   using LM = ZLaneMap<T>;
@@ -1236,216 +1231,118 @@ __global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, false, C>::MINC))
   }
 }
 
-// Stage k of the tangent z pass: the two rows it transforms.  The six
-// velocities in pairs, then per component i (d_x u_i, d_y u_i), (d_z u_i,
-// d_x v_i) with the first row times i kz, (d_y v_i, d_z v_i) with the second.
-template <typename C>
-struct ZStage {
-  static constexpr int N = 12;
-  const C* f1;
-  const C* f2;
-  int j;  // -1: velocities; else the place in a component's three
-  __device__ __forceinline__ ZStage(const ZArgs<6, C>& a, int k) {
-    if (k < 3) {
-      f1 = a.C[2 * k], f2 = a.C[2 * k + 1];
-      j = -1;
-    } else {
-      const int i = (k - 3) / 3;
-      j = k - 3 - 3 * i;
-      f1 = j == 0 ? a.E[i] : (j == 1 ? a.C[i] : a.D[3 + i]);
-      f2 = j == 0 ? a.D[i] : (j == 1 ? a.E[3 + i] : a.C[3 + i]);
-    }
-  }
+// The tangent form's rows of a z line: all fields' rows start at `base`.
+struct ZRun {
+  size_t base;
+  int Zc;
+  bool ask;  // this thread asks for the line's L2 prefetches
 };
+template <typename C>
+__device__ __forceinline__ void prefetch_z_pair(const C* f1, const C* f2, const ZRun& r) {
+  if (!r.ask) return;
+  prefetch_z_line(f1 + r.base, r.Zc);
+  prefetch_z_line(f2 + r.base, r.Zc);
+}
 
+// One component of B(u,v)_i = (v.grad) u_i + (u.grad) v_i in the z pass
+// (convolute_2p3_UV, Source/advection_2_3.cu:414-466); 3 paired C2R lines.
+template <int NZ, int P, typename C, typename Rt = RealOf<C>>
+__device__ __forceinline__ void uv_component(Rt (&q)[P], int i, const ZArgs<6, C>& a, int t,
+                                             Rt kfz, Rt sc, C* sbuf, const C* tw_s,
+                                             const Rt (&ux)[P], const Rt (&uy)[P],
+                                             const Rt (&uz)[P], const Rt (&vx)[P],
+                                             const Rt (&vy)[P], const Rt (&vz)[P],
+                                             const ZRun& r) {
+  using F = LineFFT<NZ, P>;
+  constexpr int PW = z_pw<NZ, P, C>();
+  C w[P];
+  // (d_x u_i, d_y u_i)
+  prefetch_z_pair(a.C[i], a.E[3 + i], r);
+  load_pair<NZ, P, false, false, false>(w, a.E[i] + r.base, a.D[i] + r.base, t, kfz, r.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) q[s] = vx[s] * (w[s].x * sc) + vy[s] * (w[s].y * sc);
+  // (d_z u_i, d_x v_i)
+  prefetch_z_pair(a.D[3 + i], a.C[3 + i], r);
+  load_pair<NZ, P, true, false, false>(w, a.C[i] + r.base, a.E[3 + i] + r.base, t, kfz, r.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) {
+    q[s] = q[s] + vz[s] * (w[s].x * sc);
+    q[s] = q[s] + ux[s] * (w[s].y * sc);
+  }
+  // (d_y v_i, d_z v_i)
+  if (i < 2) prefetch_z_pair(a.E[i + 1], a.D[i + 1], r);
+  load_pair<NZ, P, false, true, false>(w, a.D[3 + i] + r.base, a.C[3 + i] + r.base, t, kfz, r.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) q[s] = q[s] + (uy[s] * (w[s].x * sc) + uz[s] * (w[s].y * sc));
+}
+
+// The tangent z pass: 4 (6) points per thread, all six velocities and three
+// products in registers.  A form with 8 (12) points, staged rows and the
+// velocities in tensor memory is faster (linearised product 128^3 390 us
+// against 495, 96^3 206 against 251) but rounds differently, and the tangent of
+// a thin grid at a large step amplifies round-off past any fixed tolerance
+// (96 x 48 x 16, 12 steps: 1e-16 to 2e-9), so its results would not be those of
+// earlier releases to 1e-9.  Fields beyond what L2 keeps between inv_y and this
+// pass are asked for one transform ahead; below, that only costs issue slots.
 template <int NZ, int P, typename C>
-__global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, true, C>::MINC))
+__global__ void __launch_bounds__(kThreads, kMinCtasZ)
     z_uv_kernel(const __grid_constant__ ZArgs<6, C> a, PassGeom g) {
   using F = LineFFT<NZ, P>;
   using Rt = RealOf<C>;
-  using S = ZSmem<NZ, P, true, C>;
-  using St = ZStage<C>;
   constexpr int T = F::T;
-  constexpr bool TM = S::TM;
-  using LM = ZLaneMap<T>;
   constexpr int PW = z_pw<NZ, P, C>();
-  extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ uint32_t tm_base_s;  // TMEM address of the CTA's columns (TM)
-  const int warp = threadIdx.x >> 5;
+  using LM = ZLaneMap<T>;
+  __shared__ C tw_s[F::TWLEN];
+  __shared__ C sbuf_all[LM::LPC][F::BUF];
+  F::load_tw(tw_s, a.tw);
   int li, t;
   LM::get(li, t);
   const int nb = g.Nx * g.Ny;
   const int b = blockIdx.x * LM::LPC + li;
   const bool valid = b < nb;
   const size_t qbase = (size_t)(valid ? b : 0) * g.Mz;  // Qh
-  // staging: this thread's group of GL consecutive lines, its place in it, and
-  // the group's ring of two slots
-  constexpr int GL = S::GL;
-  const int grp = threadIdx.x / S::GT;
-  const int gt = threadIdx.x % S::GT;
-  const int row = li % GL;
-  const int b0 = blockIdx.x * LM::LPC + (li - row);  // the group's first line
-  const int nrow = nb - b0 < GL ? (nb - b0 > 0 ? nb - b0 : 0) : GL;
-  C* slots = (C*)(dsm + S::SLOT_OFF) + (size_t)grp * 2 * (S::SLOT / sizeof(C));
-  uint64_t* bar = (uint64_t*)(dsm + S::BAR_OFF) + 2 * grp;
-  volatile int* bad = (volatile int*)(dsm + S::BAD_OFF);  // a wait of this CTA gave up
-  if (threadIdx.x == 0) *bad = 0;
-  if (gt == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_init_fence();
-  }
-  const size_t field2 = S::KEPT ? (size_t)S::ROW : (size_t)GL * g.Zp;  // the second field's rows
-  // copies the rows of stage k into its slot (the group's first thread)
-  auto stage = [&](int k) {
-    const St s(a, k);
-    C* dst = slots + (k & 1) * (S::SLOT / sizeof(C));
-    const uint32_t bytes = (uint32_t)(nrow * (S::KEPT ? g.Zc : g.Zp)) * (uint32_t)sizeof(C);
-    const size_t off = (size_t)b0 * g.Zp;
-    mbar_expect_tx(&bar[k & 1], 2 * bytes);
-    if (bytes) {
-      bulk_load(dst, s.f1 + off, bytes, &bar[k & 1]);
-      bulk_load(dst + field2, s.f2 + off, bytes, &bar[k & 1]);
-    }
-  };
-  if (gt == 0) stage(0);  // in flight while the twiddles are read
-  if constexpr (TM) {
-    if (warp == 0) tmem_alloc_warp(&tm_base_s, S::TM_COLS);
-    tmem_fence_before_sync();
-  }
-  C* tw_s = (C*)dsm;
-  F::load_tw(tw_s, a.tw);  // ends with a CTA barrier: the TMEM address is published
-  uint32_t tm = 0;         // this warp's lane quarter, column 0
-  if constexpr (TM) {
-    tmem_fence_after_sync();
-    tm = tmem_addr(tm_base_s, 32 * (warp & 3), 0);
-  }
-  C* sbuf = (C*)(dsm + S::SBUF_OFF) + li * S::BUF;
-  Rt* stash = (Rt*)(dsm + S::ST_OFF) + threadIdx.x;
-  // stash component c: the P values v(s)
-  auto park = [&](int c, auto v) {
-    if constexpr (TM) {
-#pragma unroll
-      for (int s0 = 0; s0 < P; s0 += 4) {
-        uint32_t r[8];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const double d = v(s0 + k);
-          r[2 * k] = (uint32_t)__double2loint(d);
-          r[2 * k + 1] = (uint32_t)__double2hiint(d);
-        }
-        tmem_st8(tm + (uint32_t)(c * 2 * P + 2 * s0), r);
-      }
-      tmem_wait_st();
-    } else {
-#pragma unroll
-      for (int s = 0; s < P; ++s) stash[(c * P + s) * kThreads] = v(s);
-    }
-  };
-  // hands f(s, values of the NC components from c0 on) every sample
-  auto parked = [&](auto nc, int c0, auto f) {
-    constexpr int NC = decltype(nc)::value;
-    if constexpr (TM) {
-#pragma unroll
-      for (int s0 = 0; s0 < P; s0 += 4) {
-        uint32_t r[NC][8];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) tmem_ld8(tm + (uint32_t)((c0 + c) * 2 * P + 2 * s0), r[c]);
-        tmem_wait_ld();
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          Rt v[NC];
-#pragma unroll
-          for (int c = 0; c < NC; ++c)
-            v[c] = __hiloint2double((int)r[c][2 * k + 1], (int)r[c][2 * k]);
-          f(s0 + k, v);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int s = 0; s < P; ++s) {
-        Rt v[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) v[c] = stash[((c0 + c) * P + s) * kThreads];
-        f(s, v);
-      }
-    }
-  };
-  using One = std::integral_constant<int, 1>;
-  using Two = std::integral_constant<int, 2>;
+  C* sbuf = sbuf_all[li];
   const Rt sc = (Rt)g.inv_vol;
   const Rt kfz = (Rt)g.kfz;
+  const bool beyond = (size_t)g.Nx * g.Ny * g.Zp * (9 * sizeof(double2)) > ((size_t)64 << 20);
+  const ZRun r{(size_t)(valid ? b : 0) * g.Zp, g.Zc, valid && t == 0 && beyond};
   C w[P];
-  Rt q0[P], qy[P], qz[P];
-#pragma unroll 1
-  for (int k = 0; k < St::N; ++k) {
-    // the next stage's rows, into the slot of stage k - 1: the group's threads
-    // have read it (they have passed a barrier of its transform)
-    if constexpr (T == 1) __syncwarp();  // (one-stage transforms have none)
-    if (gt == 0 && k + 1 < St::N && !*bad) {
-      fence_proxy_async_smem();
-      stage(k + 1);
-    }
-    mbar_wait(&bar[k & 1], (uint32_t)((k >> 1) & 1), a.err, bad);
-    {
-      const St st(a, k);
-      const C* f1 = slots + (k & 1) * (S::SLOT / sizeof(C)) + (size_t)row * g.Zp;  // (row 0 where GL = 1)
-      const C* f2 = f1 + field2;
-      if (st.j < 1)
-        load_pair<NZ, P, false, false, true>(w, f1, f2, t, kfz, g.Zc);
-      else if (st.j == 1)
-        load_pair<NZ, P, true, false, true>(w, f1, f2, t, kfz, g.Zc);
-      else
-        load_pair<NZ, P, false, true, true>(w, f1, f2, t, kfz, g.Zc);
-    }
-    F::template run<+1, PW>(w, t, sbuf, tw_s);
-    // B(u,v)_i = (v.grad) u_i + (u.grad) v_i (convolute_2p3_UV,
-    // Source/advection_2_3.cu:414-466); fields 0..2 are u, 3..5 are v
-    const int j = k < 3 ? -1 : (k - 3) % 3;
-    if (k < 3) {
-      park(2 * k, [&](int s) { return w[s].x * sc; });
-      park(2 * k + 1, [&](int s) { return w[s].y * sc; });
-    } else if (j == 0) {  // (d_x u_i, d_y u_i); the previous component moves on
+  Rt ux[P], uy[P], uz[P], vx[P], vy[P], vz[P], q0[P], q1[P], q2[P];
+  prefetch_z_pair(a.C[2], a.C[3], r);
+  load_pair<NZ, P, false, false, false>(w, a.C[0] + r.base, a.C[1] + r.base, t, kfz, r.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
 #pragma unroll
-      for (int s = 0; s < P; ++s) { q0[s] = qy[s]; qy[s] = qz[s]; }
-      parked(Two{}, 3, [&](int s, const Rt* v) {
-        qz[s] = v[0] * (w[s].x * sc) + v[1] * (w[s].y * sc);
-      });
-    } else if (j == 1) {  // (d_z u_i, d_x v_i)
-      parked(One{}, 5, [&](int s, const Rt* v) { qz[s] = qz[s] + v[0] * (w[s].x * sc); });
-      parked(One{}, 0, [&](int s, const Rt* v) { qz[s] = qz[s] + v[0] * (w[s].y * sc); });
-    } else {  // (d_y v_i, d_z v_i)
-      parked(Two{}, 1, [&](int s, const Rt* v) {
-        qz[s] = qz[s] + (v[0] * (w[s].x * sc) + v[1] * (w[s].y * sc));
-      });
-    }
-  }
-  if (gt == 0 && *bad) {  // a broken ring: the last copies may still be in flight
-    mbar_drain(&bar[0], (uint32_t)(((St::N - 2) >> 1) & 1));
-    mbar_drain(&bar[1], (uint32_t)(((St::N - 1) >> 1) & 1));
-  }
+  for (int s = 0; s < P; ++s) { ux[s] = w[s].x * sc; uy[s] = w[s].y * sc; }
+  prefetch_z_pair(a.C[4], a.C[5], r);
+  load_pair<NZ, P, false, false, false>(w, a.C[2] + r.base, a.C[3] + r.base, t, kfz, r.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) { uz[s] = w[s].x * sc; vx[s] = w[s].y * sc; }
+  prefetch_z_pair(a.E[0], a.D[0], r);
+  load_pair<NZ, P, false, false, false>(w, a.C[4] + r.base, a.C[5] + r.base, t, kfz, r.Zc);
+  F::template run<+1, PW>(w, t, sbuf, tw_s);
+#pragma unroll
+  for (int s = 0; s < P; ++s) { vy[s] = w[s].x * sc; vz[s] = w[s].y * sc; }
+  uv_component<NZ, P>(q0, 0, a, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, r);
+  uv_component<NZ, P>(q1, 1, a, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, r);
+  uv_component<NZ, P>(q2, 2, a, t, kfz, sc, sbuf, tw_s, ux, uy, uz, vx, vy, vz, r);
   // forward R2C along z: (Q_x, Q_y) packed, then Q_z alone
-#pragma unroll 1
-  for (int r = 0; r < 2; ++r) {
 #pragma unroll
-    for (int s = 0; s < P; ++s) w[s] = r == 0 ? mkc<C>(q0[s], qy[s]) : mkc<C>(qz[s], (Rt)0);
-    F::template run<-1, PW>(w, t, sbuf, tw_s);
-    if (r == 0) {
-      store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
-    } else if (valid) {
+  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q0[s], q1[s]);
+  F::template run<-1, PW>(w, t, sbuf, tw_s);
+  store_pair_spectrum<NZ, P>(w, sbuf, t, a.Qh[0], a.Qh[1], qbase, valid);
 #pragma unroll
-      for (int s = 0; s < P; ++s) {
-        const int k = t + T * s;
-        if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
-      }
+  for (int s = 0; s < P; ++s) w[s] = mkc<C>(q2[s], (Rt)0);
+  F::template run<-1, PW>(w, t, sbuf, tw_s);
+  if (valid) {
+#pragma unroll
+    for (int s = 0; s < P; ++s) {
+      const int k = t + T * s;
+      if (k <= NZ / 2) a.Qh[2][qbase + k] = w[s];
     }
-  }
-  if constexpr (TM) {
-    // every thread's TMEM reads have completed (waited); free the columns
-    tmem_fence_before_sync();
-    __syncthreads();
-    tmem_fence_after_sync();
-    if (warp == 0) tmem_dealloc_warp(tm_base_s, S::TM_COLS);
   }
 }
 
