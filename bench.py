@@ -338,24 +338,23 @@ def run_ours(args, world, rank, local, pg):
 
     # per-pass timing (CUDA events on the launching stream), dominant kernel
     names = ["inv_x", "inv_y", "z", "fwd_y", "fwd_x"]
-    # algorithmic bytes per launch; FP32 scratch halves every field but the state
-    alg = ([6 * Sc, 7.5 * Sc, 6 * Sc, 3 * Sc, 7.5 * Sc] if fp32 else
-           [9 * Sc, 15 * Sc, 12 * Sc, 6 * Sc, 9 * Sc])
+    # algorithmic bytes per launch: the inverse passes move what the 2/3 mask
+    # leaves (0.52 of the modes, 0.60 of the x lines, 2/3 of the y and z lines);
+    # FP32 scratch halves every field but the state
+    h = 0.5 if fp32 else 1.0
+    alg = [(3 * 0.52 + 6 * 0.60 * h) * Sc, (6 * 0.60 + 9 * 2 / 3) * h * Sc,
+           (9 * 2 / 3 + 3) * h * Sc, 6 * h * Sc, (3 * h + 6) * Sc]
     with torch.cuda.stream(stream):
         pm = S.profile_passes(U, dt, Re, reps=20)
     dom = max(range(5), key=lambda i: pm[i])
     peak, peak_src = peaks()
     achieved = alg[dom] / (pm[dom] * 1e-3) / 1e9
-    # the kernels the step launches: the nonlinear term's z pass with the
-    # velocities in shared memory for FP64 lines; the ring-pipelined fwd_x
-    # where a line fits in a warp (8 points per thread, 12 for multiples of 3)
-    t_ring = N // (12 if N % 3 == 0 else min(N, 8))
-    t_plain = N // (12 if N % 3 == 0 else min(N, 16))
-    ring = t_ring <= 32 and (t_ring == 32 or t_plain < 8)
+    # fwd_x: 12-point lines spread over the CTA keep fwd_x_kernel, the rest its ring
+    ring = N % 3 != 0 or N // 12 < 8 or N // 12 >= 32
     # inv_y's tile 2 is the bulk-copy (TMA) form for FP64 lines
     ytma = S.tiles[1] == 2 and not fp32
     kname = {0: "inv_x_kernel", 1: "inv_y_tma_kernel" if ytma else "inv_y_kernel",
-             2: "z_kernel" if fp32 else "z_kernel_st",
+             2: "z_kernel",
              3: "fwd_y_kernel", 4: "fwd_x_ring_kernel" if ring else "fwd_x_kernel"}[dom]
     traffic = traffic_from_profiles(kname, N)
     roofline = {"bound": "hbm", "kernel": kname, "achieved": round(achieved, 1),
@@ -518,9 +517,10 @@ def run_reference(args, world, rank, local, pg):
 # ---------------------------------------------------------------------------
 def arnoldi_bytes(n, m):
     """Gram-Schmidt bytes of one factorisation: the sum over columns of
-    4 (j+1) n 8 B (one classical pass plus one reorthogonalisation pass,
-    each reading V(:, 0..j) twice)."""
-    return sum(4 * (j + 1) * n * 8 for j in range(1, m))
+    3 (j+1) n 8 B: the dots, the update that forms the reorthogonalisation's
+    dots, and its update each read V(:, 0..j) once (4 past 48 columns, where
+    every pass reads it by itself)."""
+    return sum((3 if j < 48 else 4) * (j + 1) * n * 8 for j in range(1, m))
 
 
 def arnoldi_start(n, seed):
@@ -796,7 +796,7 @@ def run_ours_ira(args, world, rank, local, pg):
     gs = 0
     for c in cols:
         for j in range(m - c, m):
-            gs += 4 * (j + 1) * 8 * n
+            gs += (3 if j < 48 else 4) * (j + 1) * 8 * n
     B = mv_bytes * calls + gs
     # the map alone, timed on the device
     x = torch.as_tensor(ira_start(n, 99), device="cuda")
