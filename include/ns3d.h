@@ -89,6 +89,13 @@ const char* ns3d_status_string(ns3d_status s);
  * otherwise.  Synchronous on the current device; allocates a 4-byte flag. */
 ns3d_status ns3d_selftest_bounded_wait(double* seconds);
 
+/* Runs on the current device the wait that a z pass ends with when its row
+ * copies broke down: the drain of the copies it armed last (stage `last`,
+ * 0 .. 5).  complete = 0 leaves that stage open: *drained must be 0, after the
+ * bounded wait (0.1 s).  complete = 1 completes it 20 us later: *drained must
+ * be 1 (-1: the drain returned before that). */
+ns3d_status ns3d_selftest_stage_drain(int last, int complete, int* drained);
+
 /* Device bytes the handle holds (scratch + tables). */
 size_t ns3d_device_bytes(const ns3d_solver* h);
 

@@ -1215,7 +1215,8 @@ __global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C>::MINC))
 #pragma unroll 1
     for (int k = 0; k < 6; ++k) transform(k);
   }
-  if (STAGE && gt == 0 && *bad) mbar_drain(bar, 1);  // a broken ring: the last copies may be in flight
+  // a broken ring, at any stage: the copies armed last may be in flight
+  if (STAGE && gt == 0 && *bad) mbar_drain_current(bar);
   if constexpr (TM) parked(3, [&](int s, Rt v) { q0[s] = v; });
   // R2C of (Q_x, Q_y) packed
 #pragma unroll

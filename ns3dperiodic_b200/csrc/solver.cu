@@ -331,8 +331,46 @@ __global__ void bounded_wait_probe(int* err) {
   __syncthreads();
   ns3d::mbar_wait(&bar, 0, err, &bad);
 }
+
+// Thread 0 arms phases 0 .. last of an mbarrier, completes all but the last and
+// drains it; thread 32 completes the last some 20 us later, if asked to.
+// *out: 1 where the drain saw the phase complete, after thread 32 had said so;
+// 0 where it gave up; -1 where it returned early.
+__global__ void stage_drain_probe(int last, int complete, int* out) {
+  __shared__ uint64_t bar;
+  __shared__ volatile int done;
+  if (threadIdx.x == 0) {
+    ns3d::mbar_init(&bar, 1);
+    done = 0;
+    for (int k = 0; k < last; ++k) ns3d::mbar_expect_tx(&bar, 0);
+  }
+  __syncthreads();
+  if (threadIdx.x == 32 && complete) {
+    for (int i = 0; i < 20; ++i) __nanosleep(1000);
+    done = 1;
+    ns3d::mbar_expect_tx(&bar, 0);
+  }
+  if (threadIdx.x == 0) {
+    const bool saw = ns3d::mbar_drain_current(&bar);
+    *out = !saw ? 0 : (done ? 1 : -1);
+  }
+}
 }  // namespace
 }  // extern "C++"
+
+ns3d_status ns3d_selftest_stage_drain(int last, int complete, int* drained) {
+  if (last < 0 || last > 5 || !drained) return NS3D_ERR_BAD_ARG;
+  int* out = nullptr;
+  if (cudaMalloc(&out, sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    return NS3D_ERR_OOM;
+  }
+  stage_drain_probe<<<1, 64>>>(last, complete, out);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpy(drained, out, sizeof(int), cudaMemcpyDeviceToHost);
+  cudaFree(out);
+  return e == cudaSuccess ? NS3D_OK : NS3D_ERR_CUDA;
+}
 
 ns3d_status ns3d_selftest_bounded_wait(double* seconds) {
   int* flag = nullptr;

@@ -123,6 +123,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
 __device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity) {
   return mbar_poll(bar, parity);
 }
+// ... whichever phase was armed last (by this thread, which arms no more): waits
+// for the phase in progress, whose parity is not that of the last complete one.
+// Where the last armed phase is complete, the one in progress was never armed:
+// the wait runs out.
+__device__ __forceinline__ bool mbar_drain_current(uint64_t* bar) {
+  return mbar_drain(bar, mbar_test_wait(bar, 0) ? 1u : 0u);
+}
 
 // orders this thread's earlier generic-proxy accesses of shared memory
 // before later async-proxy (TMA) writes to it
