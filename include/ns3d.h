@@ -96,6 +96,11 @@ ns3d_status ns3d_selftest_bounded_wait(double* seconds);
  * be 1 (-1: the drain returned before that). */
 ns3d_status ns3d_selftest_stage_drain(int last, int complete, int* drained);
 
+/* Runs on the current device a bounded wait whose phase completes between its
+ * last poll and the end of its limit (as for a context switched out there):
+ * *seen must be 1. */
+ns3d_status ns3d_selftest_late_phase(int* seen);
+
 /* Device bytes the handle holds (scratch + tables). */
 size_t ns3d_device_bytes(const ns3d_solver* h);
 

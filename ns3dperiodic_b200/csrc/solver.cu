@@ -358,6 +358,38 @@ __global__ void stage_drain_probe(int last, int complete, int* out) {
 }  // namespace
 }  // extern "C++"
 
+extern "C++" {
+namespace {
+// A wait whose clock, read after failed polls, says that its limit has passed,
+// the phase having completed just before: what a context that was switched out
+// there sees.
+__global__ void late_phase_probe(int* out) {
+  __shared__ uint64_t bar;
+  ns3d::mbar_init(&bar, 1);
+  int reads = 0;
+  *out = ns3d::mbar_poll(&bar, 0, [&]() -> unsigned long long {
+    if (reads++ == 0) return 0;
+    ns3d::mbar_expect_tx(&bar, 0);
+    return 2 * ns3d::kMbarLimitNs;
+  });
+}
+}  // namespace
+}  // extern "C++"
+
+ns3d_status ns3d_selftest_late_phase(int* seen) {
+  int* out = nullptr;
+  if (!seen) return NS3D_ERR_BAD_ARG;
+  if (cudaMalloc(&out, sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    return NS3D_ERR_OOM;
+  }
+  late_phase_probe<<<1, 1>>>(out);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpy(seen, out, sizeof(int), cudaMemcpyDeviceToHost);
+  cudaFree(out);
+  return e == cudaSuccess ? NS3D_OK : NS3D_ERR_CUDA;
+}
+
 ns3d_status ns3d_selftest_stage_drain(int last, int complete, int* drained) {
   if (last < 0 || last > 5 || !drained) return NS3D_ERR_BAD_ARG;
   int* out = nullptr;

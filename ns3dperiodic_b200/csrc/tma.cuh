@@ -90,9 +90,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // Polls until the phase completes (true) or the limits of a bounded wait
-// pass (false).
-__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
-  const unsigned long long t0 = global_ns();
+// pass (false).  The last look comes after the limit: a context that was
+// switched out between a failed poll and the clock finds the phase that
+// completed meanwhile.  now: the clock (the self-test brings its own).
+template <typename Clock>
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity, Clock now) {
+  const unsigned long long t0 = now();
   for (int i = 0; i < kMbarSpins; ++i) {
     if (NS3D_TMA_WAIT) {
       if (mbar_try_wait(bar, parity, kMbarHintNs)) return true;
@@ -100,9 +103,12 @@ __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
       if (mbar_test_wait(bar, parity)) return true;
       if (i >= kMbarFast) __nanosleep(kMbarSleepNs);
     }
-    if ((i & 63) == 63 && global_ns() - t0 > kMbarLimitNs) break;
+    if ((i & 63) == 63 && now() - t0 > kMbarLimitNs) break;
   }
-  return false;
+  return mbar_test_wait(bar, parity);
+}
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
+  return mbar_poll(bar, parity, [] { return global_ns(); });
 }
 
 // Bounded wait; false (and *err set) when it gave up.  `bad` is a CTA flag in
