@@ -365,7 +365,8 @@ cudaError_t launch_inv_y(const InvYArgs<NF, C>& a, const PassGeom& gi, cudaStrea
   }
 }
 
-template <typename C, int NF>
+// STAGED: as z_kernel (the tangent form stages nothing)
+template <typename C, int NF, bool STAGED = true>
 cudaError_t launch_z(const ZArgs<NF, C>& a, const PassGeom& gi, cudaStream_t st) {
   const PassGeom g = planes_geom(gi);
   const long long lines = (long long)g.Nx * g.Ny;
@@ -378,11 +379,12 @@ cudaError_t launch_z(const ZArgs<NF, C>& a, const PassGeom& gi, cudaStream_t st)
       z_uv_kernel<N, P, C>                                                            \
           <<<blocks_for(lines, lines_per_cta_z<N, P>()), kThreads, 0, st>>>(a, g);    \
     } else {                                                                          \
-      using S = ZSmem<N, P, C>;                                                       \
+      constexpr bool ST = STAGED || N <= 64; /* short lines: one form */              \
+      using S = ZSmem<N, P, C, ST>;                                                   \
       const unsigned groups = blocks_for(lines, S::LM::LPC);                          \
-      const unsigned grid = persistent_grid<KTag<40, N, P, prec_tag<C>()>>(           \
-          z_kernel<N, P, C>, S::BYTES, groups);                                       \
-      z_kernel<N, P, C><<<grid, kThreads, S::BYTES, st>>>(a, g);                      \
+      const unsigned grid = persistent_grid<KTag<ST ? 40 : 41, N, P, prec_tag<C>()>>( \
+          z_kernel<N, P, C, ST>, S::BYTES, groups);                                   \
+      z_kernel<N, P, C, ST><<<grid, kThreads, S::BYTES, st>>>(a, g);                  \
     }                                                                                 \
     return cudaGetLastError();                                                        \
   }

@@ -202,7 +202,9 @@ extern "C" ns3d_status ns3d_convolution_noalloc(int Nx, int Ny, int Nz, double L
   fx.Re = 1.0;
   if (ns3d::run_inv_x(ax, g, st) != cudaSuccess) return NS3D_ERR_CUDA;
   if (ns3d::run_inv_y(ay, g, st) != cudaSuccess) return NS3D_ERR_CUDA;
-  if (ns3d::run_z(az, g, st) != cudaSuccess) return NS3D_ERR_CUDA;
+  // rows read in place: a caller without a handle has nowhere to learn of a
+  // staged row that did not arrive
+  if (ns3d::launch_z<double2, 3, false>(az, g, st) != cudaSuccess) return NS3D_ERR_CUDA;
   if (ns3d::run_fwd_y(fy, g, st) != cudaSuccess) return NS3D_ERR_CUDA;
   if (ns3d::run_fwd_x(ns3d::kConvOut, false, fx, g, st) != cudaSuccess) return NS3D_ERR_CUDA;
   return NS3D_OK;

@@ -922,7 +922,10 @@ struct ZLaneMap {  // lanes of one line are adjacent: the line is contiguous in 
 #define NS3D_MINCTA_Z64 3
 #endif
 
-template <int NZ, int P, typename C>
+// STAGED: long lines' rows come through bulk copies (the handles' passes); else
+// every row is read where it is used, and the kernel waits on no copy: the form
+// of the entry point that has no handle to report a wait that gave up on
+template <int NZ, int P, typename C, bool STAGED = true>
 struct ZSmem {
   using F = LineFFT<NZ, P>;
   using LM = ZLaneMap<F::T>;
@@ -932,7 +935,7 @@ struct ZSmem {
   static constexpr bool TM = sizeof(C) == 16 && NZ > 64;
   // rows staged by bulk copies; else (short lines, whose transforms are over
   // before a copy is) read where they are used
-  static constexpr bool STAGE = NZ > 64;
+  static constexpr bool STAGE = STAGED && NZ > 64;
   static constexpr int NTM = TM ? 4 : 0;
   static constexpr int NST = TM ? 1 : 3;
   static constexpr int NSLOT = STAGE ? 1 : 0;  // staging slots
@@ -993,12 +996,12 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
       : "memory");
 }
 
-template <int NZ, int P, typename C>
-__global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C>::MINC))
+template <int NZ, int P, typename C, bool STAGED = true>
+__global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C, STAGED>::MINC))
     z_kernel(const __grid_constant__ ZArgs<3, C> a, PassGeom g) {
   using F = LineFFT<NZ, P>;
   using Rt = RealOf<C>;
-  using S = ZSmem<NZ, P, C>;
+  using S = ZSmem<NZ, P, C, STAGED>;
   constexpr bool TM = S::TM, STAGE = S::STAGE;
   constexpr int T = F::T;
   using LM = ZLaneMap<T>;
