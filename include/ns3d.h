@@ -101,6 +101,11 @@ ns3d_status ns3d_selftest_stage_drain(int last, int complete, int* drained);
  * *seen must be 1. */
 ns3d_status ns3d_selftest_late_phase(int* seen);
 
+/* Makes the next capture of a tangent step by ns3d_jvp_steps on this handle
+ * fail with NS3D_ERR_CUDA, as it does where recording a launch fails: graph 0,
+ * a call's first step, or 1, its later steps. */
+ns3d_status ns3d_selftest_fail_capture(ns3d_solver* h, int graph);
+
 /* Device bytes the handle holds (scratch + tables). */
 size_t ns3d_device_bytes(const ns3d_solver* h);
 

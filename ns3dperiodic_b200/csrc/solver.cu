@@ -658,6 +658,13 @@ ns3d_status ns3d_synchronize(ns3d_solver* h) {
   return NS3D_OK;
 }
 
+ns3d_status ns3d_selftest_fail_capture(ns3d_solver* h, int graph) {
+  NS3D_TRY(check_handle(h));
+  if (graph < 0 || graph > 1) return fail(h, NS3D_ERR_BAD_ARG, "graph is 0 or 1");
+  h->selftest_fail_capture = graph;
+  return NS3D_OK;
+}
+
 ns3d_status ns3d_set_forcing(ns3d_solver* h, const ns3d_complex* fx, const ns3d_complex* fy,
                              const ns3d_complex* fz) {
   NS3D_TRY(check_handle(h));
@@ -998,6 +1005,11 @@ ns3d_status ns3d_jvp_steps(ns3d_solver* h, ns3d_complex* ux, ns3d_complex* uy, n
         if (e) cudaGraphExecDestroy(e);
         e = nullptr;
       }
+      // the key goes with whatever is captured from here on, also where the
+      // second capture fails and the call returns with the first in place
+      for (int i = 0; i < 6; ++i) h->jvp_key[i] = key[i];
+      h->jvp_dt = dt; h->jvp_Re = Re; h->jvp_stream = h->stream;
+      h->jvp_fversion = h->f_version;
     }
     // [0] the first step of a call, [1] the later ones
     for (int k = 0; k < (nsteps > 1 && apart ? 2 : 1) && !h->graphs_off; ++k) {
@@ -1006,6 +1018,10 @@ ns3d_status ns3d_jvp_steps(ns3d_solver* h, ns3d_complex* ux, ns3d_complex* uy, n
       cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
         ns3d_status s = one(k == 1);
+        if (h->selftest_fail_capture == k) {
+          h->selftest_fail_capture = -1;
+          s = fail(h, NS3D_ERR_CUDA, "self-test: failed capture");
+        }
         e = cudaStreamEndCapture(h->stream, &graph);
         if (s != NS3D_OK) {
           if (graph) cudaGraphDestroy(graph);
@@ -1021,9 +1037,6 @@ ns3d_status ns3d_jvp_steps(ns3d_solver* h, ns3d_complex* ux, ns3d_complex* uy, n
       }
     }
     if (!h->graphs_off) {
-      for (int i = 0; i < 6; ++i) h->jvp_key[i] = key[i];
-      h->jvp_dt = dt; h->jvp_Re = Re; h->jvp_stream = h->stream;
-      h->jvp_fversion = h->f_version;
       for (int s = 0; s < nsteps; ++s)
         NS3D_CHECK(h, cudaGraphLaunch(h->jvp_exec[s > 0 && apart], h->stream), "graph launch");
       return NS3D_OK;

@@ -71,6 +71,7 @@ struct ns3d_solver {
   double jvp_dt = 0.0, jvp_Re = 0.0;
   cudaStream_t jvp_stream = nullptr;
   int jvp_fversion = -1;
+  int selftest_fail_capture = -1;  // the next capture of this jvp_exec fails
   // tensor maps of inv_y's bulk-copy form (tile 2 of the inv_y family) over
   // A and B; null when the extent has no such form
   ns3d::InvYMaps* ymaps = nullptr;
