@@ -73,7 +73,11 @@ int ns3d_supported_extent(int n);
  * every later launch of this handle. */
 ns3d_status ns3d_set_stream(ns3d_solver* h, void* stream);
 
-/* Blocks until the handle's stream is idle. */
+/* Blocks until the handle's stream is idle.  NS3D_ERR_TIMEOUT where a bounded
+ * wait of a pass gave up: the results since the last report are invalid, the
+ * context is usable.  The calls that hand results to the host (diagnostics, the
+ * record, the spectrum, Shapiro's error, saved states, an ensemble's
+ * diagnostics) report it likewise, whichever comes first, once. */
 ns3d_status ns3d_synchronize(ns3d_solver* h);
 
 /* Human-readable text of the last error on this handle ("" if none). */
@@ -100,6 +104,10 @@ ns3d_status ns3d_selftest_stage_drain(int last, int complete, int* drained);
  * last poll and the end of its limit (as for a context switched out there):
  * *seen must be 1. */
 ns3d_status ns3d_selftest_late_phase(int* seen);
+
+/* Enqueues on the handle's stream a bounded wait that gives up and reports on
+ * the handle's flag, as a pass whose copies break down does. */
+ns3d_status ns3d_selftest_expire_wait(ns3d_solver* h);
 
 /* Makes the next capture of a tangent step by ns3d_jvp_steps on this handle
  * fail with NS3D_ERR_CUDA, as it does where recording a launch fails: graph 0,

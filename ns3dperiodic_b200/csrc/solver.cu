@@ -268,6 +268,23 @@ ns3d_status check_handle(ns3d_solver* h) {
   return NS3D_OK;
 }
 
+ns3d_status flagged(ns3d_solver* h, const double* word) {
+  int flag;
+  std::memcpy(&flag, word, sizeof(int));
+  if (!flag) return NS3D_OK;
+  cudaMemsetAsync(h->dev_err, 0, sizeof(int), h->stream);
+  return fail(h, NS3D_ERR_TIMEOUT, "a bounded wait of a pass kernel gave up");
+}
+
+ns3d_status settle(ns3d_solver* h, const char* where) {
+  double word = 0.0;
+  NS3D_CHECK(h, cudaStreamSynchronize(h->stream), where);
+  NS3D_CHECK(h, cudaMemcpyAsync(&word, h->dev_err, sizeof(int), cudaMemcpyDeviceToHost,
+                                h->stream), "error flag");
+  NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "error flag");
+  return flagged(h, &word);
+}
+
 ns3d_status check_step(ns3d_solver* h, double dt, double Re) {
   if (!(Re > 0.0) || !std::isfinite(Re) || !std::isfinite(dt))
     return fail(h, NS3D_ERR_BAD_ARG, "dt must be finite and Re > 0");
@@ -577,9 +594,11 @@ ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double L
       cudaMalloc(&h->f_idx, sizeof(int) * kForcingCap) != cudaSuccess ||
       cudaMalloc(&h->f_val, sizeof(double2) * 3 * kForcingCap) != cudaSuccess ||
       cudaMalloc(&h->diag_partial, sizeof(double) * 3 * kDiagBlocks) != cudaSuccess ||
-      cudaMalloc(&h->diag_out, sizeof(double) * 3 * batch) != cudaSuccess)
+      cudaMalloc(&h->results, sizeof(double) * (kFlagAt + 1 + 3 * batch)) != cudaSuccess)
     return bail(NS3D_ERR_OOM);
-  if (cudaMalloc(&h->dev_err, sizeof(int)) != cudaSuccess) return bail(NS3D_ERR_OOM);
+  h->rec_out = h->results;
+  h->dev_err = reinterpret_cast<int*>(h->results + kFlagAt);
+  h->diag_out = h->results + kFlagAt + 1;
   cudaMemset(h->dev_err, 0, sizeof(int));
   build_inv_y_maps(h);
   if (batch > 1) {
@@ -616,12 +635,10 @@ ns3d_status ns3d_destroy(ns3d_solver* h) {
   cudaFree(h->f_idx);
   cudaFree(h->f_val);
   cudaFree(h->diag_partial);
-  cudaFree(h->diag_out);
   cudaFree(h->dtRe);
   cudaFree(h->rec_tab);
   cudaFree(h->rec_partial);
-  cudaFree(h->rec_out);
-  cudaFree(h->dev_err);
+  cudaFree(h->results);
   delete h->ymaps;
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   delete h;
@@ -643,18 +660,13 @@ ns3d_status ns3d_set_stream(ns3d_solver* h, void* stream) {
 
 ns3d_status ns3d_synchronize(ns3d_solver* h) {
   NS3D_TRY(check_handle(h));
-  NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
-  // a bounded wait of a bulk-copy pass that gave up (its results are invalid)
-  int flag = 0;
-  if (h->dev_err) {
-    NS3D_CHECK(h, cudaMemcpyAsync(&flag, h->dev_err, sizeof(int), cudaMemcpyDeviceToHost,
-                                  h->stream), "error flag");
-    NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "error flag");
-  }
-  if (flag) {
-    cudaMemsetAsync(h->dev_err, 0, sizeof(int), h->stream);
-    return fail(h, NS3D_ERR_TIMEOUT, "a bounded wait of a pass kernel gave up");
-  }
+  return settle(h, "cudaStreamSynchronize");
+}
+
+ns3d_status ns3d_selftest_expire_wait(ns3d_solver* h) {
+  NS3D_TRY(check_handle(h));
+  bounded_wait_probe<<<1, 64, 0, h->stream>>>(h->dev_err);
+  NS3D_CHECK(h, cudaGetLastError(), "bounded_wait_probe");
   return NS3D_OK;
 }
 
@@ -852,7 +864,7 @@ ns3d_status ns3d_save_control_fourier(ns3d_solver* h, const char* path, const ns
     NS3D_CHECK(h, cudaMemcpyAsync(b[c].data(), d[c], sizeof(ns3d_complex) * h->nc,
                                   cudaMemcpyDeviceToHost, h->stream), "checkpoint copy");
   }
-  NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "checkpoint sync");
+  NS3D_TRY(settle(h, "checkpoint sync"));
   const ns3d_status s = ns3d_write_control_fourier_host(path, h->Nx, h->Ny, h->Nz, b[0].data(),
                                                         b[1].data(), b[2].data());
   return s == NS3D_OK ? s : fail(h, s, std::string("cannot write ") + path);
@@ -890,7 +902,7 @@ ns3d_status ns3d_save_control_file(ns3d_solver* h, const char* path, const ns3d_
     NS3D_CHECK(h, cudaMemcpyAsync(b[c].data(), phys, sizeof(double) * nr, cudaMemcpyDeviceToHost,
                                   h->stream), "checkpoint copy");
   }
-  NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "checkpoint sync");
+  NS3D_TRY(settle(h, "checkpoint sync"));
   const ns3d_status s = ns3d_write_control_file_host(path, h->Nx, h->Ny, h->Nz, b[0].data(),
                                                      b[1].data(), b[2].data());
   return s == NS3D_OK ? s : fail(h, s, std::string("cannot write ") + path);
@@ -1152,10 +1164,12 @@ ns3d_status ns3d_diagnostics(ns3d_solver* h, const ns3d_complex* ux, const ns3d_
   NS3D_CHECK(h, cudaGetLastError(), "diag_partial");
   ns3d::diag_final_kernel<<<1, 1024, 0, h->stream>>>(h->diag_partial, kDiagBlocks, h->diag_out);
   NS3D_CHECK(h, cudaGetLastError(), "diag_final");
-  double r[3];
-  NS3D_CHECK(h, cudaMemcpyAsync(r, h->diag_out, sizeof(r), cudaMemcpyDeviceToHost, h->stream),
-             "diag copy");
+  double out[4];  // the flag, then the sums
+  NS3D_CHECK(h, cudaMemcpyAsync(out, h->diag_out - 1, sizeof(out), cudaMemcpyDeviceToHost,
+                                h->stream), "diag copy");
   NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "diag sync");
+  NS3D_TRY(flagged(h, out));
+  const double* r = out + 1;
   if (energy) *energy = r[0];
   if (dissipation) *dissipation = r[1];
   if (div_max) *div_max = r[2];
@@ -1234,10 +1248,8 @@ ns3d_status ensure_record(ns3d_solver* h) {
   for (int i = 0; i < 3; ++i) h->rec_points[i] = P[i];
   double2* t = nullptr;
   double* part = nullptr;
-  double* out = nullptr;
   cudaError_t e = cudaMalloc(&t, sizeof(double2) * tab.size());
   if (e == cudaSuccess) e = cudaMalloc(&part, sizeof(double) * ns3d::kRecordSums * kDiagBlocks);
-  if (e == cudaSuccess) e = cudaMalloc(&out, sizeof(double) * 64);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(t, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice,
                         h->stream);
@@ -1245,12 +1257,10 @@ ns3d_status ensure_record(ns3d_solver* h) {
   if (e != cudaSuccess) {
     cudaFree(t);
     cudaFree(part);
-    cudaFree(out);
     return cuda_fail(h, e, "record buffers");
   }
   h->rec_tab = t;
   h->rec_partial = part;
-  h->rec_out = out;
   return NS3D_OK;
 }
 
@@ -1295,11 +1305,15 @@ ns3d_status shapiro_minmax(ns3d_solver* h, const double* ux, const double* uy, c
       ux, uy, uz, grid_geom(h), decay, h->rec_partial);
   NS3D_CHECK(h, cudaGetLastError(), "shapiro_error");
   ns3d::minmax_final_kernel<<<1, 1024, 0, h->stream>>>(h->rec_partial, kDiagBlocks,
-                                                       h->rec_out + 50);
+                                                       h->rec_out + kMinMaxAt);
   NS3D_CHECK(h, cudaGetLastError(), "minmax_final");
-  NS3D_CHECK(h, cudaMemcpyAsync(mm, h->rec_out + 50, 2 * sizeof(double), cudaMemcpyDeviceToHost,
+  double out[3];  // min, max, the flag
+  NS3D_CHECK(h, cudaMemcpyAsync(out, h->rec_out + kMinMaxAt, sizeof(out), cudaMemcpyDeviceToHost,
                                 h->stream), "shapiro copy");
   NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "shapiro sync");
+  NS3D_TRY(flagged(h, out + 2));
+  mm[0] = out[0];
+  mm[1] = out[1];
   return NS3D_OK;
 }
 
@@ -1349,9 +1363,12 @@ ns3d_status ns3d_record(ns3d_solver* h, const ns3d_complex* ux, const ns3d_compl
       h->rec_partial, kDiagBlocks, h->diag_out, (const double2*)ux, (const double2*)uy,
       (const double2*)uz, h->rec_reads, total_time, Re, h->geom.inv_vol, h->rec_out);
   NS3D_CHECK(h, cudaGetLastError(), "record_final");
-  NS3D_CHECK(h, cudaMemcpyAsync(rec, h->rec_out, sizeof(double) * NS3D_RECORD_COLUMNS,
-                                cudaMemcpyDeviceToHost, h->stream), "record copy");
+  double out[kFlagAt + 1];
+  NS3D_CHECK(h, cudaMemcpyAsync(out, h->rec_out, sizeof(out), cudaMemcpyDeviceToHost, h->stream),
+             "record copy");
   NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "record sync");
+  NS3D_TRY(flagged(h, out + kFlagAt));
+  std::memcpy(rec, out, sizeof(double) * NS3D_RECORD_COLUMNS);
   for (int i = 0; i < NS3D_RECORD_COLUMNS; ++i)
     if (!std::isfinite(rec[i])) return fail(h, NS3D_ERR_NONFINITE, "record is not finite");
   return NS3D_OK;
@@ -1370,7 +1387,7 @@ ns3d_status ns3d_energy_spectrum(ns3d_solver* h, const ns3d_complex* ux, const n
   NS3D_CHECK(h, cudaGetLastError(), "spectrum");
   NS3D_CHECK(h, cudaMemcpyAsync(E, d, sizeof(double) * size, cudaMemcpyDeviceToHost, h->stream),
              "spectrum copy");
-  NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "spectrum sync");
+  NS3D_TRY(settle(h, "spectrum sync"));
   return NS3D_OK;
 }
 
@@ -1762,10 +1779,12 @@ ns3d_status ns3d_ensemble_diagnostics(ns3d_ensemble* e, const ns3d_complex* ux,
                                                        h->diag_out + 3 * b);
     NS3D_CHECK(h, cudaGetLastError(), "diag_final");
   }
-  std::vector<double> r(3 * (size_t)h->batch);
-  NS3D_CHECK(h, cudaMemcpyAsync(r.data(), h->diag_out, sizeof(double) * r.size(),
+  std::vector<double> out(1 + 3 * (size_t)h->batch);  // the flag, then the sums
+  NS3D_CHECK(h, cudaMemcpyAsync(out.data(), h->diag_out - 1, sizeof(double) * out.size(),
                                 cudaMemcpyDeviceToHost, h->stream), "diag copy");
   NS3D_CHECK(h, cudaStreamSynchronize(h->stream), "diag sync");
+  NS3D_TRY(flagged(h, out.data()));
+  const double* r = out.data() + 1;
   bool finite = true;
   for (int b = 0; b < h->batch; ++b) {
     energy[b] = r[3 * b];

@@ -51,11 +51,15 @@ struct ns3d_solver {
   const double2* f_dense[3] = {};
   // diagnostics
   double* diag_partial = nullptr;
-  double* diag_out = nullptr;
   // record / spectrum / Shapiro buffers (allocated on first use)
   double2* rec_tab = nullptr;
   double* rec_partial = nullptr;  // kDiagBlocks x kRecordSums, then 2 x kDiagBlocks min/max
-  double* rec_out = nullptr;      // 50 record columns, then 2 min/max
+  // what goes to the host, in one allocation, so that a read-back of a part next
+  // to the flag of the bounded waits brings the flag along: the record's columns,
+  // 2 min/max, the flag, 3 sums per instance
+  double* results = nullptr;
+  double* rec_out = nullptr;
+  double* diag_out = nullptr;
   ns3d::RecordReads rec_reads{};
   long long rec_points[3] = {};
   // cached RK3 step graph
@@ -75,7 +79,7 @@ struct ns3d_solver {
   // tensor maps of inv_y's bulk-copy form (tile 2 of the inv_y family) over
   // A and B; null when the extent has no such form
   ns3d::InvYMaps* ymaps = nullptr;
-  int* dev_err = nullptr;  // device flag of the bounded mbarrier waits (0: none gave up)
+  int* dev_err = nullptr;  // device flag of the bounded mbarrier waits (0: none gave up), in results
   size_t bytes = 0;
   std::string err;
 };
@@ -89,6 +93,12 @@ constexpr int kDiagThreads = 256;
 ns3d_status fail(ns3d_solver* h, ns3d_status s, const std::string& msg);
 ns3d_status cuda_fail(ns3d_solver* h, cudaError_t e, const char* where);
 ns3d_status check_handle(ns3d_solver* h);
+// Every call that hands results to the host reports a bounded wait that gave up
+// (NS3D_ERR_TIMEOUT, once).  flagged: `word` is the flag's double as copied with
+// the results; settle: waits for the stream and copies the flag by itself.
+constexpr int kMinMaxAt = NS3D_RECORD_COLUMNS, kFlagAt = kMinMaxAt + 2;
+ns3d_status flagged(ns3d_solver* h, const double* word);
+ns3d_status settle(ns3d_solver* h, const char* where);
 // What the mask (qcut[Nx][Ny], build_mask_cutoff) leaves: the tables of PassGeom.
 struct LiveTables {
   int Zc = 0, Zp = 0;
