@@ -512,7 +512,9 @@ typedef struct ns3d_result {
   int steps;
   double arrival, admitted, done; /* -1: not yet */
   double v_norm;
-  int status; /* -1 pending, NS3D_OK, NS3D_ERR_NONFINITE, NS3D_ERR_CANCELLED */
+  int status; /* -1 pending, NS3D_OK, NS3D_ERR_NONFINITE, NS3D_ERR_CANCELLED, or
+               * NS3D_ERR_TIMEOUT: a bounded wait gave up in a step of its grid
+               * while it ran (its fields are invalid) */
 } ns3d_result;
 
 /* A request that brings its own fields: the work a Newton-Krylov,
@@ -570,6 +572,8 @@ ns3d_status ns3d_server_set_forcing(ns3d_server* s, int N, const ns3d_complex* f
  * host thread while ns3d_server_run runs.  NS3D_ERR_BAD_ARG for an unknown
  * or finished request. */
 ns3d_status ns3d_server_cancel(ns3d_server* s, long long id);
+/* ns3d_selftest_expire_wait on the stream and flag of grid N. */
+ns3d_status ns3d_selftest_expire_server_wait(ns3d_server* s, int N);
 /* Runs the engine like ns3d_server_run but returns as soon as request `id`
  * is done (other requests progress meanwhile and keep their slots). */
 ns3d_status ns3d_server_run_until(ns3d_server* s, long long id, double max_seconds,

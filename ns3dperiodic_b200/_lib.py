@@ -28,7 +28,7 @@ STATUS = {
 EXPORTS = (
     "ns3d_create", "ns3d_destroy", "ns3d_supported_extent", "ns3d_selftest_bounded_wait",
     "ns3d_selftest_stage_drain", "ns3d_selftest_late_phase", "ns3d_selftest_fail_capture",
-    "ns3d_selftest_expire_wait", "ns3d_set_stream",
+    "ns3d_selftest_expire_wait", "ns3d_selftest_expire_server_wait", "ns3d_set_stream",
     "ns3d_synchronize", "ns3d_last_error", "ns3d_status_string", "ns3d_device_bytes",
     "ns3d_set_forcing", "ns3d_forcing_modes", "ns3d_rk3_step", "ns3d_rk3_steps",
     "ns3d_euler_step", "ns3d_rhs", "ns3d_convolution", "ns3d_convolution_uv",
@@ -152,6 +152,7 @@ def _sig(lib):
         "ns3d_selftest_late_phase": ([_P], c_int),
         "ns3d_selftest_fail_capture": ([_P, c_int], c_int),
         "ns3d_selftest_expire_wait": ([_P], c_int),
+        "ns3d_selftest_expire_server_wait": ([_P, c_int], c_int),
         "ns3d_set_stream": ([_P, _P], c_int),
         "ns3d_synchronize": ([_P], c_int),
         "ns3d_last_error": ([_P], ctypes.c_char_p),

@@ -222,6 +222,7 @@ using Clock = std::chrono::steady_clock;
 struct Slot {
   long long req;
   int steps_total, steps_launched;
+  bool timed_out = false;  // a bounded wait gave up in one of its steps
 };
 
 struct Group {
@@ -236,6 +237,7 @@ struct Group {
   double* params_host = nullptr;  // pinned (dt, Re) x capacity
   double* scratch = nullptr;      // kSumBlocks + 1 doubles
   double* norm_host = nullptr;    // pinned
+  int* flag_host = nullptr;       // the handle's flag of the bounded waits (behind norm_host)
   std::deque<long long> queue;    // requests of this grid not yet admitted, arrival order
   long long instance_steps = 0;   // JVP steps launched, summed over the active slots
   // captured JVP step per active-slot count (index active - 1): the 25
@@ -319,7 +321,9 @@ ns3d_status free_slot(ns3d_server* s, Group& g, size_t b) {
   return NS3D_OK;
 }
 
-// retire finished requests of a grid whose stream is idle
+// Retires the finished requests of a grid whose stream is idle.  A step's kernels
+// carry all active slots, so a bounded wait that gave up since the last
+// retirement counts against each of them.
 ns3d_status retire(ns3d_server* s, Group& g, double now) {
   for (size_t b = 0; b < g.slots.size();) {
     Slot& sl = g.slots[b];
@@ -336,6 +340,8 @@ ns3d_status retire(ns3d_server* s, Group& g, double now) {
     SRV_CHECK(s, cudaGetLastError(), "norm");
     SRV_CHECK(s, cudaMemcpyAsync(g.norm_host, g.scratch + kSumBlocks, sizeof(double),
                                  cudaMemcpyDeviceToHost, st), "norm copy");
+    SRV_CHECK(s, cudaMemcpyAsync(g.flag_host, g.h->dev_err, sizeof(int),
+                                 cudaMemcpyDeviceToHost, st), "error flag");
     if (s->req[(size_t)sl.req].keep) {
       std::vector<double2>& out = s->kept[sl.req];
       out.resize(3 * g.nc);
@@ -354,9 +360,15 @@ ns3d_status retire(ns3d_server* s, Group& g, double now) {
       }
     }
     SRV_CHECK(s, cudaStreamSynchronize(st), "retire sync");
+    if (*g.flag_host) {
+      SRV_CHECK(s, cudaMemsetAsync(g.h->dev_err, 0, sizeof(int), st), "error flag");
+      for (auto& each : g.slots) each.timed_out = true;
+    }
     r.v_norm = std::sqrt(*g.norm_host);
     r.done = now;
-    r.status = std::isfinite(r.v_norm) ? NS3D_OK : NS3D_ERR_NONFINITE;
+    r.status = sl.timed_out                ? NS3D_ERR_TIMEOUT
+               : std::isfinite(r.v_norm) ? NS3D_OK
+                                         : NS3D_ERR_NONFINITE;
     {
       std::lock_guard<std::mutex> lk(s->mu);
       s->finished[(size_t)sl.req] = 1;
@@ -601,9 +613,10 @@ ns3d_status ns3d_server_create(const int* Ns, int nN, const int* capacity, doubl
         return bail(NS3D_ERR_OOM);
     if (cudaMalloc(&g.scratch, sizeof(double) * (kSumBlocks + 1)) != cudaSuccess ||
         cudaMallocHost(&g.params_host, sizeof(double) * 2 * cap) != cudaSuccess ||
-        cudaMallocHost(&g.norm_host, sizeof(double)) != cudaSuccess ||
+        cudaMallocHost(&g.norm_host, 2 * sizeof(double)) != cudaSuccess ||
         cudaEventCreateWithFlags(&g.ev, cudaEventDisableTiming) != cudaSuccess)
       return bail(NS3D_ERR_OOM);
+    g.flag_host = reinterpret_cast<int*>(g.norm_host + 1);
     // the Kolmogorov forcing sin(4y) x of the base flow
     std::vector<double2> f(g.nc, make_double2(0.0, 0.0));
     const double a = 0.5 * (double)N * N * N;
@@ -765,6 +778,11 @@ ns3d_status ns3d_server_set_forcing(ns3d_server* s, int N, const ns3d_complex* f
   if (st != NS3D_OK) return sfail(s, st, ns3d_last_error(g->h));
   drop_step_graphs(*g);
   return NS3D_OK;
+}
+
+ns3d_status ns3d_selftest_expire_server_wait(ns3d_server* s, int N) {
+  Group* g = s ? group_of(s, N) : nullptr;
+  return g ? ns3d_selftest_expire_wait(g->h) : NS3D_ERR_BAD_ARG;
 }
 
 ns3d_status ns3d_server_cancel(ns3d_server* s, long long id) {
