@@ -423,6 +423,20 @@ constexpr int p_fxr(int n) {
 }
 constexpr int nslot_fxr(int p) { return p > 12 ? 2 : (p > 8 ? 3 : NS3D_FX_SLOTS); }
 constexpr bool fx_use_ring(int n) { return n % 3 != 0 || n / 12 < NS3D_SPREAD_T || n / 12 >= 32; }
+// The 16-point ring keeps fwd_x_kernel's results bit for bit, and loses to it
+// while an SM has one CTA of it, or not even that: its update then waits for one
+// unit after the other with no other CTA's transforms to cover them.  FP64 lines,
+// whose fwd_x_kernel is slower, cross over at two thirds of the SMs; the implicit
+// update (two divisions a point, and fwd_x_kernel spills) stays with the ring, and
+// so does the plain convolution, which has no update.
+// The RK3 step on a B200, fwd_x_kernel / ring: 128 x 32 x 64 (66 groups) 120 / 135
+// us, FP32 lines 109 / 123; 128 x 64 x 64 (132 groups) 188 / 180, FP32 129 / 141;
+// 512 x 8 x 8 (10 groups) 98 / 113.  Implicit step at 128 x 64 x 64 134 / 118 us.
+constexpr long long kSms = 148;
+template <typename C>
+inline bool fx_few_groups(long long groups) {
+  return groups <= (sizeof(C) == 8 ? kSms : 2 * kSms / 3);
+}
 
 template <int N, int P, int MODE, bool COMBINE, typename C>
 cudaError_t launch_fwd_x_ring(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t st,
@@ -439,6 +453,26 @@ cudaError_t launch_fwd_x_ring(const FwdXArgs<C>& a, const PassGeom& g, cudaStrea
   return cudaGetLastError();
 }
 
+template <int N, int MODE, bool COMBINE, typename C>
+cudaError_t launch_fwd_x_n(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t st,
+                           bool prepare_only) {
+  if constexpr (!fx_use_ring(N)) {
+    return launch_fwd_x_p<N, p_fx(N), MODE, COMBINE, C>(a, g, st, prepare_only);
+  } else if constexpr (p_fxr(N) != 16 || MODE == kImplicit || MODE == kConvOut) {
+    return launch_fwd_x_ring<N, p_fxr(N), MODE, COMBINE, C>(a, g, st, prepare_only);
+  } else {
+    static_assert(p_fx(N) == p_fxr(N), "the same transform in both kernels");
+    const long long lines = (long long)g.Ny * g.Mz * nbatch(g);
+    constexpr int LPC = LaneMap<N / p_fx(N)>::LPC;
+    if (prepare_only || !fx_few_groups<C>((lines + LPC - 1) / LPC)) {
+      const cudaError_t e =
+          launch_fwd_x_ring<N, p_fxr(N), MODE, COMBINE, C>(a, g, st, prepare_only);
+      if (!prepare_only || e != cudaSuccess) return e;
+    }
+    return launch_fwd_x_p<N, p_fx(N), MODE, COMBINE, C>(a, g, st, prepare_only);
+  }
+}
+
 template <int MODE, bool COMBINE, typename C>
 cudaError_t launch_fwd_x(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t st,
                          bool prepare_only = false) {
@@ -449,9 +483,7 @@ cudaError_t launch_fwd_x(const FwdXArgs<C>& a, const PassGeom& g, cudaStream_t s
       if (g.tile[kTileFwdX])                                                          \
         return launch_fwd_x_p<N, p_alt(N), MODE, COMBINE, C>(a, g, st, prepare_only); \
     }                                                                                 \
-    if constexpr (fx_use_ring(N))                                                \
-      return launch_fwd_x_ring<N, p_fxr(N), MODE, COMBINE, C>(a, g, st, prepare_only); \
-    return launch_fwd_x_p<N, p_fx(N), MODE, COMBINE, C>(a, g, st, prepare_only);
+    return launch_fwd_x_n<N, MODE, COMBINE, C>(a, g, st, prepare_only);
     NS3D_FOR_EACH_EXTENT(NS3D_CASE)
 #undef NS3D_CASE
     default:
