@@ -773,10 +773,10 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void* p, unsigned bytes) 
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// L2 prefetch of a row of n elements, trimmed to 16-byte boundaries
+// L2 prefetch of n elements, trimmed to 16-byte boundaries
 template <typename C>
-__device__ __forceinline__ void prefetch_z_line(const C* row, int n) {
-  const uintptr_t b = (uintptr_t)row & ~(uintptr_t)15, e = (uintptr_t)(row + n) & ~(uintptr_t)15;
+__device__ __forceinline__ void prefetch_z_rows(const C* rows, int n) {
+  const uintptr_t b = (uintptr_t)rows & ~(uintptr_t)15, e = (uintptr_t)(rows + n) & ~(uintptr_t)15;
   if (e > b) prefetch_l2_bulk((const void*)b, (unsigned)(e - b));
 }
 
@@ -1134,10 +1134,14 @@ __global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C, STAGED>::MINC))
         q[s] = u(0, s) * (w[s].x * sc) + u(1, s) * (w[s].y * sc) + u(2, s) * q[s];
     }
   };
-  // rows read where they are used: worth an L2 prefetch where the nine fields
-  // are larger than what L2 keeps of them between inv_y and this pass
-  const bool ask = !STAGE && valid && t == 0 &&
-                   (size_t)nb * g.Zp * (9 * sizeof(C)) > ((size_t)64 << 20);
+  // Rows read where they are used: the CTA's rows of a field are one run, and
+  // threads 0 and 1 ask for the next stage's two runs into L2.  A request per row
+  // costs more than the loads: 32 a warp and field at one thread per line.  Per
+  // launch on a B200, a request per row / this: 512 x 128 x 16 51 / 38 us, 256 x
+  // 512 x 16 90 / 62 (FP32 lines 51 / 37), 384 x 512 x 8 68 / 37.
+  const size_t run0 = (size_t)blockIdx.x * LM::LPC * g.Zp;
+  const int nrun = (nb - (int)blockIdx.x * LM::LPC < LM::LPC ? nb - (int)blockIdx.x * LM::LPC
+                                                             : LM::LPC) * g.Zp;
   auto transform = [&](auto k) {
     // stage k's fields: (C_0, C_1), (C_2, C_2), (E_2, D_2), (C_0, C_1), (E_0, D_0), (E_1, D_1)
     auto f1 = [&](int n) { return n == 0 || n == 3 ? a.C[0] : (n == 1 ? a.C[2] : a.E[n < 3 ? 2 : n - 4]); };
@@ -1159,9 +1163,9 @@ __global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C, STAGED>::MINC))
       // and its product
       if (k < 5) next(f1(k + 1), f2(k + 1));
     } else {
-      if (ask && k < 5) {  // the next stage's rows into L2
-        prefetch_z_line(f1(k + 1) + base, g.Zc);
-        prefetch_z_line(f2(k + 1) + base, g.Zc);
+      if (k < 5) {  // the next stage's rows into L2
+        if (threadIdx.x == 0) prefetch_z_rows(f1(k + 1) + run0, nrun);
+        if (threadIdx.x == 1 && f2(k + 1) != f1(k + 1)) prefetch_z_rows(f2(k + 1) + run0, nrun);
       }
       load(f1(k) + base, f2(k) + base);
     }
@@ -1244,8 +1248,8 @@ struct ZRun {
 template <typename C>
 __device__ __forceinline__ void prefetch_z_pair(const C* f1, const C* f2, const ZRun& r) {
   if (!r.ask) return;
-  prefetch_z_line(f1 + r.base, r.Zc);
-  prefetch_z_line(f2 + r.base, r.Zc);
+  prefetch_z_rows(f1 + r.base, r.Zc);
+  prefetch_z_rows(f2 + r.base, r.Zc);
 }
 
 // One component of B(u,v)_i = (v.grad) u_i + (u.grad) v_i in the z pass
