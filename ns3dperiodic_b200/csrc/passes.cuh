@@ -72,8 +72,8 @@ struct PassGeom {
   // Everything outside is zero through inv_x and inv_y, so the passes neither
   // compute, store nor read it, and their scratch (A..E) is compact:
   // [Nx][Ny][Zp], Zp = Zc rounded up to whole 128-byte blocks of 8 FP64
-  // elements where that fits Mz, so that every row of the x / y passes'
-  // scratch starts on a 128-byte boundary.  Per launch on a B200 at 256^3 FP64 (whole
+  // elements where that fits Mz and pays (build_live), so that every row of the
+  // x / y passes' scratch starts on a 128-byte boundary.  Per launch on a B200 at 256^3 FP64 (whole
   // lines at row stride Mz / the mask's lines at row stride Mz, misaligned /
   // this layout): inv_x 217 / 177 / 173 us, inv_y 448 / 335 / 267, z 450 /
   // 457 / 403; the RK3 step 4.84 -> 3.96 ms.

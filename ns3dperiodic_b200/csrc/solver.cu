@@ -112,6 +112,14 @@ LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut) {
       t.Zp = (t.Zc + a - 1) / a * a;
       break;
     }
+  // No padding where it would be above an eighth of an even row (6 and 12 modes,
+  // Nz = 16 and 32): a third more of every pass, and rows a power of two apart,
+  // which a z pass of one or two threads a line reads from the same banks.  The
+  // RK3 step on a B200, padded / not: 128 x 128 x 32 260 / 243 us (FP32 lines 184 /
+  // 155), 512 x 192 x 16 695 / 623 (548 / 535).  Odd rows (9, 17, 33 modes) stay
+  // padded: FP32 rows of 10 and 36 elements lose (256 x 256 x 24 408 / 424, 96^3
+  // 237 / 242), and pairs of lines need an even number.
+  if (t.Zc % 2 == 0 && 8 * (t.Zp - t.Zc) > t.Zc) t.Zp = t.Zc;
   for (int k = 0; k < Ny; ++k)
     for (int l = 0; l < t.ycut[k]; l += 8) t.live.push_back(k << 16 | l);
   return t;
