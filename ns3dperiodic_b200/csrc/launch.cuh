@@ -190,7 +190,7 @@ constexpr int prec_tag() { return sizeof(C) == 16 ? 0 : 100; }
 template <int N, int P, int NF, typename C, int V = 0>
 cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStream_t st,
                            bool prepare_only) {
-  const long long lines = 8LL * g.nlive * nbatch(g);
+  const long long lines = ((long long)g.nlive * nbatch(g)) << g.lw;
   using S = PassSmem<N, P, C, double2, V>;
   const long long groups = (lines + S::LPC - 1) / S::LPC;
   const unsigned grid = persistent_grid<KTag<0, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(

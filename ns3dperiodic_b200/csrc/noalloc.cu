@@ -57,7 +57,7 @@ struct DeviceSlot {
   int Nx = 0, Ny = 0, Nz = 0;
   double Lx = 0, Ly = 0, Lz = 0;
   // what that grid's mask leaves (PassGeom); the tables follow the cut-offs
-  int Zc = 0, Zp = 0, nlive = 0;
+  int Zc = 0, Zp = 0, nlive = 0, lw = 0;
 };
 
 // the live blocks and row cut-offs, after the Nx Ny cut-offs
@@ -145,6 +145,7 @@ extern "C" ns3d_status ns3d_convolution_noalloc(int Nx, int Ny, int Nz, double L
     slot.Zc = lt.Zc;
     slot.Zp = lt.Zp;
     slot.nlive = (int)n;
+    slot.lw = lt.lw;
     // the host staging arrays are reused by the next refresh
     if (cudaStreamSynchronize(st) != cudaSuccess) return NS3D_ERR_CUDA;
     slot.Nx = Nx; slot.Ny = Ny; slot.Nz = Nz;
@@ -160,6 +161,7 @@ extern "C" ns3d_status ns3d_convolution_noalloc(int Nx, int Ny, int Nz, double L
   g.Zc = slot.Zc;
   g.Zp = slot.Zp;
   g.nlive = slot.nlive;
+  g.lw = slot.lw;
   g.live = live_tables(qcut, Nx, Ny);
   g.ycut = (const uint16_t*)(g.live + slot.nlive);
 

@@ -67,8 +67,8 @@ struct PassGeom {
   int tile[4];
   // What the 2/3 mask leaves of the inverse transforms' input (build_live):
   // Zc kz modes (every mode l >= Zc is masked on every line), per y row the
-  // ycut[y] leading modes that survive for some kx, and the nlive blocks of 8
-  // consecutive z that hold a surviving x line (y << 16 | z of the first).
+  // ycut[y] leading modes that survive for some kx, and the nlive blocks of
+  // 1 << lw consecutive z that hold a surviving x line (y << 16 | z of the first).
   // Everything outside is zero through inv_x and inv_y, so the passes neither
   // compute, store nor read it, and their scratch (A..E) is compact:
   // [Nx][Ny][Zp], Zp = Zc rounded up to whole 128-byte blocks of 8 FP64
@@ -78,7 +78,7 @@ struct PassGeom {
   // this layout): inv_x 217 / 177 / 173 us, inv_y 448 / 335 / 267, z 450 /
   // 457 / 403; the RK3 step 4.84 -> 3.96 ms.
   int Zc, Zp;
-  int nlive;
+  int nlive, lw;
   const int* live;
   const uint16_t* ycut;
 };
@@ -333,20 +333,18 @@ __global__ void __launch_bounds__(kThreads, xy_ctas<C>(P, NB))
   double2* pf = S::pf(dsm);
   const int nlines = g.Ny * g.Mz;       // x stride of the state
   const int olines = g.Ny * g.Zp;       // x stride of the scratch
-  // only the blocks of 8 lines with a mode inside the mask: about 0.62 of the lines
-  const int tlines = 8 * g.nlive * nbatch(g);
+  // only the blocks of lines with a mode inside the mask: about 0.62 of the lines
+  const int tlines = (g.nlive * nbatch(g)) << g.lw;
   const int groups = (tlines + LM::LPC - 1) / LM::LPC;
-  // Line G: block G / 8 of the batch's live blocks.  Sets its elements at
+  // Line G: block G >> lw of the batch's live blocks.  Sets its elements at
   // x = 0 in the state and the scratch, the surviving modes, and whether it exists.
   auto line = [&](int G, size_t& in, size_t& out, uint32_t& keep) -> bool {
-    bool valid = G < tlines;
-    const int blk = valid ? G >> 3 : 0;
+    const bool valid = G < tlines;
+    const int blk = valid ? G >> g.lw : 0;
     const int inst = blk / g.nlive;
     const int e = __ldg(g.live + (blk - inst * g.nlive));
     const int y = e >> 16;
-    int z = (e & 0xffff) + (G & 7);
-    valid = valid && z < g.Zp;
-    z = valid ? z : 0;
+    const int z = (e & 0xffff) + (G & ((1 << g.lw) - 1));  // below Zp: 1 << lw divides it
     in = (size_t)inst * NX * nlines + (size_t)(y * g.Mz + z);
     out = (size_t)inst * NX * olines + (size_t)(y * g.Zp + z);
     keep = mask_bits<NX>(a.qcut, g.Ny, y, z, valid, t, T, P);

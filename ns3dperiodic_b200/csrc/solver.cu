@@ -120,8 +120,14 @@ LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut) {
   // padded: FP32 rows of 10 and 36 elements lose (256 x 256 x 24 408 / 424, 96^3
   // 237 / 242), and pairs of lines need an even number.
   if (t.Zc % 2 == 0 && 8 * (t.Zp - t.Zc) > t.Zc) t.Zp = t.Zc;
+  // Blocks of 8 lines, fewer where 8 does not divide a row: blocks that run past
+  // it left a quarter (Zp = 6, 12) or half (4) of inv_x's lines idle.  inv_x on a
+  // B200, blocks of 8 / these: 384 x 512 x 8 74 / 50 us, 512 x 192 x 16 60 / 36, 128
+  // x 128 x 32 16.4 / 14.1, 512 x 512 x 32 163 / 150.
+  t.lw = 3;
+  while (t.Zp % (1 << t.lw)) --t.lw;
   for (int k = 0; k < Ny; ++k)
-    for (int l = 0; l < t.ycut[k]; l += 8) t.live.push_back(k << 16 | l);
+    for (int l = 0; l < t.ycut[k]; l += 1 << t.lw) t.live.push_back(k << 16 | l);
   return t;
 }
 
@@ -573,6 +579,7 @@ ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double L
     h->geom.Zc = lt.Zc;
     h->geom.Zp = lt.Zp;
     h->geom.nlive = (int)n;
+    h->geom.lw = lt.lw;
     h->geom.live = h->live;
     h->geom.ycut = yc;
     h->bytes += bytes;

@@ -101,9 +101,9 @@ ns3d_status flagged(ns3d_solver* h, const double* word);
 ns3d_status settle(ns3d_solver* h, const char* where);
 // What the mask (qcut[Nx][Ny], build_mask_cutoff) leaves: the tables of PassGeom.
 struct LiveTables {
-  int Zc = 0, Zp = 0;
+  int Zc = 0, Zp = 0, lw = 0;
   std::vector<uint16_t> ycut;  // [Ny]
-  std::vector<int> live;       // blocks of 8 lines, y << 16 | z
+  std::vector<int> live;       // blocks of 1 << lw lines, y << 16 | z
 };
 LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut);
 // a handle for `batch` instances of one grid (batch = 1: ns3d_create)
