@@ -223,16 +223,11 @@ __device__ __forceinline__ void line_sync() {
 }
 
 // shared-memory line buffer index with one pad slot every PADW entries;
-// PADW = 0: no padding, the position inside each row of 16 elements XORed
-// with bits 3..6 of the index (the 8-byte lines of the FP32 z pass, whose
-// Stockham exchanges the padding leaves 2-way bank conflicted); PADW = -1:
-// likewise with the row's own number (16-byte lines of radix 16: no words lost
-// to padding)
+// PADW = -1: no padding, the position inside each row of 16 elements XORed with
+// the row's number (16-byte lines of radix 16: no words lost to padding)
 template <int PADW>
 __device__ __forceinline__ int spad(int p) {
-  if constexpr (PADW == 0) {
-    return (p & ~15) | ((p & 15) ^ ((p >> 3) & 15));
-  } else if constexpr (PADW < 0) {
+  if constexpr (PADW < 0) {
     return p ^ ((p >> 4) & 15);
   } else {
     return p + p / PADW;
@@ -450,7 +445,7 @@ struct LineFFT {
     StageTw<N, 1, L>::fill(tws, tw_g);
     __syncthreads();
   }
-  // PW: the line-buffer index scheme (PADW, or 0 for the XOR swizzle);
+  // PW: the line-buffer index scheme (PADW, or -1 for the XOR swizzle);
   // SW: the synchronisation width (T: the line's threads share a warp)
   template <int DIR, int PW = PADW, int SW = T, typename C>
   __device__ __forceinline__ static void run(C (&x)[P], int t, C* sbuf,

@@ -193,8 +193,6 @@ cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStre
   const long long lines = ((long long)g.nlive * nbatch(g)) << g.lw;
   using S = PassSmem<N, P, C, double2, V>;
   const long long groups = (lines + S::LPC - 1) / S::LPC;
-  const unsigned grid = persistent_grid<KTag<0, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
-      inv_x_kernel<N, P, NF, C, V>, S::BYTES, groups);
   const unsigned grid1 = persistent_grid<KTag<60, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_x_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
   constexpr bool DENSE = sizeof(C) == 8 ? P > 8 && N / P < 32
@@ -208,12 +206,16 @@ cudaError_t launch_inv_x_p(const InvXArgs<NF, C>& a, const PassGeom& g, cudaStre
       inv_x_kernel<N, P, NF, C, V, 1, 1><<<dim3(gridd, NF), kThreads, S1::BYTES, st>>>(a, g);
       return cudaGetLastError();
     }
+  } else {
+    const unsigned grid = persistent_grid<KTag<0, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
+        inv_x_kernel<N, P, NF, C, V>, S::BYTES, groups);
+    if (prepare_only) return cudaGetLastError();
+    if (!one_field_per_cta(groups)) {
+      inv_x_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
+      return cudaGetLastError();
+    }
   }
-  if (prepare_only) return cudaGetLastError();
-  if (one_field_per_cta(groups))
-    inv_x_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);
-  else
-    inv_x_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
+  inv_x_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);
   return cudaGetLastError();
 }
 
@@ -307,8 +309,6 @@ cudaError_t launch_inv_y_p(const InvYArgs<NF, C>& a, const PassGeom& g, cudaStre
   const long long lines = (long long)g.Nx * g.Zp;
   using S = PassSmem<N, P, C, C, V>;
   const long long groups = (lines + S::LPC - 1) / S::LPC;
-  const unsigned grid = persistent_grid<KTag<1, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
-      inv_y_kernel<N, P, NF, C, V>, S::BYTES, groups);
   const unsigned grid1 = persistent_grid<KTag<61, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
       inv_y_kernel<N, P, NF, C, V, 1>, S::BYTES, groups);
   constexpr bool DENSE = dense_ctas<P, C>(N / P >= 32);
@@ -321,12 +321,16 @@ cudaError_t launch_inv_y_p(const InvYArgs<NF, C>& a, const PassGeom& g, cudaStre
       inv_y_kernel<N, P, NF, C, V, 1, 1><<<dim3(gridd, NF), kThreads, S1::BYTES, st>>>(a, g);
       return cudaGetLastError();
     }
+  } else {
+    const unsigned grid = persistent_grid<KTag<1, N, P, NF + prec_tag<C>() + 1000 * V>, cap_grid<C, N>()>(
+        inv_y_kernel<N, P, NF, C, V>, S::BYTES, groups);
+    if (prepare_only) return cudaGetLastError();
+    if (!one_field_per_cta(groups)) {
+      inv_y_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
+      return cudaGetLastError();
+    }
   }
-  if (prepare_only) return cudaGetLastError();
-  if (one_field_per_cta(groups))
-    inv_y_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);
-  else
-    inv_y_kernel<N, P, NF, C, V><<<grid, kThreads, S::BYTES, st>>>(a, g);
+  inv_y_kernel<N, P, NF, C, V, 1><<<dim3(grid1, NF), kThreads, S::BYTES, st>>>(a, g);
   return cudaGetLastError();
 }
 

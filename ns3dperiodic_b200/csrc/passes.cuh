@@ -256,10 +256,6 @@ __device__ __forceinline__ GroupRange group_range(int groups) {
 
 constexpr size_t align16(size_t b) { return (b + 15) / 16 * 16; }
 
-// Dynamic shared memory of a pipelined pass: the stage twiddles and the line
-// buffers in the line precision C, then each thread's NB buffers of
-// prefetched elements of type E (the pass's input, FP64 state or scratch).
-// V: the radix schedule (PlanV).
 // CTAs per SM asked of ptxas by a form of the x / y passes with NB prefetch
 // buffers: the one-buffer form's shared memory leaves room for three
 // (168 registers), four for FP32 lines (128 registers).
@@ -268,6 +264,10 @@ __host__ __device__ constexpr int xy_ctas(int p, int nb) {
   return nb == 1 ? (sizeof(C) == 8 ? 4 : 3) : min_ctas_xy(p);
 }
 
+// Dynamic shared memory of a pipelined pass: the stage twiddles and the line
+// buffers in the line precision C, then each thread's NB buffers of
+// prefetched elements of type E (the pass's input, FP64 state or scratch).
+// V: the radix schedule (PlanV).
 // NB: prefetch buffers (2: the next unit's copies run under this unit; 1: the
 // buffer is refilled once its samples are in registers).
 template <int N, int P, typename C = double2, typename E = C, int V = 0, int NB = 2>
@@ -834,20 +834,17 @@ __device__ __forceinline__ void load_pair(C (&w)[P], const C* f1, const C* f2, i
   }
 }
 
+// Line-buffer index scheme of the z pass: for FP64 lines of 512 points the
+// swizzle by rows, as free of conflicts as the padding and without its words
+// (three CTAs then fit an SM); the padding else.
+template <int NZ, int P, typename C>
+__host__ __device__ constexpr int z_pw() {
+  return sizeof(C) == 16 && P == 16 && NZ == 512 ? -1 : LineFFT<NZ, P>::PADW;
+}
+
 // w holds FFT_z(Q1 + i Q2) at k = t + T s.  Split it with the mirror bin
 // W[N-k] (exchanged through shared memory) and store the half spectra
 // Q1h[k], Q2h[k] for k = 0..N/2.
-// Line-buffer index scheme of the z pass: the XOR swizzle for FP32 lines of
-// 128 points and more (fewer shared-memory wavefronts); for FP64 lines of 512
-// points the swizzle by rows, as free of conflicts as the padding and without
-// its words (three CTAs then fit an SM); the padding else.
-template <int NZ, int P, typename C>
-__host__ __device__ constexpr int z_pw() {
-  return (sizeof(C) == 8 && P == 8 && (NZ & (NZ - 1)) == 0 && NZ >= 128) ? 0
-         : (sizeof(C) == 16 && P == 16 && NZ == 512)                     ? -1
-                                                     : LineFFT<NZ, P>::PADW;
-}
-
 template <int NZ, int P, typename C>
 __device__ __forceinline__ void store_pair_spectrum(const C (&w)[P], C* sbuf, int t,
                                                     C* __restrict__ o1,
@@ -1897,8 +1894,11 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
   constexpr int T = F::T;
   constexpr int NUPD = MODE == kConvOut ? 0 : (COMBINE ? 6 : 3);
   constexpr int UPG = 3 + NUPD;  // units per group
-  // The 16-point extents ran fwd_x_kernel before: its compiled form's choice of
-  // fused multiply-adds is written out for them, so their results keep every bit.
+  // 16 points a thread (lines of 128 and 512 points) run here or in fwd_x_kernel by
+  // the number of groups, and a result must not depend on that: the explicit
+  // update's fused multiply-adds are written out in the order that gives
+  // fwd_x_kernel's outputs bit for bit (the one of the eight possible orders that
+  // does).
   constexpr bool FUSED = P == 16;
   static_assert(NSLOT >= 2 && P % 2 == 0, "ring depth, halves of a combining unit");
   extern __shared__ __align__(16) unsigned char dsm[];
