@@ -1849,8 +1849,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasFwdX) fwd_x_kernel(FwdXArgs<
 // per point.  The loop over the components is not unrolled: three copies of
 // the update's code stall on instruction fetches (2.1 of 10 stall cycles per
 // issue at 256^3; FP32 lines of 384 points 117 against 85 us, of 64 points 16.4
-// against 14.3).  FP32 lines of 256 points, one wave after the other of resident
-// CTAs, gain from the unrolled form (260 against 299 us).  An in-place update is
+// against 14.3, of 256 points, 256 x 64 x 64, 38.9 against 28.5).  An in-place update is
 // safe: every element is copied once, by the thread that later writes it,
 // before it writes it.  Per plain FP64 launch on a B200 (unrolled, separate
 // units for u^n; 128^3 and 512^3: fwd_x_kernel -> this form): 128^3 56 -> 49
@@ -2009,8 +2008,7 @@ __global__ void __launch_bounds__(kThreads, (FxRingSmem<NX, P, NSLOT, C>::MINC))
                                 : kx * qi[0][s] + ky * qi[1][s] + kz * qi[2][s];
         kq[s] = kk > 0.0 ? kQ / kk : 0.0;
       }
-      constexpr int UNROLL_C = sizeof(C) == 8 && NX == 256 ? 3 : 1;
-#pragma unroll UNROLL_C
+#pragma unroll 1
       for (int c = 0; c < 3; ++c) {
         const double kc = c == 0 ? 0.0 : (c == 1 ? ky : kz);
         constexpr int NH = COMBINE ? 2 : 1;  // units of a component
