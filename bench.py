@@ -244,6 +244,46 @@ def sizes(N):
     return nc, Sc, Sr
 
 
+def pass_bytes(N, fp32=False):
+    """Bytes the passes move at N^3, by name: what the 2/3 mask leaves, counted
+    from the library's own cut-offs.  rhs: the five passes of one right-hand
+    side (fwd_x in its plain form); rk3: one RK3_SSP step (two of its three
+    updates also read u^n); jvp: one RK3_SSP_UV step, with u transformed anew
+    for the first tangent evaluation; jvp_held: a later step of the same call,
+    which finds u transformed; linearised: one product J(u) v without packing.
+    FP32 mode: half of everything but the state."""
+    import ctypes
+
+    import numpy as np
+
+    from ns3dperiodic_b200 import _lib
+
+    cut = np.zeros((N, N), np.uint16)
+    box = [2.0 * math.pi] * 3
+    if _lib.lib().ns3d_mask_cutoff(N, N, N, *box, ctypes.c_void_p(cut.ctypes.data)) != 0:
+        raise ValueError(f"no mask for {N}^3")
+    rows = cut.max(axis=0).astype(np.int64)
+    f = 16.0 * N * N  # bytes per kz mode of a field
+    h = 0.5 if fp32 else 1.0
+    kept = 16.0 * float(cut.sum())          # modes inside the mask
+    lines = f * float(rows.sum()) / N * h   # x lines with one
+    kz = f * float(rows.max()) * h          # y and z lines to the highest one
+    Sc = f * (N // 2 + 1)
+    rhs = {"inv_x": 3 * kept + 6 * lines, "inv_y": 6 * lines + 9 * kz, "z": 9 * kz + 3 * h * Sc,
+           "fwd_y": 6 * h * Sc, "fwd_x": 3 * h * Sc + 6 * Sc}
+    nl = sum(rhs.values())
+    front = rhs["inv_x"] + rhs["inv_y"]     # three fields' transforms
+    uv = nl + front + 9 * kz                # six fields into the z pass
+    step3 = 3 * nl + 2 * 3 * Sc
+    # the first stage of a JVP step finds u's transforms, a held step's first
+    # tangent evaluation too; its second update combines
+    jvp = uv + (step3 - front) + uv + 3 * Sc
+    return {"rhs": rhs, "rk3": step3, "jvp": jvp, "jvp_held": jvp - front, "linearised": uv}
+
+
+JVP_LAUNCHES = 23  # of one RK3_SSP_UV step
+
+
 # ---------------------------------------------------------------------------
 # CPU baseline: the oracle (numpy/scipy pocketfft) on the host cores
 # ---------------------------------------------------------------------------
@@ -338,12 +378,8 @@ def run_ours(args, world, rank, local, pg):
 
     # per-pass timing (CUDA events on the launching stream), dominant kernel
     names = ["inv_x", "inv_y", "z", "fwd_y", "fwd_x"]
-    # algorithmic bytes per launch: the inverse passes move what the 2/3 mask
-    # leaves (0.52 of the modes, 0.60 of the x lines, 2/3 of the y and z lines);
-    # FP32 scratch halves every field but the state
-    h = 0.5 if fp32 else 1.0
-    alg = [(3 * 0.52 + 6 * 0.60 * h) * Sc, (6 * 0.60 + 9 * 2 / 3) * h * Sc,
-           (9 * 2 / 3 + 3) * h * Sc, 6 * h * Sc, (3 * h + 6) * Sc]
+    moved = pass_bytes(N, fp32)
+    alg = [moved["rhs"][n] for n in names]
     with torch.cuda.stream(stream):
         pm = S.profile_passes(U, dt, Re, reps=20)
     dom = max(range(5), key=lambda i: pm[i])
@@ -415,9 +451,7 @@ def run_ours(args, world, rank, local, pg):
                     "energy_rel_diff_vs_fp64": abs(e32 - e64) / abs(e64),
                     "tolerance": 1e-5}
     S.close()
-    # P3L bytes; FP32 mode: 3 RHS of 30 S_c (6 + 7.5 + 6 + 3 + 7.5) plus the
-    # FP64 partners u^n of stages 2 and 3 (6 S_c)
-    p3l = (90 + 6) * Sc + 9 * Sr if fp32 else 159 * Sc + 18 * Sr
+    p3l = moved["rk3"]
     line = {
         "metric": f"RK3 steps/s (Kolmogorov {N}^3 {'FP32 mode' if fp32 else 'FP64'})",
         "value": round(value, 3),
@@ -515,12 +549,12 @@ def run_reference(args, world, rank, local, pg):
 # Krylov workload: Arnoldi factorisations with the reference's self-test
 # operator (Source/Arnoldi/cuda_test.cu:63-70: N = 2,300,000, m = k*5 = 30)
 # ---------------------------------------------------------------------------
-def arnoldi_bytes(n, m):
-    """Gram-Schmidt bytes of one factorisation: the sum over columns of
-    3 (j+1) n 8 B: the dots, the update that forms the reorthogonalisation's
-    dots, and its update each read V(:, 0..j) once (4 past 48 columns, where
-    every pass reads it by itself)."""
-    return sum((3 if j < 48 else 4) * (j + 1) * n * 8 for j in range(1, m))
+def arnoldi_bytes(n, m, first=1, fused=True):
+    """Gram-Schmidt bytes of one factorisation's columns first .. m - 1: the dots,
+    the update that forms the reorthogonalisation's dots, and its update each
+    read V(:, 0..j) once, 3 (j+1) n 8 B a column; 4 reads where every pass reads
+    it by itself: past 48 columns, and in the reference (fused False)."""
+    return sum((3 if fused and j < 48 else 4) * (j + 1) * n * 8 for j in range(first, m))
 
 
 def arnoldi_start(n, seed):
@@ -567,11 +601,12 @@ def run_ours_arnoldi(args, world, rank, local, pg):
     ms_step = ms / args.steps
     value = world * args.steps / (ms / 1e3)
     peak, peak_src = peaks()
-    # dominant kernel: the dot products over all m columns (the widest launch)
+    # dominant kernel: the dot products over all m columns (the widest launch);
+    # the factorisation's own kernel, gs_pass to 48 columns
     pm = kr.profile(V, m, f0d, reps=20)
     alg_t = (m + 1) * n * 8
     achieved = alg_t / (pm[0] * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "gemv_t_partial+reduce_cols",
+    roofline = {"bound": "hbm", "kernel": "gs_pass" if m <= 48 else "gemv_t_partial+reduce_cols",
                 "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": None, "peak_source": peak_src,
                 "alg_bytes_per_launch": alg_t, "ms_per_launch": round(pm[0], 5),
@@ -675,7 +710,7 @@ def run_reference_arnoldi(args, world, rank, local, pg):
     if ms < 0:
         return {"impl": "reference", "unavailable": "reference Arnoldi_driver run failed"}
     value = args.steps / (ms / 1e3)
-    B = arnoldi_bytes(n, m)
+    B = arnoldi_bytes(n, m, fused=False)
     return {"impl": "reference",
             "metric": f"Arnoldi factorisations/s (1-D periodic Laplacian, n={n}, m={m}, FP64)",
             "value": round(value, 3), "unit": "factorisations/s", "n_gpus": 1,
@@ -748,8 +783,9 @@ def run_ours_ira(args, world, rank, local, pg):
     kr = Krylov(n, m)
     A = kr.exponential_map(S, Ud, Vs, dt, Re, steps) if expo else kr.linearised_map(S, Ud, Re)
     # launches per map call: unpack, the steps' passes (JVP step: 2 tangent
-    # right-hand sides of 5 launches and a base RK3 step of 15), pack
-    per_call = 2 + 25 * steps if expo else 7
+    # right-hand sides of 5 launches and a base RK3 step of 13, whose first stage
+    # finds u transformed), pack
+    per_call = 2 + JVP_LAUNCHES * steps if expo else 7
 
     launches = [0]
 
@@ -789,15 +825,12 @@ def run_ours_ira(args, world, rank, local, pg):
     value = world * args.steps / (ms / 1e3)
     w, X, res, rn, cols, it = out
     peak, peak_src = peaks()
-    # bytes of one run: map calls (P3L) + Gram-Schmidt (one reorthogonalisation)
-    _, Sc, Sr = sizes(N)
-    mv_bytes = steps * (330 * Sc + 30 * Sr) if expo else 84 * Sc + 6 * Sr
+    # bytes of one run: map calls + Gram-Schmidt (one reorthogonalisation)
+    moved = pass_bytes(N)
+    mv_bytes = (moved["jvp"] + (steps - 1) * moved["jvp_held"] if expo
+                else moved["linearised"])
     calls = sum(cols) + k
-    gs = 0
-    for c in cols:
-        for j in range(m - c, m):
-            gs += (3 if j < 48 else 4) * (j + 1) * 8 * n
-    B = mv_bytes * calls + gs
+    B = mv_bytes * calls + sum(arnoldi_bytes(n, m, first=m - c) for c in cols)
     # the map alone, timed on the device
     x = torch.as_tensor(ira_start(n, 99), device="cuda")
     y = torch.empty_like(x)
@@ -1043,12 +1076,9 @@ def ensemble_instances(count, seed0=0):
 
 
 def ensemble_bytes(instances, steps, fp32=False):
-    """P3L bytes of every instance (FP32 mode: scratch fields halved, state FP64)."""
-    tot = 0
-    for _, N, _ in instances:
-        _, Sc, Sr = sizes(N)
-        tot += steps * ((96 * Sc + 9 * Sr) if fp32 else (159 * Sc + 18 * Sr))
-    return tot
+    """Bytes of every instance's steps."""
+    step = {N: pass_bytes(N, fp32)["rk3"] for N in {N for _, N, _ in instances}}
+    return steps * sum(step[N] for _, N, _ in instances)
 
 
 def run_ours_ensemble(args, world, rank, local, pg):
@@ -1323,11 +1353,6 @@ def latency_stats(res):
             "per_N": {str(N): sum(1 for r in done if r["N"] == N) for N in SERVE_NS}}
 
 
-def jvp_bytes(N):
-    _, Sc, Sr = sizes(N)
-    return 330 * Sc + 30 * Sr
-
-
 def run_ours_serving(args, world, rank, local, pg):
     import torch
 
@@ -1355,7 +1380,7 @@ def run_ours_serving(args, world, rank, local, pg):
     done = [r for r in res if r["done"] >= 0.0]
     wall = max_over_ranks(wall, pg)
     thr = world * len(done) / wall
-    step_bytes = sum(jvp_bytes(N) * k for N, k in work.items())
+    step_bytes = sum(pass_bytes(N)["jvp"] * k for N, k in work.items())
     sat = latency_stats(res)
 
     # 2. below saturation: 60% of the measured completion rate, drained
@@ -1418,7 +1443,7 @@ def run_ours_serving(args, world, rank, local, pg):
                                       "CUDA events",
                    "speedup_vs_serial": round(thr / world / serial, 3)},
         "roofline": {"bound": "hbm", "kernel": "all passes of every JVP step the server ran "
-                                               "in the window (330 S_c + 30 S_r per step)",
+                                               "in the window",
                      "achieved": round(step_bytes / wall / 1e9, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(step_bytes / wall / 1e9 / peak, 4),
                      "traffic": None, "peak_source": peak_src},

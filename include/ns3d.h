@@ -701,7 +701,7 @@ ns3d_status ns3d_ira_restart(ns3d_krylov* kr, double* V, double* f, double* Q, c
  * `reps` after one warm-up) of the three basis kernels on the first `ncols`
  * columns of V (device, n x ncols, leading dimension n) and the vector x:
  * ms[0] the dot products V^T x (with their fixed-order reduction), ms[1]
- * y = x - V c, ms[2] the restart pass over V with identity coefficients (V
+ * y = x - V c (with ||y||, as the factorisation forms it, to 48 columns), ms[2] the restart pass over V with identity coefficients (V
  * and x are not changed).  For roofline reports. */
 ns3d_status ns3d_krylov_profile(ns3d_krylov* kr, const double* V, int ncols, const double* x,
                                 int reps, double* ms);

@@ -946,9 +946,13 @@ ns3d_status ns3d_krylov_profile(ns3d_krylov* kr, const double* V, int ncols, con
     for (int r = -1; r < reps; ++r) {  // r = -1: warm-up
       if (r == 0) cudaEventRecord(e0, kr->stream);
       if (which == 0) {
-        KR_TRY(dots(kr, V, ncols, x, kStore, cd, nullptr, nullptr));
+        KR_TRY(ncols <= kGsMaxCols
+                   ? gs<kDots>(kr, V, ncols, nullptr, x, nullptr, kStore, cd, nullptr, nullptr)
+                   : dots(kr, V, ncols, x, kStore, cd, nullptr, nullptr));
       } else if (which == 1) {
-        KR_TRY(subtract(kr, V, ncols, cd, x, kr->w));
+        KR_TRY(ncols <= kGsMaxCols
+                   ? gs<kSubNorm>(kr, V, ncols, cd, x, kr->w, kNorm, kr->small, nullptr, nullptr)
+                   : subtract(kr, V, ncols, cd, x, kr->w));
       } else {
         KR_CHECK(kr, launch_restart(const_cast<double*>(V), kr->n, ncols, k0, kr->qcoef, 0.0,
                                     1.0, kr->w, kr->stream),
