@@ -1129,14 +1129,16 @@ __global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C, STAGED>::MINC))
         q[s] = u(0, s) * (w[s].x * sc) + u(1, s) * (w[s].y * sc) + u(2, s) * q[s];
     }
   };
-  // Rows read where they are used: the CTA's rows of a field are one run, and
-  // threads 0 and 1 ask for the next stage's two runs into L2.  A request per row
-  // costs more than the loads: 32 a warp and field at one thread per line.  Per
-  // launch on a B200, a request per row / this: 512 x 128 x 16 51 / 38 us, 256 x
-  // 512 x 16 90 / 62 (FP32 lines 51 / 37), 384 x 512 x 8 68 / 37.
-  const size_t run0 = (size_t)blockIdx.x * LM::LPC * g.Zp;
-  const int nrun = (nb - (int)blockIdx.x * LM::LPC < LM::LPC ? nb - (int)blockIdx.x * LM::LPC
-                                                             : LM::LPC) * g.Zp;
+  // Rows read where they are used: worth an L2 prefetch where the nine fields are
+  // larger than what L2 keeps of them between inv_y and this pass.  The CTA's rows
+  // of a field are one run, which thread 0 (on the first row) asks for.  A request
+  // per row costs more than the loads: 32 a warp and field at one thread
+  // per line.  Per launch on a B200, a request per row / this: 512 x 128 x 16 51 /
+  // 38 us, 256 x 512 x 16 90 / 62 (FP32 lines 51 / 37), 384 x 512 x 8 68 / 37.
+  // Grids that stay in L2 lose to the requests (three 32^3 solvers in turn 43 / 47 us
+  // a step).
+  const bool ask = !STAGE && threadIdx.x == 0 &&
+                   (size_t)nb * g.Zp * (9 * sizeof(C)) > ((size_t)64 << 20);
   auto transform = [&](auto k) {
     // stage k's fields: (C_0, C_1), (C_2, C_2), (E_2, D_2), (C_0, C_1), (E_0, D_0), (E_1, D_1)
     auto f1 = [&](int n) { return n == 0 || n == 3 ? a.C[0] : (n == 1 ? a.C[2] : a.E[n < 3 ? 2 : n - 4]); };
@@ -1158,9 +1160,10 @@ __global__ void __launch_bounds__(kThreads, (ZSmem<NZ, P, C, STAGED>::MINC))
       // and its product
       if (k < 5) next(f1(k + 1), f2(k + 1));
     } else {
-      if (k < 5) {  // the next stage's rows into L2
-        if (threadIdx.x == 0) prefetch_z_rows(f1(k + 1) + run0, nrun);
-        if (threadIdx.x == 1 && f2(k + 1) != f1(k + 1)) prefetch_z_rows(f2(k + 1) + run0, nrun);
+      if (ask && k < 5) {  // the next stage's rows into L2
+        const int n = (nb - b < LM::LPC ? nb - b : LM::LPC) * g.Zp;
+        prefetch_z_rows(f1(k + 1) + base, n);
+        if (k != 0) prefetch_z_rows(f2(k + 1) + base, n);  // stage 1 reads one field
       }
       load(f1(k) + base, f2(k) + base);
     }
