@@ -337,14 +337,17 @@ __global__ void __launch_bounds__(kThreads, xy_ctas<C>(P, NB))
   const int tlines = (g.nlive * nbatch(g)) << g.lw;
   const int groups = (tlines + LM::LPC - 1) / LM::LPC;
   // Line G: block G >> lw of the batch's live blocks.  Sets its elements at
-  // x = 0 in the state and the scratch, the surviving modes, and whether it exists.
+  // x = 0 in the state and the scratch, the surviving modes, and whether it exists
+  // (a block may run past its row).
   auto line = [&](int G, size_t& in, size_t& out, uint32_t& keep) -> bool {
-    const bool valid = G < tlines;
+    bool valid = G < tlines;
     const int blk = valid ? G >> g.lw : 0;
     const int inst = blk / g.nlive;
     const int e = __ldg(g.live + (blk - inst * g.nlive));
     const int y = e >> 16;
-    const int z = (e & 0xffff) + (G & ((1 << g.lw) - 1));  // below Zp: 1 << lw divides it
+    int z = (e & 0xffff) + (G & ((1 << g.lw) - 1));
+    valid = valid && z < g.Zp;
+    z = valid ? z : 0;
     in = (size_t)inst * NX * nlines + (size_t)(y * g.Mz + z);
     out = (size_t)inst * NX * olines + (size_t)(y * g.Zp + z);
     keep = mask_bits<NX>(a.qcut, g.Ny, y, z, valid, t, T, P);

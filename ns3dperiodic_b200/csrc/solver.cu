@@ -99,7 +99,8 @@ bool build_mask_cutoff(int Nx, int Ny, int Nz, double Lx, double Ly, double Lz,
   return true;
 }
 
-LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut) {
+LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut, int batch) {
+  const long long planes = (long long)Nx * batch;
   LiveTables t;
   t.ycut.assign(Ny, 0);
   for (int j = 0; j < Nx; ++j)
@@ -120,12 +121,17 @@ LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut) {
   // padded: FP32 rows of 10 and 36 elements lose (256 x 256 x 24 408 / 424, 96^3
   // 237 / 242), and pairs of lines need an even number.
   if (t.Zc % 2 == 0 && 8 * (t.Zp - t.Zc) > t.Zc) t.Zp = t.Zc;
-  // Blocks of 8 lines, fewer where 8 does not divide a row: blocks that run past
-  // it left a quarter (Zp = 6, 12) or half (4) of inv_x's lines idle.  inv_x on a
-  // B200, blocks of 8 / these: 384 x 512 x 8 74 / 50 us, 512 x 192 x 16 60 / 36, 128
-  // x 128 x 32 16.4 / 14.1, 512 x 512 x 32 163 / 150.
+  // Blocks of 8 lines.  Where 8 does not divide a row the last block runs past it
+  // and leaves a quarter (Zp = 6, 12) or half (4) of inv_x's threads without a
+  // line; the largest power of two that divides it then, on grids of at least 32
+  // CTAs a field (2048 points each).  inv_x on a B200, blocks of 8 / these: 384 x
+  // 512 x 8 74 / 50 us, 512 x 192 x 16 60 / 36, 128 x 128 x 32 17.1 / 14.8; smaller
+  // grids gain nothing, and three 32^3 solvers in turn lose (43.4 / 45.5 us a step).
+  long long slots = 0;
+  for (int k = 0; k < Ny; ++k) slots += (t.ycut[k] + 7) / 8 * 8;
   t.lw = 3;
-  while (t.Zp % (1 << t.lw)) --t.lw;
+  if (slots * planes >= 32 * 2048)
+    while (t.Zp % (1 << t.lw)) --t.lw;
   for (int k = 0; k < Ny; ++k)
     for (int l = 0; l < t.ycut[k]; l += 1 << t.lw) t.live.push_back(k << 16 | l);
   return t;
@@ -569,7 +575,7 @@ ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double L
     return bail(NS3D_ERR_OOM);
   cudaMemcpy(h->qcut, qc.data(), sizeof(uint16_t) * qc.size(), cudaMemcpyHostToDevice);
   {
-    const LiveTables lt = build_live(Nx, Ny, h->Mz, qc.data());
+    const LiveTables lt = build_live(Nx, Ny, h->Mz, qc.data(), batch);
     const size_t n = lt.live.size();
     const size_t bytes = sizeof(int) * n + sizeof(uint16_t) * Ny;
     if (cudaMalloc(&h->live, bytes) != cudaSuccess) return bail(NS3D_ERR_OOM);

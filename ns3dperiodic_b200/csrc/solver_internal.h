@@ -105,7 +105,7 @@ struct LiveTables {
   std::vector<uint16_t> ycut;  // [Ny]
   std::vector<int> live;       // blocks of 1 << lw lines, y << 16 | z
 };
-LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut);
+LiveTables build_live(int Nx, int Ny, int Mz, const uint16_t* qcut, int batch = 1);
 // a handle for `batch` instances of one grid (batch = 1: ns3d_create)
 ns3d_status create_solver(int batch, int Nx, int Ny, int Nz, double Lx, double Ly, double Lz,
                           ns3d_solver** out);
