@@ -392,7 +392,7 @@ def run_ours(args, world, rank, local, pg):
     kname = {0: "inv_x_kernel", 1: "inv_y_tma_kernel" if ytma else "inv_y_kernel",
              2: "z_kernel",
              3: "fwd_y_kernel", 4: "fwd_x_ring_kernel" if ring else "fwd_x_kernel"}[dom]
-    traffic = traffic_from_profiles(kname, N)
+    traffic = traffic_from_profiles(kname + (" (FP32)" if fp32 else ""), N)
     roofline = {"bound": "hbm", "kernel": kname, "achieved": round(achieved, 1),
                 "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
                 "traffic": traffic, "peak_source": peak_src,

@@ -121,6 +121,8 @@ constexpr int lines_per_cta_z() {
 
 inline unsigned blocks_for(long long lines, int lpc) { return (unsigned)((lines + lpc - 1) / lpc); }
 
+constexpr long long kSms = 148;  // of a B200: the unit of the rules on group counts below
+
 // Persistent grid for a pipelined pass: set the dynamic shared-memory
 // attribute and query the resident CTAs per SM once per kernel instantiation
 // (Tag) and device; grid = min(groups, SMs x resident CTAs).
@@ -170,7 +172,7 @@ inline unsigned persistent_grid(Kern kern, size_t smem, long long groups) {
 // the shorter chain gives.  The RK3 step on a B200, all fields / one per CTA:
 // 32^3 (16 to 18 groups) 144 / 109 us, 64^3 (48 to 66) 149 / 116; 96^3 (192 to
 // 294) 350 / 372.
-inline bool one_field_per_cta(long long groups) { return groups < 148; }
+inline bool one_field_per_cta(long long groups) { return groups < kSms; }
 // Whether larger grids too run one field per CTA, with one prefetch buffer and
 // three CTAs per SM instead of two: then 12 warps per SM hide what 8 with a
 // deeper pipeline cannot.  FP64 lines of 12 and 16 points only (the others have
@@ -436,7 +438,6 @@ constexpr bool fx_use_ring(int n) { return n % 3 != 0 || n / 12 < NS3D_SPREAD_T 
 // The RK3 step on a B200, fwd_x_kernel / ring: 128 x 32 x 64 (66 groups) 120 / 135
 // us, FP32 lines 109 / 123; 128 x 64 x 64 (132 groups) 188 / 180, FP32 129 / 141;
 // 512 x 8 x 8 (10 groups) 98 / 113.  Implicit step at 128 x 64 x 64 134 / 118 us.
-constexpr long long kSms = 148;
 template <typename C>
 inline bool fx_few_groups(long long groups) {
   return groups <= (sizeof(C) == 8 ? kSms : 2 * kSms / 3);

@@ -892,7 +892,7 @@ struct ZLaneMap {  // lanes of one line are adjacent: the line is contiguous in 
 // z pass: C2R along z of the paired rows, the products, R2C along z.
 //
 // What bounds it is its line transforms: the FP64 pipe and the shared memory the
-// exchanges and rows pass through (59% and 66% busy at 256^3 FP64).  Each
+// exchanges and rows pass through (60% and 66% busy at 256^3 FP64).  Each
 // Stockham exchange moves the whole line through shared memory, so 16 points
 // per thread (one exchange at 256) beat 8 (two): 503 against 534 us per launch.
 // The rest of the form gets 12 warps per SM to run at 16 points per thread:
@@ -903,13 +903,13 @@ struct ZLaneMap {  // lanes of one line are adjacent: the line is contiguous in 
 //    FP32 lines park the velocities in shared memory and keep the rest.
 //  * the rows a transform reads are staged by bulk copies (cp.async.bulk, one
 //    per field for a warp's consecutive rows, completed on an mbarrier), the
-//    next transform's while this one runs (96 to 384 points; ZSmem::STAGE).
+//    next transform's while this one runs (from 96 points; ZSmem::STAGE).
 //  * the six inverse transforms are one loop: unrolled, the eight transforms
 //    outgrow the instruction cache (435 us against 379, a third of all stalls
 //    waiting for instructions).
 // Per launch on a B200 (plain loads behind L2 prefetches, unrolled, stash in
 // shared memory, 8 warps per SM -> this form): FP64 256^3 403 -> 379 us, 128^3
-// 62.4 -> 56.5; FP32 275 -> 229, 47.1 -> 37.9.
+// 62.4 -> 56.3; FP32 275 -> 239, 47.1 -> 37.0.
 // ---------------------------------------------------------------------------
 // CTAs per SM the FP32 lines ask for (they take half the registers)
 #ifndef NS3D_MINCTA_Z32

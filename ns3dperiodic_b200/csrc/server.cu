@@ -240,7 +240,7 @@ struct Group {
   int* flag_host = nullptr;       // the handle's flag of the bounded waits (behind norm_host)
   std::deque<long long> queue;    // requests of this grid not yet admitted, arrival order
   long long instance_steps = 0;   // JVP steps launched, summed over the active slots
-  // captured JVP step per active-slot count (index active - 1): the 25
+  // captured JVP step per active-slot count (index active - 1): the 23
   // launches replay as one graph; dropped when tiles, precision or forcing change
   std::vector<cudaGraphExec_t> step_exec;
   bool graphs_off = false;
